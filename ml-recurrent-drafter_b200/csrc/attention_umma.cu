@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   if (warp == 0 || warp == 6) {
     // ---------------- TMA producers: warp 0 = Q and the K ring, warp 6 = the V ring ----------------
-    if (lane == 0) {
+    if (rd::elect_one()) {
       // a stage is free when the product that read it is done: QK^T of the tile kKStages before for K, PV of the tile
       // kVStages before for V.  Each of these barriers completes once per two tiles, so a parity wait is unambiguous.
       bool ok = true;
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (rd::elect_one()) {
       const uint32_t idesc_qk = idesc_f16(BNK, false);
       const uint32_t idesc_pv = idesc_f16(HD, true);
       const uint32_t tS = tmem_base + kColS, tP = tmem_base + kColP, tO = tmem_base + kColO;

@@ -851,7 +851,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (rd::elect_one()) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       int stage = 0;
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (rd::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -1174,7 +1174,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0) {
+    if (rd::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -1213,7 +1213,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && rd::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;

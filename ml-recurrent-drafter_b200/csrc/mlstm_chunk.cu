@@ -240,7 +240,8 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_states_kernel(const __grid_
   rd_umma::fence_before();
   __syncthreads();
   rd_umma::fence_after();
-  if (tid == 0) load(0);  // the barriers are initialised
+  const bool leader = warp == 0 && rd::elect_one();  // issues the copies and the products
+  if (leader) load(0);  // the barriers are initialised
   const uint32_t tmem = *tmem_slot;
   const int quarter = warp & 3, cg = warp >> 2;
   const int v = v0 + quarter * 32 + lane, dq = d0 + cg * 32;  // this thread's value column and its 32 dims
@@ -251,9 +252,9 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_states_kernel(const __grid_
   for (int c = 0; c < n_chunks; ++c) {
     // the products of chunk c - 1 are in the tile, and its operands' shared memory is free
     if (c > 0) ok = wait_warp(bar, (c - 1) & 1);
-    if (tid == 0) rd_umma::tma_store_wait_read();
+    if (leader) rd_umma::tma_store_wait_read();
     if (!__syncthreads_and(ok)) break;
-    if (tid == 0 && c + 1 < n_chunks) load(c + 1);
+    if (leader && c + 1 < n_chunks) load(c + 1);
     ok = wait_warp(&full[c & 1], (c >> 1) & 1);
     rd_umma::fence_after();
     const float w_next = c + 1 < n_chunks ? w_of(c + 1) : 0.f, A_next = c + 1 < n_chunks ? decay_of(c + 1) : 0.f;
@@ -310,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_states_kernel(const __grid_
       ok = false;
       break;
     }
-    if (tid == 0) {
+    if (leader) {
       rd_umma::fence_after();
       const uint32_t idesc = rd_umma::idesc_f16(DN, true, true);
 #pragma unroll
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_states_kernel(const __grid_
     if (tid < L) s_w[((c + 1) & 1) * L + tid] = w_next;
     A = A_next;
   }
-  if (tid == 0) rd_umma::tma_store_wait();
+  if (leader) rd_umma::tma_store_wait();
   if (ok) ok = wait_warp(bar, (n_chunks - 1) & 1);
   ok = __syncthreads_and(ok);
   if (ok) {
@@ -448,7 +449,8 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_outputs_kernel(const __grid
   __syncthreads();
   rd_umma::fence_after();
   const uint32_t tmem = *tmem_slot;
-  if (tid == 0) {
+  const bool leader = warp == 0 && rd::elect_one();  // issues the copies and the products
+  if (leader) {
     const uint32_t idesc = rd_umma::idesc_f16(128, false, false);
 #pragma unroll
     for (int k = 0; k < DP / 16; ++k) {
@@ -529,7 +531,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_outputs_kernel(const __grid
     }
     return true;
   };
-  if (ok && tid == 0)
+  if (ok && leader)
     for (int i = 0; i < kOutStages && i < n_items; ++i) load(i);  // K has been read: its place is the ring
   __syncwarp();
   // P of this thread's token and a quarter of the keys
@@ -563,7 +565,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_outputs_kernel(const __grid
 
   // ---- O = Q S, then O = e_t O + P V
   if (ok) {
-    if (tid == 0) {
+    if (leader) {
       rd_umma::fence_after();
       ok = run_items(0, n_state);
       if (ok) rd_umma::commit(state_done);
@@ -585,7 +587,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlstm_outputs_kernel(const __grid
   }
   ok = __syncthreads_and(ok);
   if (ok) {
-    if (tid == 0) {
+    if (leader) {
       rd_umma::fence_after();
       ok = run_items(n_state, n_items);
       if (ok) rd_umma::commit(all_done);
