@@ -177,6 +177,13 @@ RD_API void rd_gemm_plan_destroy(void* plan);
 RD_API int rd_gemm_bf16_tc(const void* plan, int out_dtype, void* C, int64_t ldc, const void* bias, const void* R,
                     int64_t ldr, const int32_t* m_dev, int epilogue, int32_t* status, void* stream);
 
+/* C = A W^T + R (RD_EPI_RES), or, for few rows, the shares that a norm kernel adds up (rd_rmsnorm_shares,
+ * rd_stream_norm_shares): up to 256 live rows of at most 1024, K is cut among CTA pairs that the weight tiles alone would leave idle, and
+ * C is not written.  parts: rd_gemm_shares_bytes(m_max, N, K) bytes, 16-byte aligned; 0 means that no row count is cut. */
+RD_API int64_t rd_gemm_shares_bytes(int m_max, int N, int K);
+RD_API int rd_gemm_bf16_tc_res_shares(const void* plan, int out_dtype, void* C, int64_t ldc, const void* R, int64_t ldr,
+                               const int32_t* m_dev, float* parts, int64_t parts_bytes, int32_t* status, void* stream);
+
 /* C = xIELU(A W^T): pos z^2 + z/2 for z > 0, neg (e^z - 1 - z) + z/2 otherwise (pos = softplus(p),
  * neg = 1/2 + softplus(q) of the activation's two parameters).  No counterpart in the reference. */
 RD_API int rd_gemm_xielu(int dtype, const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int m_max,
@@ -280,6 +287,10 @@ RD_API int rd_embed_gather(int dtype, const void* table, const int64_t* ids, voi
 /* y = weight * (x * rsqrt(mean(x^2) + eps)) computed in fp32 (LlamaRMSNorm, modeling_llama.py:21-32). */
 RD_API int rd_rmsnorm(int dtype, const void* x, const void* weight, void* y, int m_max, const int32_t* m_dev, int H,
                float eps, void* stream);
+/* The same for an x that rd_gemm_bf16_tc_res_shares left in shares (same m_max and m_dev, N = H, the same residual, parts and
+ * K): the rows are formed as residual + shares, written to x and normalised.  residual may be x. */
+RD_API int rd_rmsnorm_shares(int dtype, void* x, const void* residual, const float* parts, int K, const void* weight, void* y,
+                      int m_max, const int32_t* m_dev, int H, float eps, void* stream);
 
 /* Splits qkv [M, (nh+2*nkv)*hd], applies NeoX rotary embedding at tok_pos to q and k
  * (apply_rotary_pos_emb, modeling_llama.py:87-110; cos/sin [n_pos, hd] fp32 tables), writes q to
@@ -450,6 +461,11 @@ RD_API int rd_cache_unpack_static(int dtype, void* cache, int NL, int B, int nkv
 RD_API int rd_stream_norm(int dtype, const void* table, const int64_t* ids, float embed_scale, const float* hist,
                    int64_t hist_stride, const float* coeff, int n_hist, float* x_out, const void* weight, void* y, int m_max,
                    const int32_t* m_dev, int H, int groups, float eps, void* stream);
+/* The same for stored rows of which the last (hist + (n_hist - 1) * hist_stride) was left in shares by
+ * rd_gemm_bf16_tc_res_shares: it is formed as residual + shares and written there first.  residual may be that row. */
+RD_API int rd_stream_norm_shares(int dtype, float* hist, int64_t hist_stride, const float* coeff, int n_hist, const float* residual,
+                          const float* parts, int K, float* x_out, const void* weight, void* y, int m_max, const int32_t* m_dev,
+                          int H, int groups, float eps, void* stream);
 
 /* Rotary embedding of the first rot_dims features of every q and k head (feature i paired with i + rot_dims/2;
  * cos/sin tables [n_pos, rot_dims/2]) and the cache append.  proj row: q [nh*dim] | k [nkv*dim] | v [nkv*vdim] | anything;

@@ -265,6 +265,10 @@ struct EpiArgs {
   float norm_dim, norm_eps;
   // RD_EPI_XIELU: the activation's two coefficients; RD_EPI_CLAMPED_GLU: its limit and alpha
   float act0, act1;
+  // kEpiResShares only: with few live rows K is cut (rd::share_count), share i goes to parts[i][part_rows][N] and C is
+  // left to the kernel that adds the shares to R
+  float* parts;
+  int shares, part_rows;
   // kEpiSplit only: output features >= n_split go to C_hi in fp32
   float* C_hi;
   int64_t ld_hi;
@@ -286,6 +290,9 @@ constexpr int kEpiSliceMax = 8;
 // projection whose last output features are needed unrounded: features [0, n_split) are stored as usual, features
 // [n_split, N) as fp32 in a second matrix; n_split is a multiple of 32, so a warp has one kind only
 constexpr int kEpiSplit = 10;
+
+// RD_EPI_RES whose K may be cut into shares; a kernel of its own, so that prompts run without the question
+constexpr int kEpiResShares = 12;
 
 // gated units: weight rows (2i, 2i+1) = (gate_i, up_i), half as many outputs as features
 template <int EPI>
@@ -398,7 +405,7 @@ __device__ __forceinline__ void epilogue_block(float* v, const EpiArgs& e, float
                                                const ResidualRegs<OUT_F32, (kGlu<EPI> ? 16 : 32)>& res,
                                                const float* s_scale, uint4 gamma8, float* ss_red_block) {
   constexpr int kOut = kGlu<EPI> ? 16 : 32;  // output features per token of this warp
-  constexpr bool kRes = (EPI == RD_EPI_BIAS_SILU_RES || EPI == RD_EPI_RES);
+  constexpr bool kRes = (EPI == RD_EPI_BIAS_SILU_RES || EPI == RD_EPI_RES || EPI == kEpiResShares);
   using G = EpiLanes<OUT_F32, kOut>;
   const int out0 = kGlu<EPI> ? (n_warp0 >> 1) : n_warp0;  // first output column of the warp
   if (!vec_ok) {
@@ -929,7 +936,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) belong to this warp
     float* scr = scratch + (warp - 2) * 32 * kScrLd;
     constexpr int kOut = kGlu<EPI> ? 16 : 32;
-    constexpr bool kRes = (EPI == RD_EPI_BIAS_SILU_RES || EPI == RD_EPI_RES);
+    constexpr bool kRes = (EPI == RD_EPI_BIAS_SILU_RES || EPI == RD_EPI_RES || EPI == kEpiResShares);
     const int esz = OUT_F32 ? 4 : 2;
     const bool aligned = (((uintptr_t)epi.C | (uintptr_t)(kRes ? epi.R : epi.C)) % 16 == 0) && ((epi.ldc * esz) % 16 == 0) &&
                          (!kRes || (epi.ldr * esz) % 16 == 0);
@@ -1159,9 +1166,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int M = rd::live_rows(m_dev, m_max);
   RD_TIMING_BEGIN();
   const int w_pairs = (N + 2 * BM - 1) / (2 * BM);
-  const Chunking ch = make_chunking(M, w_pairs, n_pairs);
-  const int all_tiles = M > 0 ? w_pairs * ch.n_chunks : 0;
+  const int shares = EPI == kEpiResShares ? rd::live_shares(epi.shares, M) : 1;
+  const Chunking ch = shares > 1 ? Chunking{1, max(16, (M + 15) / 16 * 16)} : make_chunking(M, w_pairs, n_pairs);
+  const int per_w = shares > 1 ? shares : ch.n_chunks;  // tiles of one weight tile: token chunks, or shares of K
+  const int all_tiles = M > 0 ? w_pairs * per_w : 0;
   const int k_blocks = (K + BK - 1) / BK;  // past K the operand tiles read as zeros
+  auto first_block = [&](int tile) { return shares > 1 ? tile % per_w * k_blocks / shares : 0; };
+  auto end_block = [&](int tile) { return shares > 1 ? (tile % per_w + 1) * k_blocks / shares : k_blocks; };
   // The launch lasts rounds = ceil(tiles / pairs) tile times however the tiles are dealt, so only as many
   // pairs take part as fill those rounds evenly (258 tiles on 74 pairs: 4 rounds, 65 pairs); the others
   // leave at once, and the SMs they free lower the power the busy ones share (c2 step 12.99 -> 12.97 ms).
@@ -1179,18 +1190,19 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = pair_id; ok && tile < total_tiles; tile += n_active) {
-        const int w_pair = tile / ch.n_chunks, ci = tile % ch.n_chunks;
+        const int w_pair = tile / per_w, ci = shares > 1 ? 0 : tile % per_w;
+        const int kb0 = first_block(tile), kb1 = end_block(tile);
         const int cols = chunk_cols(ch, ci, M);
         const int tok0 = ci * ch.chunk + (int)rank * (cols >> 1);  // this CTA's half of the chunk
         const int n_box = ((cols >> 1) + kTokBox - 1) / kTokBox;
         const CUtensorMap* map_a = &maps_a.m[n_box - 1];
         const int w_row0 = w_pair * 2 * BM + (int)rank * BM;
-        for (int kb = 0; kb < k_blocks; kb += L::kSub) {
+        for (int kb = kb0; kb < kb1; kb += L::kSub) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
             ok = false;
             break;
           }
-          const int n_sub = min(L::kSub, k_blocks - kb);
+          const int n_sub = min(L::kSub, kb1 - kb);
           const uint32_t leader_full = mapa_u32(smem_u32(&full[stage]), 0);
           if (rank == 0) mbar_expect_tx(&full[stage], 2 * n_sub * (L::kBoxW + n_box * kTokBoxBytes));
           for (int sb = 0; sb < n_sub; ++sb) {
@@ -1219,7 +1231,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool ok = true;
       int local = 0;
       for (int tile = pair_id; ok && tile < total_tiles; tile += n_active, ++local) {
-        const int ci = tile % ch.n_chunks;
+        const int ci = shares > 1 ? 0 : tile % per_w;
+        const int kb0 = first_block(tile), kb1 = end_block(tile);
         const uint32_t idesc = umma_instr_desc_pair(chunk_cols(ch, ci, M));
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
@@ -1229,18 +1242,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kMaxChunk;
-        for (int kb = 0; kb < k_blocks; kb += L::kSub) {
+        for (int kb = kb0; kb < kb1; kb += L::kSub) {
           if (!mbar_wait(&full[stage], phase, abort_flag)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const int n_sub = min(L::kSub, k_blocks - kb);
+          const int n_sub = min(L::kSub, kb1 - kb);
           for (int sb = 0; sb < n_sub; ++sb) {
             const uint64_t dw = umma_smem_desc(smem_u32(sW + stage * L::kStageW + sb * L::kBoxW));
             const uint64_t da = umma_smem_desc(smem_u32(sA + stage * L::kStageA + sb * L::kBoxA));
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_pair(d_tmem, dw + 2 * k, da + 2 * k, idesc, (kb | sb | k) != 0);
+            for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_pair(d_tmem, dw + 2 * k, da + 2 * k, idesc, ((kb - kb0) | sb | k) != 0);
           }
           umma_commit_pair_both(&empty[stage]);  // frees the stage in both CTAs
           if (++stage == kStages) {
@@ -1259,14 +1272,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int quarter = warp & 3;
     float* scr = scratch + (warp - 2) * 32 * kScrLd;
     constexpr int kOut = kGlu<EPI> ? 16 : 32;
-    constexpr bool kRes = (EPI == RD_EPI_BIAS_SILU_RES || EPI == RD_EPI_RES);
+    constexpr bool kRes = (EPI == RD_EPI_BIAS_SILU_RES || EPI == RD_EPI_RES || EPI == kEpiResShares);
     const int esz = OUT_F32 ? 4 : 2;
     const bool aligned = (((uintptr_t)epi.C | (uintptr_t)(kRes ? epi.R : epi.C)) % 16 == 0) && ((epi.ldc * esz) % 16 == 0) &&
                          (!kRes || (epi.ldr * esz) % 16 == 0);
     bool ok = true;
     int local = 0;
     for (int tile = pair_id; ok && tile < total_tiles; tile += n_active, ++local) {
-      const int w_pair = tile / ch.n_chunks, ci = tile % ch.n_chunks;
+      const int w_pair = tile / per_w, ci = shares > 1 ? 0 : tile % per_w;
       const int cols = chunk_cols(ch, ci, M);
       const int tok_base = ci * ch.chunk;
       const int tok_limit = min(M, tok_base + ch.chunk);
@@ -1291,7 +1304,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint4 gamma8 = make_uint4(0u, 0u, 0u, 0u);
       if (kRes && !OUT_F32 && epi.gamma != nullptr && vec_ok)
         gamma8 = *reinterpret_cast<const uint4*>(epi.gamma + n_warp0 + (lane & 3) * 8);
-      if (kRes && vec_ok) {
+      if (kRes && vec_ok && shares == 1) {
         if (OUT_F32)
           res_next.load(epi, tok_base, out0, tok_limit, lane);
         else
@@ -1306,9 +1319,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * kMaxChunk;
 #pragma unroll 1
       for (int c = 0; c < cols; c += 32) {
-        if (kRes && vec_ok && !OUT_F32) res_next.take(res_buf, lane);
+        if (kRes && vec_ok && !OUT_F32 && shares == 1) res_next.take(res_buf, lane);
         ResidualRegs<OUT_F32, kOut> res_cur = res_next;
-        if (kRes && vec_ok && c + 32 < cols) {
+        if (kRes && vec_ok && c + 32 < cols && shares == 1) {
           if (OUT_F32)
             res_next.load(epi, tok_base + c + 32, out0, tok_limit, lane);
           else
@@ -1328,6 +1341,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                               norm_in ? s_scale + c : nullptr, ss_red + ((c >> 5) & 1) * 128);
         } else if (EPI == kEpiArgmax) {
           epilogue_argmax_block(v, epi, scr, lane, n_warp0, tok_base + c, tok_limit, N);
+        } else if (EPI == kEpiResShares && shares > 1) {
+          EpiArgs part = epi;
+          part.C = epi.parts + (int64_t)(tile % per_w) * epi.part_rows * N;
+          part.ldc = N;
+          epilogue_block<RD_EPI_NONE, true>(v, part, scr, lane, n_warp0, tok_base + c, tok_limit, N, N % 4 == 0 && n_warp0 + 32 <= N,
+                                            ResidualRegs<true, 32>(), nullptr, gamma8, ss_red);
         } else if (EPI == kEpiSplit && n_warp0 >= epi.n_split) {
           epilogue_hi_block(v, epi, lane, n_warp0, tok_base + c, tok_limit, N);
         } else {
@@ -1436,8 +1455,7 @@ int launch_cluster2(Kern kern, int grid, int smem_bytes, cudaStream_t s, const G
   return RD_OK;
 }
 
-template <int EPI>
-int launch_out(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t* m_dev, int32_t* status, cudaStream_t s) {
+int multiprocessors() {
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;
@@ -1445,11 +1463,19 @@ int launch_out(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (sm_count <= 0) sm_count = 148;
   }
+  return sm_count;
+}
+
+template <int EPI>
+int launch_out(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t* m_dev, int32_t* status, cudaStream_t s) {
+  const int sm_count = multiprocessors();
   // upper bound of the tile count with the finest chunking the kernel may choose (64 tokens)
   const int chunks = (p->m_max + 63) / 64;
   if (p->N >= 2 * BM && g_use_pairs) {
     // CTA pairs: one pair per 256 weight rows x token chunk
-    const int tiles = chunks * ((p->N + 2 * BM - 1) / (2 * BM));
+    const int w_pairs = (p->N + 2 * BM - 1) / (2 * BM);
+    int tiles = chunks * w_pairs;
+    if (EPI == kEpiResShares) tiles = max(tiles, w_pairs * e.shares);
     const int max_pairs = sm_count / 2;
     const int grid = 2 * (tiles < max_pairs ? tiles : max_pairs);
     int rc;
@@ -1500,6 +1526,7 @@ int launch_epi(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t
     case RD_EPI_SWIGLU: return launch_out<RD_EPI_SWIGLU>(p, out_dtype, e, m_dev, status, s);
     case RD_EPI_XIELU: return launch_out<RD_EPI_XIELU>(p, out_dtype, e, m_dev, status, s);
     case RD_EPI_CLAMPED_GLU: return launch_out<RD_EPI_CLAMPED_GLU>(p, RD_BF16, e, m_dev, status, s);
+    case kEpiResShares: return launch_out<kEpiResShares>(p, out_dtype, e, m_dev, status, s);
     case kEpiSplit: return launch_out<kEpiSplit>(p, RD_BF16, e, m_dev, status, s);
     case kEpiQkvRope: return launch_out<kEpiQkvRope>(p, out_dtype, e, m_dev, status, s);
     case kEpiArgmax: return launch_out<kEpiArgmax>(p, out_dtype, e, m_dev, status, s);
@@ -1509,6 +1536,8 @@ int launch_epi(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t
 }
 
 }  // namespace
+
+int rd_gemm_pairs() { return g_use_pairs ? multiprocessors() / 2 : 0; }
 
 extern "C" void* rd_gemm_plan_create(const void* A, int64_t lda, int m_max, const void* W, int64_t ldw, int N, int K) {
   if (!A || !W || m_max < 1 || N < 1 || K < BK || K % 8 != 0 || lda < K || ldw < K) return nullptr;
@@ -1546,6 +1575,30 @@ extern "C" int rd_gemm_bf16_tc(const void* plan, int out_dtype, void* C, int64_t
   e.ldr = ldr;
   cudaStream_t s = (cudaStream_t)stream;
   return launch_epi(p, out_dtype, e, m_dev, epilogue, status, s);
+}
+
+extern "C" int64_t rd_gemm_shares_bytes(int m_max, int N, int K) {
+  if (m_max < 1 || N < 1 || K < 1) return 0;
+  const int s = rd::share_count(m_max, N, K, rd_gemm_pairs());
+  return s > 1 ? (int64_t)s * min(m_max, rd::kShareRows) * N * (int64_t)sizeof(float) : 0;
+}
+
+extern "C" int rd_gemm_bf16_tc_res_shares(const void* plan, int out_dtype, void* C, int64_t ldc, const void* R, int64_t ldr,
+                                          const int32_t* m_dev, float* parts, int64_t parts_bytes, int32_t* status, void* stream) {
+  RD_REQUIRE(plan && C && R && parts, RD_ERR_ARG);
+  RD_REQUIRE(out_dtype == RD_F32 || out_dtype == RD_BF16, RD_ERR_DTYPE);
+  const GemmPlan* p = static_cast<const GemmPlan*>(plan);
+  RD_REQUIRE(((uintptr_t)parts & 15) == 0, RD_ERR_ALIGN);
+  RD_REQUIRE(parts_bytes >= rd_gemm_shares_bytes(p->m_max, p->N, p->K), RD_ERR_CAPACITY);
+  EpiArgs e{};
+  e.C = C;
+  e.ldc = ldc;
+  e.R = R;
+  e.ldr = ldr;
+  e.parts = parts;
+  e.shares = rd::share_count(p->m_max, p->N, p->K, rd_gemm_pairs());
+  e.part_rows = min(p->m_max, rd::kShareRows);
+  return launch_epi(p, out_dtype, e, m_dev, e.shares > 1 ? kEpiResShares : RD_EPI_RES, status, (cudaStream_t)stream);
 }
 
 extern "C" int rd_gemm_bf16_tc_xielu(const void* plan, void* C, int64_t ldc, const int32_t* m_dev, float pos, float neg,

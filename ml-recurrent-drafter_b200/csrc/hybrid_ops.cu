@@ -14,19 +14,21 @@ constexpr int kNormMaxThreads = 1024;
 // One block per token.  The row is formed in fp32 (embedding gather, or the weighted sum of `n_hist` stored
 // rows), written to x when asked for, kept in shared memory, and normalised in groups of H / groups
 // features: each group over its own sqrt(mean of squares + eps), the whole times w.
-template <typename T, int VEC>
+template <typename T, int VEC, bool SHARES>
 __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
-    const T* table, const int64_t* ids, float embed_scale, const float* hist,
+    const T* table, const int64_t* ids, float embed_scale, float* hist,
     int64_t hist_stride, const float* coeff, int n_hist, float* x_out, const T* w,
-    T* y, int m_max, const int32_t* m_dev, int H, int groups, int parts, float eps) {
+    T* y, int m_max, const int32_t* m_dev, int H, int groups, int parts, float eps, rd::Shares<float> sh) {
   extern __shared__ float smem[];
   float* row = smem;              // [H]
   float* part_sum = smem + H;     // [groups * parts]
   rd::pdl_launch_dependents();
   rd::pdl_wait();
   const int t = blockIdx.x;
-  if (t >= rd::live_rows(m_dev, m_max)) return;
+  const int M = rd::live_rows(m_dev, m_max);
+  if (t >= M) return;
   const int tid = threadIdx.x, n_thr = blockDim.x;
+  const bool shares = SHARES && rd::live_shares(sh.count, M) > 1;
   if (table != nullptr) {
     const T* src = table + ids[t] * (int64_t)H;
     for (int d = tid * VEC; d < H; d += n_thr * VEC) {
@@ -34,11 +36,21 @@ __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
       for (int e = 0; e < VEC; ++e) row[d + e] = rd::Num<T>::to_f(src[d + e]) * embed_scale;
     }
   } else {
-    const float* src = hist + (int64_t)t * H;
+    float* src = hist + (int64_t)t * H;
     for (int d = tid * VEC; d < H; d += n_thr * VEC) {
       float acc[VEC];
 #pragma unroll
       for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
+      if (shares) {
+        // the last stored row is still in shares: formed here, by the thread that reads it below
+        float f[VEC];
+        rd::add_shares<VEC>(sh, t, H, d, f);
+        float* dst = src + (int64_t)(n_hist - 1) * hist_stride + d;
+        if constexpr (VEC == 4)
+          *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
+        else
+          *dst = f[0];
+      }
       if (coeff == nullptr) {
         if constexpr (VEC == 4) {
           *reinterpret_cast<float4*>(acc) = *reinterpret_cast<const float4*>(src + d);
@@ -220,13 +232,13 @@ __global__ void decode_advance_kernel(const int64_t* next_tok, int64_t* token_bu
     return RD_ERR_DTYPE;                           \
   }
 
-extern "C" int rd_stream_norm(int dtype, const void* table, const int64_t* ids, float embed_scale, const float* hist,
-                              int64_t hist_stride, const float* coeff, int n_hist, float* x_out, const void* weight, void* y,
-                              int m_max, const int32_t* m_dev, int H, int groups, float eps, void* stream) {
+static int stream_norm_launch(int dtype, const void* table, const int64_t* ids, float embed_scale, float* hist, int64_t hist_stride,
+                              const float* coeff, int n_hist, float* x_out, const void* weight, void* y, int m_max,
+                              const int32_t* m_dev, int H, int groups, float eps, const rd::Shares<float>& sh, void* stream) {
   RD_REQUIRE(weight && y && ((table && ids && !hist) || (!table && hist)), RD_ERR_ARG);
   RD_REQUIRE(m_max >= 1 && H >= 1 && groups >= 1 && H % groups == 0 && (table || n_hist >= 1), RD_ERR_SIZE);
   RD_REQUIRE(coeff || table || n_hist == 1, RD_ERR_ARG);
-  const uintptr_t bits = (uintptr_t)hist | (uintptr_t)x_out | (uintptr_t)y | (uintptr_t)weight;
+  const uintptr_t bits = (uintptr_t)hist | (uintptr_t)x_out | (uintptr_t)y | (uintptr_t)weight | (uintptr_t)sh.parts | (uintptr_t)sh.residual;
   const bool vec = H % 4 == 0 && bits % 16 == 0 && hist_stride % 4 == 0;
   int threads = ((vec ? H / 4 : H) + 31) / 32 * 32;
   // few tokens: the row's loads all in flight at once; many tokens: small blocks, several per SM
@@ -238,17 +250,34 @@ extern "C" int rd_stream_norm(int dtype, const void* table, const int64_t* ids, 
   RD_REQUIRE(smem <= 200 * 1024, RD_ERR_SIZE);
   cudaError_t err = cudaSuccess;
   RD_DISPATCH_T(dtype, {
-    auto kern = vec ? stream_norm_kernel<T, 4> : stream_norm_kernel<T, 1>;
+    auto kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true> : stream_norm_kernel<T, 1, true>)
+                             : (vec ? stream_norm_kernel<T, 4, false> : stream_norm_kernel<T, 1, false>);
     if (smem > 48 * 1024) {
       err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       RD_CHECK_CHAINED(err);
     }
     err = rd::launch_chained(kern, dim3(m_max), dim3(threads), smem, (cudaStream_t)stream, 1, (const T*)table, ids,
                              embed_scale, hist, hist_stride, coeff, n_hist, x_out, (const T*)weight, (T*)y, m_max, m_dev, H,
-                             groups, parts, eps);
+                             groups, parts, eps, sh);
   });
   RD_CHECK_CHAINED(err);
   return RD_OK;
+}
+
+extern "C" int rd_stream_norm(int dtype, const void* table, const int64_t* ids, float embed_scale, const float* hist,
+                              int64_t hist_stride, const float* coeff, int n_hist, float* x_out, const void* weight, void* y,
+                              int m_max, const int32_t* m_dev, int H, int groups, float eps, void* stream) {
+  return stream_norm_launch(dtype, table, ids, embed_scale, const_cast<float*>(hist), hist_stride, coeff, n_hist, x_out, weight, y, m_max,
+                            m_dev, H, groups, eps, rd::Shares<float>{nullptr, nullptr, 1, 0}, stream);  // hist is only read
+}
+
+extern "C" int rd_stream_norm_shares(int dtype, float* hist, int64_t hist_stride, const float* coeff, int n_hist, const float* residual,
+                                     const float* parts, int K, float* x_out, const void* weight, void* y, int m_max,
+                                     const int32_t* m_dev, int H, int groups, float eps, void* stream) {
+  RD_REQUIRE(hist && residual && parts && K >= 1, RD_ERR_ARG);
+  return stream_norm_launch(dtype, nullptr, nullptr, 0.f, hist, hist_stride, coeff, n_hist, x_out, weight, y, m_max, m_dev, H, groups, eps,
+                            rd::Shares<float>{parts, residual, rd::share_count(m_max, H, K, rd_gemm_pairs()), m_max < rd::kShareRows ? m_max : rd::kShareRows},
+                            stream);
 }
 
 extern "C" int rd_rotary_append(int dtype, void* proj, int64_t ld, void* k_cache, void* v_cache, const int32_t* tok_row,

@@ -22,22 +22,33 @@ __global__ void embed_gather_kernel(const T* table, const int64_t* ids, T* out,
   for (int d = threadIdx.x; d < H; d += blockDim.x) dst[d] = src[d];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const T* x, const T* w, T* y,
+template <typename T, bool SHARES>
+__global__ void __launch_bounds__(256, SHARES ? 4 : 8) rmsnorm_kernel(T* x, const T* w, T* y,
                                                       int m_max, const int32_t* m_dev, int H, float eps,
-                                                      int vectorised) {
+                                                      int vectorised, rd::Shares<T> sh) {
   constexpr int VEC = 16 / sizeof(T);
   const int t = blockIdx.x;
   rd::pdl_launch_dependents();
   rd::pdl_wait();
-  if (t >= rd::live_rows(m_dev, m_max)) return;
-  const T* xr = x + (int64_t)t * H;
+  const int M = rd::live_rows(m_dev, m_max);
+  if (t >= M) return;
+  T* xr = x + (int64_t)t * H;
   T* yr = y + (int64_t)t * H;
   float ss = 0.f;
+  const bool shares = SHARES && rd::live_shares(sh.count, M) > 1;
   if (vectorised) {
     for (int v = threadIdx.x; v < H / VEC; v += 256) {
       T e[VEC];
-      *reinterpret_cast<uint4*>(e) = reinterpret_cast<const uint4*>(xr)[v];
+      if (shares) {
+        // x is still in shares: formed here, rounded to the model dtype and written before it is normalised
+        float f[VEC];
+        rd::add_shares<VEC>(sh, t, H, v * VEC, f);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) e[i] = rd::Num<T>::from_f(f[i]);
+        reinterpret_cast<uint4*>(xr)[v] = *reinterpret_cast<const uint4*>(e);
+      } else {
+        *reinterpret_cast<uint4*>(e) = reinterpret_cast<const uint4*>(xr)[v];
+      }
 #pragma unroll
       for (int i = 0; i < VEC; ++i) {
         const float f = rd::Num<T>::to_f(e[i]);
@@ -46,6 +57,11 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const T* x, const T* w, T*
     }
   } else {
     for (int d = threadIdx.x; d < H; d += 256) {
+      if (shares) {
+        float f;
+        rd::add_shares<1>(sh, t, H, d, &f);
+        xr[d] = rd::Num<T>::from_f(f);
+      }
       float v = rd::Num<T>::to_f(xr[d]);
       ss += v * v;
     }
@@ -286,18 +302,31 @@ extern "C" int rd_embed_gather(int dtype, const void* table, const int64_t* ids,
   return RD_OK;
 }
 
-extern "C" int rd_rmsnorm(int dtype, const void* x, const void* weight, void* y, int m_max, const int32_t* m_dev, int H,
-                          float eps, void* stream) {
+static int rmsnorm_launch(int dtype, void* x, const void* weight, void* y, int m_max, const int32_t* m_dev, int H, float eps,
+                          const float* parts, const void* residual, int shares, void* stream) {
   RD_REQUIRE(x && weight && y, RD_ERR_ARG);
   RD_REQUIRE(m_max >= 1 && H >= 1, RD_ERR_SIZE);
   cudaStream_t s = (cudaStream_t)stream;
   const int vec = dtype == RD_F32 ? 4 : 8;
-  const int vectorised = (H % vec == 0) && (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)y) % 16 == 0);
+  const int vectorised =
+      (H % vec == 0) && (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)y | (uintptr_t)parts | (uintptr_t)residual) % 16 == 0);
   cudaError_t err = cudaSuccess;
-  RD_DISPATCH_T(dtype, (err = rd::launch_chained(rmsnorm_kernel<T>, dim3(m_max), dim3(256), 0, s, 1, (const T*)x, (const T*)weight,
-                                                 (T*)y, m_max, m_dev, H, eps, vectorised)));
+  RD_DISPATCH_T(dtype, (err = rd::launch_chained(shares > 1 ? rmsnorm_kernel<T, true> : rmsnorm_kernel<T, false>, dim3(m_max), dim3(256), 0, s, 1, (T*)x, (const T*)weight,
+                                                 (T*)y, m_max, m_dev, H, eps, vectorised,
+                                                 rd::Shares<T>{parts, (const T*)residual, shares, m_max < rd::kShareRows ? m_max : rd::kShareRows})));
   RD_CHECK_CHAINED(err);
   return RD_OK;
+}
+
+extern "C" int rd_rmsnorm(int dtype, const void* x, const void* weight, void* y, int m_max, const int32_t* m_dev, int H,
+                          float eps, void* stream) {
+  return rmsnorm_launch(dtype, const_cast<void*>(x), weight, y, m_max, m_dev, H, eps, nullptr, nullptr, 1, stream);  // x is only read
+}
+
+extern "C" int rd_rmsnorm_shares(int dtype, void* x, const void* residual, const float* parts, int K, const void* weight, void* y,
+                                 int m_max, const int32_t* m_dev, int H, float eps, void* stream) {
+  RD_REQUIRE(residual && parts && K >= 1, RD_ERR_ARG);
+  return rmsnorm_launch(dtype, x, weight, y, m_max, m_dev, H, eps, parts, residual, rd::share_count(m_max, H, K, rd_gemm_pairs()), stream);
 }
 
 extern "C" int rd_rope_kv_write(int dtype, const void* qkv, void* q_out, void* k_cache, void* v_cache,

@@ -39,6 +39,8 @@ void rd_set_last_cuda_error(int e);
 // chain with programmatic stream serialisation so that a kernel's launch and prologue overlap the
 // tail of its predecessor.
 int rd_pdl_enabled();
+// CTA pairs that the tcgen05 GEMM launches at most; 0 when it runs without pairs.
+int rd_gemm_pairs();
 
 namespace rd {
 
@@ -110,6 +112,63 @@ __device__ __forceinline__ int live_rows(const int* m_dev, int m_max) {
   if (m_dev == nullptr) return m_max;
   int m = *m_dev;
   return m < m_max ? (m < 0 ? 0 : m) : m_max;
+}
+
+// Into how many shares K of a projection with a residual is cut when few rows are live (RD_EPI_RES; 1 = never).  Up to
+// kShareRows rows are one token chunk, and the weights' tiles of 256 rows alone occupy few CTA pairs (16 of 74 for 4096
+// features); the shares fill one wave, each of at least 8 k-blocks of 64.  With more rows the token chunks fill the wave, and
+// writing and reading the shares costs what the idle pairs would gain.  Launches for more than kShareCapacity rows hardly ever run
+// with so few (a packed draft keeps about 2 rows in 5) and are left as they are: their norm would pay for the question.
+// Projection and norm together, bf16, one B200: 4096 x 11008 weights, 1 row 42 -> 24 us, some 110 rows 44 -> 27 us; 4096 x 4096,
+// 1 row 22 -> 15 us, some 110 rows 23 -> 19 us.
+constexpr int kShareRows = 256;
+constexpr int kShareCapacity = 1024;
+constexpr int kMaxShares = 8;
+inline int share_count(int m_max, int N, int K, int pairs) {
+  if (m_max > kShareCapacity || N < 256) return 1;
+  int s = pairs / ((N + 255) / 256);
+  const int by_length = (K + 63) / 64 / 8;
+  s = s < by_length ? s : by_length;
+  s = s < kMaxShares ? s : kMaxShares;
+  return s > 1 ? s : 1;
+}
+// The shares of such a projection: partial products [shares][rows][N] in fp32, rows = min(m_max, kShareRows), and what they are
+// added to.
+template <typename T>
+struct Shares {
+  const float* parts;
+  const T* residual;  // [m, N]
+  int count, rows;    // count 1: the projection's output is complete
+};
+// the projection and the norm after it come to the same answer from the live rows
+__device__ __forceinline__ int live_shares(int count, int M) { return M <= kShareRows ? count : 1; }
+// residual + sum of the shares of features [d, d + VEC) of row t, the shares in ascending order of K
+template <int VEC, typename T>
+__device__ __forceinline__ void add_shares(const Shares<T>& sh, int t, int N, int d, float* f) {
+  static_assert(VEC == 1 || VEC * sizeof(T) == 16, "vector width");
+  const float* p = sh.parts + (int64_t)t * N + d;
+  float acc[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
+#pragma unroll 2
+  for (int s = 0; s < sh.count; ++s, p += (int64_t)sh.rows * N) {
+    if constexpr (VEC == 1) {
+      acc[0] += *p;
+    } else {
+#pragma unroll
+      for (int i = 0; i < VEC; i += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(p + i);
+        acc[i] += q.x, acc[i + 1] += q.y, acc[i + 2] += q.z, acc[i + 3] += q.w;
+      }
+    }
+  }
+  T r[VEC];
+  if constexpr (VEC == 1)
+    r[0] = sh.residual[(int64_t)t * N + d];
+  else
+    *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(sh.residual + (int64_t)t * N + d);
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) f[i] = acc[i] + Num<T>::to_f(r[i]);
 }
 
 // Programmatic dependent launch.  A kernel launched with rd::launch_chained() may begin before the

@@ -11,7 +11,7 @@ import torch
 from torch import nn
 
 from . import _lib, kv_cache
-from .modeling_common import Linear
+from .modeling_common import Linear, PendingRows
 
 
 @dataclass
@@ -36,6 +36,8 @@ class StepContext:
     n_pos: int
     status: Optional[torch.Tensor]
     ws: Dict[str, torch.Tensor]
+    parts: Optional[torch.Tensor] = None  # where the projections with a residual may leave their rows in shares of K
+    pending: Optional[PendingRows] = None  # the rows that the last such projection left there: the next norm forms them
 
 
 @dataclass(frozen=True)
@@ -244,7 +246,7 @@ class GroupedAttention(_Mixer):
             self._attend_128(ctx, state, q, gate, mixed)
         else:
             self._attend(ctx, state, q, gate, mixed)
-        self.lin[1](mixed, out, _lib.EPI_RES, residual=residual, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        ctx.pending = self.lin[1].add_residual(mixed, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
 
     def _project(self, ctx: StepContext, state, xn):
         """Projection, then rotation, norm and cache append.  Returns the queries' rows and the gates."""
@@ -385,7 +387,7 @@ class LatentAttention(_Mixer):
         mixed = rows_of(ws["mixed"], c.heads * c.vdim)
         self.lin[0].split(xn, q, dkv, self.n_split, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
         (self._expanded if self._expands(ctx) else self._absorbed)(ctx, state, q, dkv, mixed)
-        self.lin[1](mixed, out, _lib.EPI_RES, residual=residual, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        ctx.pending = self.lin[1].add_residual(mixed, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
 
     def _append(self, ctx: StepContext, state, q, dkv, q_rot: torch.Tensor, rot_head: int) -> None:
         """Latents and key parts to the cache; the queries' rotated features to q_rot (rows as q_rot's, heads rot_head apart)."""
@@ -535,7 +537,7 @@ class MatrixMemory(_Mixer):
             self._chunk(ctx, state, proj, gates, mixed)
         else:
             self._scan(ctx.batch, ctx.row_start, ctx.base_len, ctx.max_new, state, proj, gates, mixed)
-        self.lin[1](mixed, out, _lib.EPI_RES, residual=residual, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        ctx.pending = self.lin[1].add_residual(mixed, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
 
     def _chunked(self, ctx: StepContext) -> bool:
         """Prompts of a bf16 model; portions of a few tokens are run one after the other."""
@@ -596,7 +598,7 @@ class _FeedForward(nn.Module):
     def run(self, ctx: StepContext, xn: torch.Tensor, residual: torch.Tensor, out: torch.Tensor) -> None:
         act = rows_of(ctx.ws["act"], row_stride(self.ff))
         self._activate(ctx, xn, act)
-        self.lin[1](act, out, _lib.EPI_RES, residual=residual, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        ctx.pending = self.lin[1].add_residual(act, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
 
 
 class DenseFeedForward(_FeedForward):

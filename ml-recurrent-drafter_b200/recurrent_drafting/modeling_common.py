@@ -1,6 +1,6 @@
 """What the base models share: linear layers on the GEMM kernels and the language-model head."""
 import os
-from typing import Dict, Optional, Tuple
+from typing import Dict, NamedTuple, Optional, Tuple
 
 import torch
 
@@ -14,7 +14,9 @@ class Linear:
         self.weight = weight
         self.bias = bias
         self._plans: Dict[Tuple, int] = {}
+        self._shares_bytes: Dict[int, int] = {}  # by row capacity
 
+    MAX_SHARE_ROWS = 1024  # row capacities above this are never cut (rd_gemm_shares_bytes)
     MAX_PLANS = 32  # distinct (activation buffer, row capacity) pairs remembered per weight
 
     def drop_plans(self) -> None:
@@ -109,6 +111,33 @@ class Linear:
         _lib.call("rd_gemm_bf16_tc_res_norm", plan, _lib.ptr(c), c.stride(0), _lib.ptr(residual), residual.stride(0),
                   _lib.ptr(m_dev), _lib.ptr(gamma), _lib.ptr(c2), c2.stride(0), _lib.ptr(ss), ss.stride(0), _lib.ptr(status),
                   _lib.stream())
+
+    def shares_bytes(self, m_max: int) -> int:
+        """Bytes that add_residual() needs for its shares; 0 where the projection is never cut."""
+        if m_max > self.MAX_SHARE_ROWS:
+            return 0
+        rows = min(m_max, 256)  # more rows need no more room
+        need = self._shares_bytes.get(rows)
+        if need is None:
+            n, k = self.weight.shape
+            need = _lib.load().rd_gemm_shares_bytes(rows, n, k) if self.weight.dtype == torch.bfloat16 else 0
+            self._shares_bytes[rows] = need
+        return need
+
+    def add_residual(self, a: torch.Tensor, c: torch.Tensor, residual: torch.Tensor, m_dev, m_max: int, status: Optional[torch.Tensor],
+                     parts: Optional[torch.Tensor] = None) -> Optional["PendingRows"]:
+        """c = a W^T + residual.  With `parts` given (fp32), few rows are left there in shares of K instead: then the result
+        says what the norm that follows has to add up (rd_gemm_bf16_tc_res_shares)."""
+        n, k = self.weight.shape
+        if parts is not None and self._tc_ok(a, a.stride(0)):
+            need = self.shares_bytes(m_max)
+            if 0 < need <= parts.numel() * 4 and (c.data_ptr() | residual.data_ptr()) % 16 == 0 and c.stride(0) == residual.stride(0) == n:
+                plan = self._plan(a, a.stride(0), m_max)
+                _lib.call("rd_gemm_bf16_tc_res_shares", plan, _lib.dtype_code(c.dtype), _lib.ptr(c), n, _lib.ptr(residual), n, _lib.ptr(m_dev),
+                          _lib.ptr(parts), parts.numel() * 4, _lib.ptr(status), _lib.stream())
+                return PendingRows(residual, parts, k)
+        self(a, c, _lib.EPI_RES, residual=residual, m_dev=m_dev, m_max=m_max, status=status)
+        return None
 
     def swiglu_normed(self, a: torch.Tensor, c: torch.Tensor, ss: torch.Tensor, dim: int, eps: float, m_dev, m_max: int,
                       status: Optional[torch.Tensor]) -> None:
@@ -209,6 +238,14 @@ class Linear:
             _lib.call("rd_gemm", _lib.dtype_code(self.weight.dtype), out_code, _lib.ptr(a), lda, _lib.ptr(self.weight),
                       self.weight.stride(0), _lib.ptr(c), ldc, _lib.ptr(self.bias), _lib.ptr(residual), ldr or 0, m_max,
                       _lib.ptr(m_dev), n, k, epilogue, _lib.stream())
+
+
+class PendingRows(NamedTuple):
+    """Rows that a projection may have left as shares of K: residual + the shares in parts."""
+
+    residual: torch.Tensor
+    parts: torch.Tensor
+    k: int
 
 
 class LMHead:

@@ -37,6 +37,10 @@ class DilavikForCausalLM(StreamDecoder):
     def norm_groups(self) -> int:
         return self.config.norm_groups
 
+    # Its gates are exponential and every layer's result goes on through the depth averages, so the last bit of a sum travels far:
+    # with the sums of its projections in another order a row of greedy tokens parted ways at a near tie.  They keep theirs.
+    projections_in_shares = False
+
     def _make_layers(self) -> List[DecoderLayer]:
         return [DecoderLayer(c, i, self.config, self.rotary, self.scratch) for i, c in enumerate(self.config.layers)]
 

@@ -299,6 +299,9 @@ class LlamaForCausalLM(LMHead, nn.Module):
                                 ("act", self.config.intermediate_size), ("hidden", H)):
                 full[name] = torch.empty(cap_m, width, dtype=dt, device=dev)
             # folded RMS norm: per-token sums of squares by 128-feature slice
+            # shares of the projections with a residual
+            most = max(lin.shares_bytes(min(cap_m, _Linear.MAX_SHARE_ROWS)) for lin in (self._lin()["o"] + self._lin()["down"]))
+            full["parts"] = torch.empty(most // 4, dtype=torch.float32, device=dev)
             full["ss"] = torch.empty(cap_m, ((H + 127) // 128 + 3) // 4 * 4, dtype=torch.float32, device=dev)
         if logit_rows > cap_l:
             cap_l = logit_rows
@@ -307,7 +310,7 @@ class LlamaForCausalLM(LMHead, nn.Module):
             self._ws_full, self._ws_cap = full, (cap_m, cap_l)
             self._ws = {}
             self._drop_plans()
-        ws = {k: (v[:logit_rows] if k == "logits" else v[:m_max]) for k, v in full.items()}
+        ws = {k: (v[:logit_rows] if k == "logits" else v if k == "parts" else v[:m_max]) for k, v in full.items()}
         if len(self._ws) >= 16:
             self._ws.pop(next(iter(self._ws)))
         self._ws[key] = ws
@@ -348,9 +351,19 @@ class LlamaForCausalLM(LMHead, nn.Module):
         fused_norm = (fused_rope and H % 128 == 0 and h.data_ptr() % 16 == 0
                       and os.environ.get("RD_FUSED_NORM", "0") == "1")
         ss = ws["ss"] if fused_norm else None
+        parts = ws["parts"] if ws["parts"].numel() else None
+
+        def norm(weight, y, pending):
+            if pending is None:
+                _lib.call("rd_rmsnorm", code, _lib.ptr(h), _lib.ptr(weight), _lib.ptr(y), m_max, md, H, self.eps, st)
+            else:
+                _lib.call("rd_rmsnorm_shares", code, _lib.ptr(h), _lib.ptr(pending.residual), _lib.ptr(pending.parts), pending.k,
+                          _lib.ptr(weight), _lib.ptr(y), m_max, md, H, self.eps, st)
+
+        pending = None
         for l in range(self.n_layers):
             if not fused_norm or l == 0:
-                _lib.call("rd_rmsnorm", code, _lib.ptr(h), _lib.ptr(self.ln1[l]), _lib.ptr(xn), m_max, md, H, self.eps, st)
+                norm(self.ln1[l], xn, pending)
             kc, vc = cache_tensor[l, 0], cache_tensor[l, 1]
             if fused_rope:
                 # rotary embedding and the cache append ride on the projection's epilogue
@@ -371,11 +384,11 @@ class LlamaForCausalLM(LMHead, nn.Module):
                 else:
                     lin["down"][l](act, h, _lib.EPI_RES, residual=h, m_dev=m_dev, m_max=m_max, status=self.gemm_status)
                 continue
-            lin["o"][l](attn, h, _lib.EPI_RES, residual=h, m_dev=m_dev, m_max=m_max, status=self.gemm_status)
-            _lib.call("rd_rmsnorm", code, _lib.ptr(h), _lib.ptr(self.ln2[l]), _lib.ptr(xn), m_max, md, H, self.eps, st)
+            pending = lin["o"][l].add_residual(attn, h, h, m_dev, m_max, self.gemm_status, parts)
+            norm(self.ln2[l], xn, pending)
             lin["gu"][l](xn, act, _lib.EPI_SWIGLU, m_dev=m_dev, m_max=m_max, status=self.gemm_status)
-            lin["down"][l](act, h, _lib.EPI_RES, residual=h, m_dev=m_dev, m_max=m_max, status=self.gemm_status)
-        _lib.call("rd_rmsnorm", code, _lib.ptr(h), _lib.ptr(self.norm), _lib.ptr(ws["hidden"]), m_max, md, H, self.eps, st)
+            pending = lin["down"][l].add_residual(act, h, h, m_dev, m_max, self.gemm_status, parts)
+        norm(self.norm, ws["hidden"], pending)
         return ws["hidden"]
 
     # ----------------------------------------------------------------- reference forward

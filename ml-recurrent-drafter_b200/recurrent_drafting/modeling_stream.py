@@ -46,6 +46,7 @@ class StreamDecoder(LMHead, nn.Module):
     config_class = None
     norm_groups = 1
     positions_are_columns = False  # positions count from each sequence's first real token
+    projections_in_shares = True  # few rows: projections with a residual may cut their sums over K into shares
 
     def __init__(self, config):
         super().__init__()
@@ -234,6 +235,11 @@ class StreamDecoder(LMHead, nn.Module):
             for name, (width, t) in mixers.widest(needs).items():
                 full[name] = torch.empty(cap_m, width, dtype=t, device=dev)
             full.update(self._extra_buffers(cap_m))
+            # shares of the projections with a residual
+            self._prepare()
+            most = max((b.lin[1].shares_bytes(min(cap_m, Linear.MAX_SHARE_ROWS)) for _, l in self._owners() for b in (l.mixer, l.mlp)
+                        if b is not None and self.projections_in_shares), default=0)
+            full["parts"] = torch.empty(most // 4, dtype=torch.float32, device=dev)
         if logit_rows > cap_l:
             cap_l = logit_rows
             full["logits"] = torch.empty(cap_l, self.config.vocab_size, dtype=torch.float32, device=dev)
@@ -241,7 +247,7 @@ class StreamDecoder(LMHead, nn.Module):
             self._ws_full, self._ws_cap = full, (cap_m, cap_l)
             self._ws = {}
             self._drop_plans()
-        ws = {k: (v[:logit_rows] if k == "logits" else v if k in extra else v[:m_max]) for k, v in full.items()}
+        ws = {k: (v[:logit_rows] if k == "logits" else v if k in extra or k == "parts" else v[:m_max]) for k, v in full.items()}
         if len(self._ws) >= 16:
             self._ws.pop(next(iter(self._ws)))
         self._ws[key] = ws
@@ -258,6 +264,8 @@ class StreamDecoder(LMHead, nn.Module):
         self._prepare()
         ctx = mixers.StepContext(m_max, m_dev, tok_row, tok_pos, tok_slot, row_start, kv_begin, base_len, batch, max_new, max_kv,
                                  mode, tree_mask, mask_words, n_pos, self.gemm_status, ws)
+        if self.projections_in_shares and layer_outputs is None and ws["parts"].numel():
+            ctx.parts = ws["parts"]
         self._run_layers(ctx, cache, tok_ids, layer_outputs)
         return ws["hidden"]
 
@@ -265,6 +273,12 @@ class StreamDecoder(LMHead, nn.Module):
               coeff: Optional[torch.Tensor] = None, n_hist: int = 1, hist_stride: int = 0, ids=None, scale: float = 1.0) -> None:
         """y = norm(x) * weight in the model's dtype, with x a row of src, a weighted sum of n_hist rows hist_stride apart, or
         (ids given) a scaled embedding; x_out, when given, receives x."""
+        pending, ctx.pending = ctx.pending, None
+        if pending is not None:
+            _lib.call("rd_stream_norm_shares", _lib.dtype_code(self.dtype), _lib.ptr(src), hist_stride, _lib.ptr(coeff), n_hist,
+                      _lib.ptr(pending.residual), _lib.ptr(pending.parts), pending.k, _lib.ptr(x_out), _lib.ptr(weight), _lib.ptr(y),
+                      ctx.m_max, _lib.ptr(ctx.m_dev), self.config.hidden_size, self.norm_groups, self.config.norm_eps, _lib.stream())
+            return
         _lib.call("rd_stream_norm", _lib.dtype_code(self.dtype), _lib.ptr(self.embed_tokens.weight) if ids is not None else None,
                   _lib.ptr(ids), scale, _lib.ptr(src), hist_stride, _lib.ptr(coeff), n_hist, _lib.ptr(x_out), _lib.ptr(weight), _lib.ptr(y),
                   ctx.m_max, _lib.ptr(ctx.m_dev), self.config.hidden_size, self.norm_groups, self.config.norm_eps, _lib.stream())

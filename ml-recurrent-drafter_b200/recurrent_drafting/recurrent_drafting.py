@@ -133,7 +133,8 @@ class _StepGraphs:
         _lib.launches = before
         self.draft, self.verify, self.accept = graphs
         # the captured kernels address these: they stay alive even if a larger request makes the model replace them
-        self.buffers = getattr(model.llm, "held_buffers", lambda: [])()
+        rows = st.kv_begin.shape[0] * beam_shape.width * beam_shape.length
+        self.buffers = (model.llm.workspace(rows, rows), getattr(model.llm, "held_buffers", lambda: [])())
         self.ready = True
 
 
