@@ -351,6 +351,14 @@ RD_API int rd_attention_tc_split(const void* plan, void* out, const int32_t* row
                           const int32_t* base_len, int max_new, int mode, const uint32_t* tree_mask, int mask_words,
                           int n_split, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
 
+/* rd_attention's mode RD_ATTN_DENSE on the same plans: mask_bits [m, words] 64-bit words, word w of new token t = its keys
+ * 64 w .. 64 w + 63 (rd_mask_bits packs them from bytes; words * 64 covers base_len + new tokens of every row).  Probabilities
+ * enter the second product as the sum of two bf16 numbers.  n_split and workspace as in rd_attention_tc_split. */
+RD_API int rd_mask_bits(const uint8_t* mask, int64_t ld, int rows, int cols, void* bits, int words, void* stream);
+RD_API int rd_attention_tc_dense(const void* plan, void* out, const int32_t* row_start, const int32_t* kv_begin,
+                          const int32_t* base_len, int max_new, const void* mask_bits, int words, int n_split, void* workspace,
+                          int64_t workspace_bytes, int32_t* status, void* stream);
+
 /* argmax_v logits[t, v], first maximal index (torch.argmax, recurrent_drafting.py:52), written
  * to out32 [M] and/or out64 [M] (either may be NULL). */
 RD_API int rd_argmax_rows(const float* logits, int64_t ld, int m_max, const int32_t* m_dev, int V, int32_t* out32,

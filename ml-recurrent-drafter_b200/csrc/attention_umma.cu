@@ -19,6 +19,9 @@
 //               FFMA + ex2.approx, P written back to TMEM with tcgen05.st.  O accumulates in TMEM
 //               across tiles; a warp rescales its O rows (tcgen05.ld / st) only on the tiles where
 //               one of its rows' running max moved.
+// DENSE: an explicit mask, one 64-bit word per row and key tile.  The kernel that serves these calls on the CUDA cores keeps
+// its probabilities in fp32, so here P goes to the tensor cores as the sum of two bf16 numbers, in the two buffers (a tile's P
+// then waits for PV of the tile before it).
 // QK of tile t+1 overlaps the softmax and PV of tile t; P is double-buffered in TMEM so that the
 // softmax of tile t does not wait for PV of tile t-1 before writing P; two CTAs fit on an SM (105 KB
 // of shared memory, 256 TMEM columns each) and overlap each other's latencies.  With the shared key features a CTA holds
@@ -209,7 +212,7 @@ struct WindowArgs {
   const float* sink;          // optional [nh]
 };
 
-template <bool WIN, int QB>
+template <bool WIN, int QB, bool DENSE>
 __global__ void __launch_bounds__(kThreads, 2)
     attention_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                           const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_t,
@@ -409,7 +412,12 @@ __global__ void __launch_bounds__(kThreads, 2)
           // V: keys are the K dimension (rows of 128 bytes), head_dim the MN dimension: two 64-wide
           // halves kSubTile bytes apart, 8-key groups 1024 bytes apart; 16 keys per MMA = 2048 bytes
           const uint64_t dv = desc_mn_major(smem_u32(v + ks * 2048), kSubTile, 1024);
-          umma_ts(tO, tP + (t & 1) * 32 + ks * 8, dv, idesc_pv, (t | ks) != 0);
+          if (DENSE) {
+            umma_ts(tO, tP + ks * 8, dv, idesc_pv, (t | ks) != 0);
+            umma_ts(tO, tP + 32 + ks * 8, dv, idesc_pv, 1);
+          } else {
+            umma_ts(tO, tP + (t & 1) * 32 + ks * 8, dv, idesc_pv, (t | ks) != 0);
+          }
         }
         umma_commit(&o_full[t & 1]);  // O holds tile t; its P buffer and V stage are free
       }
@@ -422,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int qi = q0 + r;              // query index within the batch row
     const bool live = qi < n_new;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    if (QB == 2 && mode == RD_ATTN_TREE) {
+    if (QB == 2 && !DENSE && mode == RD_ATTN_TREE) {
       for (int w = 0; w < mask_words; ++w) sMask[r * mask_words + w] = live ? tree_mask[(int64_t)(rs + qi) * mask_words + w] : 0u;
     }
     const uint32_t* my_mask = sMask + r * mask_words;  // written and read by this thread only
@@ -435,6 +443,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     bool ok = true;
     int site = 0;  // which wait gave up (reported in the status word)
     for (int t = 0; ok && t < n_tiles; ++t) {
+      uint64_t dense = 0;  // requested ahead of the wait for the scores
+      if (DENSE && live) dense = reinterpret_cast<const uint64_t*>(tree_mask)[(int64_t)(rs + qi) * mask_words + tile_of(t)];
       if (!mbar_wait(&s_full[t & 1], (t >> 1) & 1, abort_flag)) {
         ok = false;
         site = 1;
@@ -450,7 +460,9 @@ __global__ void __launch_bounds__(kThreads, 2)
       // visibility of the tile's 64 keys for this row as one 64-bit word
       const int j0 = tile_of(t) * BNK;
       uint64_t vis;
-      if (j0 + BNK <= base) {
+      if (DENSE) {
+        vis = dense;
+      } else if (j0 + BNK <= base) {
         vis = ~0ull;  // the whole tile lies in the cached prefix
       } else {
         const int off = j0 - base;  // index of the tile's first key among the new tokens (may be negative)
@@ -514,6 +526,11 @@ __global__ void __launch_bounds__(kThreads, 2)
         rowsum0 += p0;
         rowsum1 += p1;
         pb[i] = pack_bf16(p0, p1);
+        if (DENSE) {
+          // what the rounding to bf16 left
+          sb[2 * i] = __float_as_uint(p0 - __uint_as_float(pb[i] << 16));
+          sb[2 * i + 1] = __float_as_uint(p1 - __uint_as_float(pb[i] & 0xffff0000u));
+        }
       }
       l_run = l_run * (moved ? alpha : 1.0f) + (rowsum0 + rowsum1);
       // P buffer t&1 was last read by PV of tile t-2, seen complete before this warp's arrival for tile t-1
@@ -535,7 +552,20 @@ __global__ void __launch_bounds__(kThreads, 2)
           tmem_st32(lane_addr + kColO + c * 32, ob);
         }
       }
-      tmem_st32(lane_addr + kColP + (t & 1) * 32, pb);
+      if (DENSE) {
+        if (t >= 1 && !mbar_wait(&o_full[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag)) {
+          ok = false;
+          site = 6;
+          break;
+        }
+        tc_fence_after();
+        tmem_st32(lane_addr + kColP, pb);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pb[i] = pack_bf16(__uint_as_float(sb[2 * i]), __uint_as_float(sb[2 * i + 1]));
+        tmem_st32(lane_addr + kColP + 32, pb);
+      } else {
+        tmem_st32(lane_addr + kColP + (t & 1) * 32, pb);
+      }
       tc_fence_before();
       // The arrival for tile t must not be possible before the MMA thread has consumed the barrier's
       // phase for tile t-1: the thread issues QK of tile t before it looks at that phase, so without
@@ -603,6 +633,18 @@ __global__ void __launch_bounds__(kThreads, 2)
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
+}
+
+// A mask of bytes [rows, cols] (non-zero = visible) as 64-bit words, bit j of word w = column 64 w + j; one warp per word.
+__global__ void __launch_bounds__(256) mask_bits_kernel(const uint8_t* mask, int64_t ld, int rows, int cols, uint64_t* bits, int words) {
+  const int64_t unit = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (unit >= (int64_t)rows * words) return;
+  const int64_t row = unit / words;
+  const int c = (int)(unit % words) * 64 + lane;
+  const uint32_t lo = __ballot_sync(0xffffffffu, c < cols && mask[row * ld + c] != 0);
+  const uint32_t hi = __ballot_sync(0xffffffffu, c + 32 < cols && mask[row * ld + c + 32] != 0);
+  if (lane == 0) bits[unit] = ((uint64_t)hi << 32) | lo;
 }
 
 // Merge of the shares of a split launch: out = sum_s O_s 2^(m_s - m) / sum_s l_s 2^(m_s - m).
@@ -701,7 +743,8 @@ static int attention_tc_launch(const void* plan, void* out, const int32_t* row_s
                                int n_split, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream,
                                const WindowArgs* win, float scale) {
   RD_REQUIRE(plan && out && row_start && kv_begin && base_len, RD_ERR_ARG);
-  RD_REQUIRE(mode == RD_ATTN_CAUSAL || (mode == RD_ATTN_TREE && tree_mask && mask_words >= 1 && mask_words <= kMaxMaskWords),
+  RD_REQUIRE(mode == RD_ATTN_CAUSAL || (mode == RD_ATTN_TREE && tree_mask && mask_words >= 1 && mask_words <= kMaxMaskWords) ||
+                 (mode == RD_ATTN_DENSE && tree_mask && mask_words >= 1),
              RD_ERR_ARG);
   RD_REQUIRE(max_new >= 1 && n_split >= 1 && n_split <= RD_ATTN_MAX_SPLIT, RD_ERR_SIZE);
   RD_REQUIRE(((uintptr_t)out & 15) == 0, RD_ERR_ALIGN);
@@ -712,10 +755,13 @@ static int attention_tc_launch(const void* plan, void* out, const int32_t* row_s
     RD_REQUIRE(workspace_bytes >= rd_attention_split_workspace_bytes(p->m_max, p->nh, n_split), RD_ERR_CAPACITY);
   }
   RD_REQUIRE(!p->tail || (win && n_split == 1 && mode == RD_ATTN_CAUSAL), RD_ERR_UNSUPPORTED);
-  const int which = p->tail ? 2 : (win ? 1 : 0);
-  auto kern = p->tail ? attention_umma_kernel<true, 3> : (win ? attention_umma_kernel<true, 2> : attention_umma_kernel<false, 2>);
+  const int which = p->tail ? 2 : (win ? 1 : (mode == RD_ATTN_DENSE ? 3 : 0));
+  auto kern = which == 2   ? attention_umma_kernel<true, 3, false>
+              : which == 1 ? attention_umma_kernel<true, 2, false>
+              : which == 3 ? attention_umma_kernel<false, 2, true>
+                           : attention_umma_kernel<false, 2, false>;
   const int smem = p->tail ? Layout<3>::kBytes : Layout<2>::kBytes;
-  static bool smem_set[3] = {false, false, false};  // set once each, so that steady-state launches are pure launches
+  static bool smem_set[4] = {false, false, false, false};  // set once each, so that steady-state launches are pure launches
   if (!smem_set[which]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     RD_CHECK_CHAINED(e);
@@ -742,13 +788,34 @@ extern "C" int64_t rd_attention_split_workspace_bytes(int m_max, int nh, int n_s
 extern "C" int rd_attention_tc(const void* plan, void* out, const int32_t* row_start, const int32_t* kv_begin,
                                const int32_t* base_len, int max_new, int mode, const uint32_t* tree_mask, int mask_words,
                                int32_t* status, void* stream) {
+  RD_REQUIRE(mode != RD_ATTN_DENSE, RD_ERR_ARG);
   return attention_tc_launch(plan, out, row_start, kv_begin, base_len, max_new, mode, tree_mask, mask_words, 1, nullptr, 0,
                              status, stream, nullptr, 1.0f / sqrtf((float)HD));
+}
+
+extern "C" int rd_mask_bits(const uint8_t* mask, int64_t ld, int rows, int cols, void* bits, int words, void* stream) {
+  RD_REQUIRE(mask && bits, RD_ERR_ARG);
+  RD_REQUIRE(rows >= 1 && cols >= 1 && ld >= cols && words == (cols + 63) / 64, RD_ERR_SIZE);
+  RD_REQUIRE(((uintptr_t)bits & 7) == 0, RD_ERR_ALIGN);
+  const int64_t blocks = ((int64_t)rows * words + 7) / 8;
+  RD_REQUIRE(blocks <= 0x7fffffff, RD_ERR_SIZE);
+  mask_bits_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(mask, ld, rows, cols, (uint64_t*)bits, words);
+  RD_CHECK_LAUNCH();
+  return RD_OK;
+}
+
+extern "C" int rd_attention_tc_dense(const void* plan, void* out, const int32_t* row_start, const int32_t* kv_begin,
+                                     const int32_t* base_len, int max_new, const void* mask_bits, int words, int n_split,
+                                     void* workspace, int64_t workspace_bytes, int32_t* status, void* stream) {
+  RD_REQUIRE(((uintptr_t)mask_bits & 7) == 0, RD_ERR_ALIGN);
+  return attention_tc_launch(plan, out, row_start, kv_begin, base_len, max_new, RD_ATTN_DENSE, (const uint32_t*)mask_bits, words, n_split,
+                             workspace, workspace_bytes, status, stream, nullptr, 1.0f / sqrtf((float)HD));
 }
 
 extern "C" int rd_attention_tc_split(const void* plan, void* out, const int32_t* row_start, const int32_t* kv_begin,
                                      const int32_t* base_len, int max_new, int mode, const uint32_t* tree_mask, int mask_words,
                                      int n_split, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream) {
+  RD_REQUIRE(mode != RD_ATTN_DENSE, RD_ERR_ARG);
   return attention_tc_launch(plan, out, row_start, kv_begin, base_len, max_new, mode, tree_mask, mask_words, n_split, workspace,
                              workspace_bytes, status, stream, nullptr, 1.0f / sqrtf((float)HD));
 }
@@ -761,7 +828,7 @@ extern "C" int rd_attention_tc_masked(const void* plan, void* out, const int32_t
   // the kernel's running maximum is taken before the scale, and a tree's own tokens must all be visible by position
   RD_REQUIRE(mask_kind == RD_MASK_WINDOW || (mask_kind == RD_MASK_CHUNK && mode == RD_ATTN_CAUSAL), RD_ERR_UNSUPPORTED);
   RD_REQUIRE(scale > 0.f && window >= (mode == RD_ATTN_TREE ? RD_MAX_BEAM_LENGTH : 1) && keep_first >= 0, RD_ERR_SIZE);
-  RD_REQUIRE(mode != RD_ATTN_TREE || tok_pos, RD_ERR_ARG);
+  RD_REQUIRE((mode != RD_ATTN_TREE || tok_pos) && mode != RD_ATTN_DENSE, RD_ERR_ARG);
   const WindowArgs win{mask_kind, window, keep_first, (const __nv_bfloat16*)gate, ld_gate, tok_pos, sink};
   return attention_tc_launch(plan, out, row_start, kv_begin, base_len, max_new, mode, tree_mask, mask_words, 1, nullptr, 0, status,
                              stream, &win, scale);

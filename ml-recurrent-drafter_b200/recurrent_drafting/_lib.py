@@ -61,6 +61,8 @@ SIGNATURES = {
     "rd_gemm_bf16_tc_res_shares": (_I, [_P, _I, _P, _L, _P, _L, _P, _P, _L, _P, _P]),
     "rd_rmsnorm_shares": (_I, [_I, _P, _P, _P, _I, _P, _P, _I, _P, _I, _F, _P]),
     "rd_stream_norm_shares": (_I, [_I, _P, _L, _P, _I, _P, _P, _I, _P, _P, _P, _I, _P, _I, _I, _F, _P]),
+    "rd_mask_bits": (_I, [_P, _L, _I, _I, _P, _I, _P]),
+    "rd_attention_tc_dense": (_I, [_P, _P, _P, _P, _P, _I, _P, _I, _I, _P, _L, _P, _P]),
     "rd_rmsnorm": (_I, [_I, _P, _P, _P, _I, _P, _I, _F, _P]),
     "rd_rope_kv_write": (_I, [_I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _P, _I, _I, _I, _I, _P]),
     "rd_attention": (_I, [_I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _L, _L, _P]),

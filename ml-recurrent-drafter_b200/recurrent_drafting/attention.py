@@ -34,6 +34,9 @@ def bias(causal_mask: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 
 
 ATTN_MAX_SPLIT = 16
+# keys up to which an explicit mask is served at heads of 128 features: the CUDA-core kernel keeps 8 rows of scores in
+# 220 KB of shared memory, and longer calls are refused there
+DENSE_MAX_KEYS = 220 * 1024 // 32 - 128
 
 
 def key_range_shares(batch: int, n_heads: int, max_new: int, max_kv: int, n_sm: int = 148) -> int:

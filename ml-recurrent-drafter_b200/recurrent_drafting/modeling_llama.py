@@ -232,10 +232,10 @@ class LlamaForCausalLM(LMHead, nn.Module):
             pass
 
     def _attention(self, code, q, kc, vc, attn, row_start, kv_begin, base_len, batch, m_max, max_new, max_kv, mode, tree_mask,
-                   mask_words, dense_mask, dld_q, dld_b, st):
+                   mask_words, dense_mask, dld_q, dld_b, dense_bits, st):
         nh, nkv, hd = self.n_heads, self.n_kv_heads, self.head_dim
         max_len = kc.shape[2]
-        if self.dtype == torch.bfloat16 and hd == 128 and mode != _lib.ATTN_DENSE and mask_words <= 16:
+        if self.dtype == torch.bfloat16 and hd == 128 and (mode != _lib.ATTN_DENSE or dense_bits is not None) and mask_words <= 16:
             # tcgen05 path: TMA descriptors are tied to these exact buffers
             key = (q.data_ptr(), m_max, kc.data_ptr(), vc.data_ptr(), batch, max_len)
             plan = self._attn_plans.get(key)
@@ -252,6 +252,11 @@ class LlamaForCausalLM(LMHead, nn.Module):
                 need = _lib.load().rd_attention_split_workspace_bytes(m_max, nh, shares)
                 if self._attn_split_ws is None or self._attn_split_ws.numel() < need:
                     self._attn_split_ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+            if dense_bits is not None:
+                _lib.call("rd_attention_tc_dense", plan, _lib.ptr(attn), _lib.ptr(row_start), _lib.ptr(kv_begin), _lib.ptr(base_len),
+                          max_new, _lib.ptr(dense_bits), dense_bits.shape[1], shares, _lib.ptr(self._attn_split_ws) if shares > 1 else None,
+                          self._attn_split_ws.numel() if shares > 1 else 0, _lib.ptr(self.gemm_status), st)
+            elif shares > 1:
                 _lib.call("rd_attention_tc_split", plan, _lib.ptr(attn), _lib.ptr(row_start), _lib.ptr(kv_begin), _lib.ptr(base_len),
                           max_new, mode, _lib.ptr(tree_mask), mask_words, shares, _lib.ptr(self._attn_split_ws),
                           self._attn_split_ws.numel(), _lib.ptr(self.gemm_status), st)
@@ -342,6 +347,12 @@ class LlamaForCausalLM(LMHead, nn.Module):
         _lib.call("rd_embed_gather", code, _lib.ptr(self.model.embed_tokens.weight), _lib.ptr(tok_ids), _lib.ptr(h), m_max, md, H, st)
         dld_q = dense_mask.stride(1) if dense_mask is not None else 0
         dld_b = dense_mask.stride(0) if dense_mask is not None else 0
+        dense_bits = None
+        if (mode == _lib.ATTN_DENSE and self.dtype == torch.bfloat16 and hd == 128 and max_kv <= attention.DENSE_MAX_KEYS
+                and dense_mask.is_contiguous()):
+            # the mask in bits, once for all layers
+            dense_bits = torch.empty(m_max, (max_kv + 63) // 64, dtype=torch.int64, device=h.device)
+            _lib.call("rd_mask_bits", _lib.ptr(dense_mask), dld_q, m_max, max_kv, _lib.ptr(dense_bits), dense_bits.shape[1], st)
         fused_rope = (self.dtype == torch.bfloat16 and hd == 128 and H % 64 == 0 and xn.data_ptr() % 16 == 0
                       and os.environ.get("RD_FUSED_ROPE", "1") != "0")
         # RMS norms between the projections folded into them (RD_FUSED_NORM=1): o_proj / down_proj also write the
@@ -375,7 +386,7 @@ class LlamaForCausalLM(LMHead, nn.Module):
                           _lib.ptr(tok_pos), _lib.ptr(tok_slot), _lib.ptr(cos), _lib.ptr(sin), cos.shape[0], m_max, md, nh, nkv,
                           hd, max_len, st)
             self._attention(code, q, kc, vc, attn, row_start, kv_begin, base_len, batch, m_max, max_new, max_kv, mode, tree_mask,
-                            mask_words, dense_mask, dld_q, dld_b, st)
+                            mask_words, dense_mask, dld_q, dld_b, dense_bits, st)
             if fused_norm:
                 lin["o"][l].residual_with_norm(attn, h, h, self.ln2[l], xn, ss, m_dev, m_max, self.gemm_status)
                 lin["gu"][l].swiglu_normed(xn, act, ss, H, self.eps, m_dev, m_max, self.gemm_status)
