@@ -56,7 +56,19 @@ __global__ void __launch_bounds__(kQPB * 32) attention_rowwise_kernel(
     if (vis) {
       const T* kr = kbase + (int64_t)j * hd;
       float acc = 0.f;
-      for (int d = 0; d < hd; ++d) acc = fmaf(qs[d], rd::Num<T>::to_f(kr[d]), acc);
+      int d = 0;
+      // whole 16-byte pieces of the key, several in flight (the order of the sum stays that of the features)
+      if ((((uintptr_t)kr | (uintptr_t)(hd * sizeof(T))) & 15) == 0) {
+        constexpr int VEC = 16 / sizeof(T);
+#pragma unroll 8
+        for (; d + VEC <= hd; d += VEC) {
+          const uint4 u = *reinterpret_cast<const uint4*>(kr + d);
+          const T* e = reinterpret_cast<const T*>(&u);
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) acc = fmaf(qs[d + i], rd::Num<T>::to_f(e[i]), acc);
+        }
+      }
+      for (; d < hd; ++d) acc = fmaf(qs[d], rd::Num<T>::to_f(kr[d]), acc);
       s = acc * scale;
     }
     sc[j] = s;
@@ -76,9 +88,11 @@ __global__ void __launch_bounds__(kQPB * 32) attention_rowwise_kernel(
   T* orow = out + ((int64_t)t * nh + h) * hd;
   for (int d = lane; d < hd; d += 32) {
     float acc = 0.f;
+    // the values are read whether they count or not, so that eight of them are in flight
+#pragma unroll 8
     for (int j = 0; j < kv; ++j) {
-      const float p = sc[j];
-      if (p != 0.f) acc = fmaf(p, rd::Num<T>::to_f(vbase[(int64_t)j * hd + d]), acc);
+      const float p = sc[j], v = rd::Num<T>::to_f(vbase[(int64_t)j * hd + d]);
+      acc = p != 0.f ? fmaf(p, v, acc) : acc;
     }
     orow[d] = rd::Num<T>::from_f(acc * inv);
   }

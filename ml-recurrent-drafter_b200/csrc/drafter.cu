@@ -562,6 +562,11 @@ extern "C" int rd_drafter_prepare(int dtype, const void* embed, const int64_t* b
   return RD_OK;
 }
 
+// 16-byte loads only where they leave every thread at least one element: the bound on the K-th largest value comes from the
+// warps' four largest thread maxima, and with 250 loads for a row of 1000 half of the warps had none, the bound was -inf and
+// all 1000 elements were ranked against each other (117 us a launch; with one element per load 9 us).
+static bool vec_fills_block(int V, int vec) { return V / vec >= kTopkThreads; }
+
 static int vocab_topk_launch(int logits_dtype, const void* logits, int64_t ld, int rows_max, const int32_t* rows_dev, int V,
                              int top_k, float mask_value, int subtract_max, float temperature, const float* slice_max,
                              int64_t slice_ld, float* kept_val, int32_t* kept_idx, int32_t* kept_cnt, float* masked_logp,
@@ -577,12 +582,12 @@ static int vocab_topk_launch(int logits_dtype, const void* logits, int64_t ld, i
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t err = cudaSuccess;
   if (logits_dtype == RD_F32) {
-    const int vec_ok = ((uintptr_t)logits % 16 == 0) && ((ld * 4) % 16 == 0);
+    const int vec_ok = vec_fills_block(V, 4) && ((uintptr_t)logits % 16 == 0) && ((ld * 4) % 16 == 0);
     err = rd::launch_chained(vocab_topk_kernel<float>, dim3(rows_max), dim3(kTopkThreads), 0, s, 1, (const float*)logits, ld, rows_max,
                              rows_dev, V, top_k, mask_value, subtract_max, temperature, vec_ok, slice_max, slice_ld, kept_val, kept_idx,
                              kept_cnt, masked_logp);
   } else if (logits_dtype == RD_BF16) {
-    const int vec_ok = ((uintptr_t)logits % 16 == 0) && ((ld * 2) % 16 == 0);
+    const int vec_ok = vec_fills_block(V, 8) && ((uintptr_t)logits % 16 == 0) && ((ld * 2) % 16 == 0);
     err = rd::launch_chained(vocab_topk_kernel<__nv_bfloat16>, dim3(rows_max), dim3(kTopkThreads), 0, s, 1,
                              (const __nv_bfloat16*)logits, ld, rows_max, rows_dev, V, top_k, mask_value, subtract_max, temperature,
                              vec_ok, slice_max, slice_ld, kept_val, kept_idx, kept_cnt, masked_logp);
