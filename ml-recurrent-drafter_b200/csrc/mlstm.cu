@@ -136,24 +136,37 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
       } else {
         const bool zero = fresh && it == 0;
         float* sp = S_g + tc * VEC;
-#pragma unroll 8
-        for (int r = tr; r < dim; r += rows_par) {
-          const float kk = k_s[r], qq = q_s[r];
-          float s[VEC];
-          if constexpr (VEC == 4) {
-            *reinterpret_cast<float4*>(s) = zero ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(sp + (int64_t)r * vdim);
-          } else {
-            s[0] = zero ? 0.f : sp[(int64_t)r * vdim];
+        // Eight rows are read before the first of them is written: a load may not pass a store that could be to the same
+        // place, so reading and writing row by row was one trip to memory after the other.  6 rows, 8 heads of 256 x 512, one
+        // B200: 30 -> 23.5 us.
+        constexpr int U = 8;
+        for (int r0 = tr; r0 < dim; r0 += rows_par * U) {
+          float s[U][VEC];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int r = r0 + u * rows_par;
+            const bool read = r < dim && !zero;
+            if constexpr (VEC == 4) {
+              *reinterpret_cast<float4*>(s[u]) = read ? *reinterpret_cast<const float4*>(sp + (int64_t)r * vdim) : make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+              s[u][0] = read ? sp[(int64_t)r * vdim] : 0.f;
+            }
           }
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) {
-            s[e] = fmaf(fa, s[e], kk * v[e]);
-            o[e] = fmaf(s[e], qq, o[e]);
-          }
-          if constexpr (VEC == 4) {
-            *reinterpret_cast<float4*>(sp + (int64_t)r * vdim) = *reinterpret_cast<const float4*>(s);
-          } else {
-            sp[(int64_t)r * vdim] = s[0];
+          for (int u = 0; u < U; ++u) {
+            const int r = r0 + u * rows_par;
+            if (r >= dim) break;
+            const float kk = k_s[r], qq = q_s[r];
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+              s[u][e] = fmaf(fa, s[u][e], kk * v[e]);
+              o[e] = fmaf(s[u][e], qq, o[e]);
+            }
+            if constexpr (VEC == 4) {
+              *reinterpret_cast<float4*>(sp + (int64_t)r * vdim) = *reinterpret_cast<const float4*>(s[u]);
+            } else {
+              sp[(int64_t)r * vdim] = s[u][0];
+            }
           }
         }
       }
