@@ -658,7 +658,8 @@ __global__ void __launch_bounds__(HD) attention_merge_kernel(const float* partia
   float acc = 0.f, l = 0.f;
   for (int s = 0; s < n_split; ++s) {
     const float ms = p[s * (HD + 2) + HD];
-    const float w = (ms == -INFINITY) ? 0.f : exp2f(ms - m);
+    if (ms == -INFINITY) continue;  // a share without keys has written no O
+    const float w = exp2f(ms - m);
     acc += w * p[s * (HD + 2) + d];
     l += w * p[s * (HD + 2) + HD + 1];
   }
