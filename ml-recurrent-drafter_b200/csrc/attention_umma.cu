@@ -19,7 +19,10 @@
 //               FFMA + ex2.approx, P written back to TMEM with tcgen05.st.  O accumulates in TMEM
 //               across tiles; a warp rescales its O rows (tcgen05.ld / st) only on the tiles where
 //               one of its rows' running max moved.
-// DENSE: an explicit mask, one 64-bit word per row and key tile.  The kernel that serves these calls on the CUDA cores keeps
+// kHeads: one new token per row and several query heads to a key/value head (a decode step).  The rows of a CTA's query tile are
+// then the heads that share its keys, not the one token of a single head: the keys are read once per key/value head, and the
+// launch has nkv chains instead of nh.
+// kDense: an explicit mask, one 64-bit word per row and key tile.  The kernel that serves these calls on the CUDA cores keeps
 // its probabilities in fp32, so here P goes to the tensor cores as the sum of two bf16 numbers, in the two buffers (a tile's P
 // then waits for PV of the tile before it).
 // QK of tile t+1 overlaps the softmax and PV of tile t; P is double-buffered in TMEM so that the
@@ -69,6 +72,7 @@ struct Places {
 
 struct AttnPlan {
   CUtensorMap map_q;  // [m_max, nh * q_col] box 64 x 128
+  CUtensorMap map_qh; // the same memory as [m_max * nh, 128] (plans without a tail)
   CUtensorMap map_k;  // box 64 x 64
   CUtensorMap map_v;
   CUtensorMap map_t;  // shared key features (tail plans)
@@ -212,7 +216,9 @@ struct WindowArgs {
   const float* sink;          // optional [nh]
 };
 
-template <bool WIN, int QB, bool DENSE>
+enum Form { kPlain, kDense, kHeads };
+
+template <bool WIN, int QB, Form FORM>
 __global__ void __launch_bounds__(kThreads, 2)
     attention_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                           const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_t,
@@ -222,7 +228,9 @@ __global__ void __launch_bounds__(kThreads, 2)
                           const uint32_t* tree_mask, int mask_words, float scale_log2, int32_t* status,
                           int n_split, float* partial, const WindowArgs win) {
   using L = Layout<QB>;
-  const int b = blockIdx.z, h = blockIdx.y;
+  constexpr bool DENSE = FORM == kDense, HEADS = FORM == kHeads;
+  const int group = nh / nkv;
+  const int b = blockIdx.z, h = HEADS ? (int)blockIdx.y * group : (int)blockIdx.y;  // HEADS: the first of the heads
   rd::pdl_launch_dependents();
   if (threadIdx.x == 0) {
     if (QB == 3) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_t) : "memory");
@@ -259,7 +267,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int base = base_len[b];
-  const int hk = h / (nh / nkv);
+  const int hk = h / group;
   const int kv_end = (mode == RD_ATTN_CAUSAL) ? base + min(n_new, q0 + BMQ) : base + n_new;
   int all_tiles = (kv_end + BNK - 1) / BNK;
   int kept_tiles = 0, first_tile = 0;  // WIN: tiles of the kept tokens, then [first_tile, end)
@@ -274,9 +282,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int n_tiles = max(0, min(per_split, all_tiles - t_begin));
   if (n_split > 1 && n_tiles == 0) {
     // nothing to do for this share: leave an empty partial (max = -inf, sum = 0) for the merge
-    const int r = (int)threadIdx.x, qi = q0 + r;
-    if (r < BMQ && qi < n_new) {
-      float* ml = partial + (((int64_t)(rs + qi) * nh + h) * n_split + split) * (HD + 2) + HD;
+    const int r = (int)threadIdx.x, qi = HEADS ? 0 : q0 + r;
+    if (r < BMQ && (HEADS ? r < group : qi < n_new)) {
+      float* ml = partial + (((int64_t)(rs + qi) * nh + h + (HEADS ? r : 0)) * n_split + split) * (HD + 2) + HD;
       ml[0] = -INFINITY;
       ml[1] = 0.f;
     }
@@ -321,7 +329,11 @@ __global__ void __launch_bounds__(kThreads, 2)
     // life waiting for this first data.
     mbar_expect_tx(q_full, L::kQBytes);
 #pragma unroll
-    for (int i = 0; i < QB; ++i) tma_load_2d(sQ + i * BMQ * 128, &map_q, q_full, h * at.q_col + 64 * i, rs + q0);
+    for (int i = 0; i < QB; ++i) {
+      // HEADS: the queries as rows of one head each; rows past the group are other heads' and come to nothing
+      if (HEADS) tma_load_2d(sQ + i * BMQ * 128, &map_q, q_full, 64 * i, rs * nh + h);
+      else tma_load_2d(sQ + i * BMQ * 128, &map_q, q_full, h * at.q_col + 64 * i, rs + q0);
+    }
     for (int t = 0; t < L::kKStages && t < n_tiles; ++t) load_k(t, &k_full[t]);
     for (int t = 0; t < L::kVStages && t < n_tiles; ++t) load_v(t, &v_full[t]);
   }
@@ -427,8 +439,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     // ---------------- softmax: thread <-> query row ----------------
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;  // row of the tile = TMEM lane
-    const int qi = q0 + r;              // query index within the batch row
-    const bool live = qi < n_new;
+    const int qi = HEADS ? 0 : q0 + r;  // query index within the batch row
+    const int hq = HEADS ? h + r : h;
+    const bool live = HEADS ? r < group : qi < n_new;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     if (QB == 2 && !DENSE && mode == RD_ATTN_TREE) {
       for (int w = 0; w < mask_words; ++w) sMask[r * mask_words + w] = live ? tree_mask[(int64_t)(rs + qi) * mask_words + w] : 0u;
@@ -587,7 +600,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (ok && n_split > 1) {
       // partial result of this share: unnormalised O (relative to m_run), then m_run and l_run
       tc_fence_after();
-      float* dstp = partial + (((int64_t)(rs + qi) * nh + h) * n_split + split) * (HD + 2);
+      float* dstp = partial + (((int64_t)(rs + qi) * nh + hq) * n_split + split) * (HD + 2);
 #pragma unroll 1
       for (int c = 0; c < HD / 32; ++c) {
         uint32_t ob[32];
@@ -606,7 +619,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       tc_fence_after();
       float inv = WIN ? rd_win::finish_softmax(m_run, l_run, win.sink, h) : (l_run > 0.f ? 1.0f / l_run : 0.f);
       if (WIN && win.gate != nullptr && live) inv /= 1.0f + __expf(-__bfloat162float(win.gate[(int64_t)(rs + qi) * win.ld_gate + h]));
-      uint4* dst = reinterpret_cast<uint4*>(out + ((int64_t)(rs + qi) * nh + h) * HD);
+      uint4* dst = reinterpret_cast<uint4*>(out + ((int64_t)(rs + qi) * nh + hq) * HD);
 #pragma unroll 1
       for (int c = 0; c < HD / 32; ++c) {
         uint32_t ob[32];
@@ -651,6 +664,8 @@ __global__ void __launch_bounds__(256) mask_bits_kernel(const uint8_t* mask, int
 __global__ void __launch_bounds__(HD) attention_merge_kernel(const float* partial, __nv_bfloat16* out,
                                                              const int32_t* row_start, int B, int nh, int n_split) {
   const int tok = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
+  rd::pdl_launch_dependents();
+  rd::pdl_wait();
   if (tok >= row_start[B]) return;
   const float* p = partial + ((int64_t)tok * nh + h) * n_split * (HD + 2);
   float m = -INFINITY;
@@ -706,7 +721,7 @@ extern "C" void* rd_attention_plan_create(const void* q, int m_max, const void* 
   p->tail = false;
   p->at = Places{nkv * max_len, max_len, 0, 0, HD};
   const int64_t kv_rows = (int64_t)B * nkv * max_len;
-  if (!make_map(&p->map_q, q, m_max, (int64_t)nh * HD, (int64_t)nh * HD, BMQ) ||
+  if (!make_map(&p->map_q, q, m_max, (int64_t)nh * HD, (int64_t)nh * HD, BMQ) || !make_map(&p->map_qh, q, (int64_t)m_max * nh, HD, HD, BMQ) ||
       !make_map(&p->map_k, k_cache, kv_rows, HD, HD, BNK) || !make_map(&p->map_v, v_cache, kv_rows, HD, HD, BNK)) {
     delete p;
     return nullptr;
@@ -756,27 +771,32 @@ static int attention_tc_launch(const void* plan, void* out, const int32_t* row_s
     RD_REQUIRE(workspace_bytes >= rd_attention_split_workspace_bytes(p->m_max, p->nh, n_split), RD_ERR_CAPACITY);
   }
   RD_REQUIRE(!p->tail || (win && n_split == 1 && mode == RD_ATTN_CAUSAL), RD_ERR_UNSUPPORTED);
-  const int which = p->tail ? 2 : (win ? 1 : (mode == RD_ATTN_DENSE ? 3 : 0));
-  auto kern = which == 2   ? attention_umma_kernel<true, 3, false>
-              : which == 1 ? attention_umma_kernel<true, 2, false>
-              : which == 3 ? attention_umma_kernel<false, 2, true>
-                           : attention_umma_kernel<false, 2, false>;
+  // Heads as rows wherever a group has more than one and there is one token: 24 rows of some 350 keys, 32 heads on 8, one B200:
+  // 31 -> 11 us a layer.
+  const bool heads = !p->tail && !win && mode == RD_ATTN_CAUSAL && max_new == 1 && p->nh > p->nkv && p->nh / p->nkv <= BMQ;
+  const int which = p->tail ? 2 : (win ? 1 : (mode == RD_ATTN_DENSE ? 3 : (heads ? 4 : 0)));
+  auto kern = which == 2   ? attention_umma_kernel<true, 3, kPlain>
+              : which == 1 ? attention_umma_kernel<true, 2, kPlain>
+              : which == 3 ? attention_umma_kernel<false, 2, kDense>
+              : which == 4 ? attention_umma_kernel<false, 2, kHeads>
+                           : attention_umma_kernel<false, 2, kPlain>;
   const int smem = p->tail ? Layout<3>::kBytes : Layout<2>::kBytes;
-  static bool smem_set[4] = {false, false, false, false};  // set once each, so that steady-state launches are pure launches
+  static bool smem_set[5] = {false, false, false, false, false};  // set once each, so that steady-state launches are pure launches
   if (!smem_set[which]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     RD_CHECK_CHAINED(e);
     smem_set[which] = true;
   }
-  dim3 grid(((max_new + BMQ - 1) / BMQ) * n_split, p->nh, p->B);
+  dim3 grid(((max_new + BMQ - 1) / BMQ) * n_split, heads ? p->nkv : p->nh, p->B);
   const float scale_log2 = 1.4426950408889634f * scale;
-  cudaError_t err = rd::launch_chained(kern, grid, dim3(kThreads), smem, (cudaStream_t)stream, 1, p->map_q, p->map_k, p->map_v, p->map_t,
+  cudaError_t err = rd::launch_chained(kern, grid, dim3(kThreads), smem, (cudaStream_t)stream, 1, heads ? p->map_qh : p->map_q, p->map_k, p->map_v, p->map_t,
                                        p->at, (__nv_bfloat16*)out, row_start, kv_begin, base_len, p->nh, p->nkv, mode, tree_mask,
                                        mask_words, scale_log2, status, n_split, (float*)workspace, win ? *win : WindowArgs{});
   RD_CHECK_CHAINED(err);
   if (n_split > 1) {
-    attention_merge_kernel<<<dim3(p->m_max, p->nh), HD, 0, (cudaStream_t)stream>>>((const float*)workspace, (__nv_bfloat16*)out,
-                                                                                 row_start, p->B, p->nh, n_split);
+    err = rd::launch_chained(attention_merge_kernel, dim3(p->m_max, p->nh), dim3(HD), 0, (cudaStream_t)stream, 1, (const float*)workspace,
+                             (__nv_bfloat16*)out, row_start, p->B, p->nh, n_split);
+    RD_CHECK_CHAINED(err);
   }
   RD_CHECK_LAUNCH();
   return RD_OK;

@@ -246,7 +246,8 @@ class LlamaForCausalLM(LMHead, nn.Module):
                 if len(self._attn_plans) >= 4 * self.n_layers:
                     self._drop_attn_plans()
                 self._attn_plans[key] = plan
-            shares = attention.key_range_shares(batch, nh, max_new, max_kv)
+            chains = nkv if max_new == 1 and mode == _lib.ATTN_CAUSAL else nh  # one token: the heads of a group share a chain
+            shares = attention.key_range_shares(batch, chains, max_new, max_kv)
             if shares > 1:
                 # few (row, head) chains and a long cache: several CTAs per chain, merged by a second kernel
                 need = _lib.load().rd_attention_split_workspace_bytes(m_max, nh, shares)
