@@ -23,10 +23,12 @@ __global__ void embed_gather_kernel(const T* table, const int64_t* ids, T* out,
 }
 
 template <typename T, bool SHARES>
-__global__ void __launch_bounds__(256, SHARES ? 4 : 8) rmsnorm_kernel(T* x, const T* w, T* y,
+__global__ void __launch_bounds__(SHARES ? 512 : 256) rmsnorm_kernel(T* x, const T* w, T* y,
                                                       int m_max, const int32_t* m_dev, int H, float eps,
                                                       int vectorised, rd::Shares<T> sh) {
   constexpr int VEC = 16 / sizeof(T);
+  // rows in shares are few and wait for their loads: more threads have more of them in flight
+  constexpr int kThreads = SHARES ? 512 : 256;
   const int t = blockIdx.x;
   rd::pdl_launch_dependents();
   rd::pdl_wait();
@@ -37,7 +39,7 @@ __global__ void __launch_bounds__(256, SHARES ? 4 : 8) rmsnorm_kernel(T* x, cons
   float ss = 0.f;
   const bool shares = SHARES && rd::live_shares(sh.count, M) > 1;
   if (vectorised) {
-    for (int v = threadIdx.x; v < H / VEC; v += 256) {
+    for (int v = threadIdx.x; v < H / VEC; v += kThreads) {
       T e[VEC];
       if (shares) {
         // x is still in shares: formed here, rounded to the model dtype and written before it is normalised
@@ -56,7 +58,7 @@ __global__ void __launch_bounds__(256, SHARES ? 4 : 8) rmsnorm_kernel(T* x, cons
       }
     }
   } else {
-    for (int d = threadIdx.x; d < H; d += 256) {
+    for (int d = threadIdx.x; d < H; d += kThreads) {
       if (shares) {
         float f;
         rd::add_shares<1>(sh, t, H, d, &f);
@@ -66,17 +68,17 @@ __global__ void __launch_bounds__(256, SHARES ? 4 : 8) rmsnorm_kernel(T* x, cons
       ss += v * v;
     }
   }
-  __shared__ float red[8];
+  __shared__ float red[kThreads / 32];
   ss = rd::warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
   float tot = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) tot += red[i];
+  for (int i = 0; i < kThreads / 32; ++i) tot += red[i];
   const float rs = 1.0f / sqrtf(tot / (float)H + eps);
   // normalise in fp32, round to the model dtype, then scale by the weight (as the reference does)
   if (vectorised) {
-    for (int v = threadIdx.x; v < H / VEC; v += 256) {
+    for (int v = threadIdx.x; v < H / VEC; v += kThreads) {
       T e[VEC], g[VEC], o[VEC];
       *reinterpret_cast<uint4*>(e) = reinterpret_cast<const uint4*>(xr)[v];
       *reinterpret_cast<uint4*>(g) = reinterpret_cast<const uint4*>(w)[v];
@@ -88,7 +90,7 @@ __global__ void __launch_bounds__(256, SHARES ? 4 : 8) rmsnorm_kernel(T* x, cons
       reinterpret_cast<uint4*>(yr)[v] = *reinterpret_cast<const uint4*>(o);
     }
   } else {
-    for (int d = threadIdx.x; d < H; d += 256) {
+    for (int d = threadIdx.x; d < H; d += kThreads) {
       T n = rd::Num<T>::from_f(rd::Num<T>::to_f(xr[d]) * rs);
       yr[d] = rd::Num<T>::from_f(rd::Num<T>::to_f(w[d]) * rd::Num<T>::to_f(n));
     }
@@ -311,7 +313,7 @@ static int rmsnorm_launch(int dtype, void* x, const void* weight, void* y, int m
   const int vectorised =
       (H % vec == 0) && (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)y | (uintptr_t)parts | (uintptr_t)residual) % 16 == 0);
   cudaError_t err = cudaSuccess;
-  RD_DISPATCH_T(dtype, (err = rd::launch_chained(shares > 1 ? rmsnorm_kernel<T, true> : rmsnorm_kernel<T, false>, dim3(m_max), dim3(256), 0, s, 1, (T*)x, (const T*)weight,
+  RD_DISPATCH_T(dtype, (err = rd::launch_chained(shares > 1 ? rmsnorm_kernel<T, true> : rmsnorm_kernel<T, false>, dim3(m_max), dim3(shares > 1 ? 512 : 256), 0, s, 1, (T*)x, (const T*)weight,
                                                  (T*)y, m_max, m_dev, H, eps, vectorised,
                                                  rd::Shares<T>{parts, (const T*)residual, shares, m_max < rd::kShareRows ? m_max : rd::kShareRows})));
   RD_CHECK_CHAINED(err);

@@ -150,7 +150,7 @@ __device__ __forceinline__ void add_shares(const Shares<T>& sh, int t, int N, in
   float acc[VEC];
 #pragma unroll
   for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
-#pragma unroll 2
+#pragma unroll 4
   for (int s = 0; s < sh.count; ++s, p += (int64_t)sh.rows * N) {
     if constexpr (VEC == 1) {
       acc[0] += *p;
