@@ -230,7 +230,14 @@ __global__ void __launch_bounds__(kThreads, 2)
   using L = Layout<QB>;
   constexpr bool DENSE = FORM == kDense, HEADS = FORM == kHeads;
   const int group = nh / nkv;
-  const int b = blockIdx.z, h = HEADS ? (int)blockIdx.y * group : (int)blockIdx.y;  // HEADS: the first of the heads
+  // A causal query tile visits the more keys the later it lies.  CTAs start in the order of their index, so the last tiles of all
+  // heads come first and the launch does not end on a few long ones (8192 tokens, 32 heads, one B200: 790 -> 584 us a layer; the
+  // power that it then draws takes a part back from the projections around it).
+  const bool late_first = mode == RD_ATTN_CAUSAL && n_split == 1 && gridDim.x > 1;
+  const int linear = (int)(blockIdx.x + gridDim.x * blockIdx.y);
+  const int bx = late_first ? (int)gridDim.x - 1 - linear / (int)gridDim.y : (int)blockIdx.x;
+  const int by = late_first ? linear % (int)gridDim.y : (int)blockIdx.y;
+  const int b = blockIdx.z, h = HEADS ? by * group : by;  // HEADS: the first of the heads
   rd::pdl_launch_dependents();
   if (threadIdx.x == 0) {
     if (QB == 3) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_t) : "memory");
@@ -242,8 +249,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   rd::pdl_wait();  // row_start, Q and the new K/V rows come from the kernels before this one
   const int rs = row_start[b];
   const int n_new = row_start[b + 1] - rs;
-  const int q0 = ((int)blockIdx.x / n_split) * BMQ;
-  const int split = (int)blockIdx.x % n_split;  // this CTA's share of the key tiles (1 share = the whole row)
+  const int q0 = (bx / n_split) * BMQ;
+  const int split = bx % n_split;  // this CTA's share of the key tiles (1 share = the whole row)
   if (q0 >= n_new) return;
   extern __shared__ __align__(1024) uint8_t smem[];  // the swizzled boxes start at multiples of 1024
   if ((smem_u32(smem) & 1023) != 0) {
