@@ -350,10 +350,11 @@ class LlamaForCausalLM(LMHead, nn.Module):
         dld_b = dense_mask.stride(0) if dense_mask is not None else 0
         dense_bits = None
         if (mode == _lib.ATTN_DENSE and self.dtype == torch.bfloat16 and hd == 128 and max_kv <= attention.DENSE_MAX_KEYS
-                and dense_mask.is_contiguous()):
-            # the mask in bits, once for all layers
+                and dense_mask.shape[2] == max_kv and dense_mask.is_contiguous()):
+            # The mask in bits, once for all layers.  Its rows are max_kv apart; stride(1) does not say so where a row of the
+            # batch has one query, because torch calls a tensor contiguous whatever the stride of a dimension of size 1.
             dense_bits = torch.empty(m_max, (max_kv + 63) // 64, dtype=torch.int64, device=h.device)
-            _lib.call("rd_mask_bits", _lib.ptr(dense_mask), dld_q, m_max, max_kv, _lib.ptr(dense_bits), dense_bits.shape[1], st)
+            _lib.call("rd_mask_bits", _lib.ptr(dense_mask), max_kv, m_max, max_kv, _lib.ptr(dense_bits), dense_bits.shape[1], st)
         fused_rope = (self.dtype == torch.bfloat16 and hd == 128 and H % 64 == 0 and xn.data_ptr() % 16 == 0
                       and os.environ.get("RD_FUSED_ROPE", "1") != "0")
         # RMS norms between the projections folded into them (RD_FUSED_NORM=1): o_proj / down_proj also write the
