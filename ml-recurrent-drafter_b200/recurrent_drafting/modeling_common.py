@@ -1,6 +1,6 @@
 """What the base models share: linear layers on the GEMM kernels and the language-model head."""
 import os
-from typing import Dict, NamedTuple, Optional, Tuple
+from typing import Dict, List, NamedTuple, Optional, Tuple
 
 import torch
 
@@ -251,6 +251,11 @@ class PendingRows(NamedTuple):
 class LMHead:
     """Mixin of a causal language model: logits, greedy tokens and slice maxima from its final hidden states.  The model
     has `config` (hidden_size, vocab_size), `dtype`, `device`, `gemm_status`, `_head_ws` and a _lin()["head"] Linear."""
+
+    def held_buffers(self) -> List[torch.Tensor]:
+        """Device memory besides the workspace that captured launches address.  Any of it may be replaced when another request
+        needs more, so who captures launches keeps it."""
+        return [] if self._head_ws is None else [self._head_ws]
 
     def lm_logits(self, hidden_rows: torch.Tensor, logits: torch.Tensor, m_dev=None) -> torch.Tensor:
         """fp32 logits of the given hidden rows (modeling_llama.py:272)."""

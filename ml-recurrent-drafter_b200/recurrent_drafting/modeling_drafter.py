@@ -119,6 +119,7 @@ class DraftResult:
     beams: torch.Tensor  # [B, W, Lb] int64
     q: List[SparseLogProbs]  # Lb-1 lists over rows b*W + beam-at-that-iteration
     anc: torch.Tensor  # [B, W, Lb-1] int32 ancestor row (within the batch row) per iteration
+    buffers: Optional[Dict] = None  # all that the launches address: who captures them keeps it
 
 
 class Drafter(torch.nn.Module):
@@ -316,7 +317,7 @@ class Drafter(torch.nn.Module):
                       _lib.ptr(bin_), _lib.ptr(bout), _lib.ptr(ws["anc"][k % 2]), _lib.ptr(ws["anc"][(k + 1) % 2]),
                       _lib.ptr(ws["parent"]), st)
         last = (Lb - 1) % 2
-        return DraftResult(ws["beams"][last], ws["q"], ws["anc"][last])
+        return DraftResult(ws["beams"][last], ws["q"], ws["anc"][last], ws)
 
     @torch.inference_mode()
     def beam_search_candidates(self, prompt_state: torch.Tensor, init_token: torch.Tensor, embeddings: torch.nn.Embedding,

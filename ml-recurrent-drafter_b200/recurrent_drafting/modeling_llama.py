@@ -14,7 +14,7 @@ Two entry points share one token-major implementation:
 """
 import math
 import os
-from typing import Dict, Optional, Tuple
+from typing import Dict, List, Optional, Tuple
 
 import torch
 from torch import nn
@@ -109,6 +109,9 @@ class LlamaForCausalLM(LMHead, nn.Module):
     def graph_capturable(self) -> bool:
         """No kernel of a step is sized by the live sequence length (the CUDA-core attention's shared memory is)."""
         return self.dtype == torch.bfloat16 and self.head_dim == 128 and self.fused_head_ok()
+
+    def held_buffers(self) -> List[torch.Tensor]:
+        return super().held_buffers() + [t for t in (self._attn_split_ws, *(self._rope or ())) if t is not None]
 
     def new_cache(self, batch_size: int, max_length: int, draft_tokens: int = 0, device=None) -> kv_cache.Cache:
         """A cache for batch_size rows of at most max_length tokens (packed draft tokens included)."""

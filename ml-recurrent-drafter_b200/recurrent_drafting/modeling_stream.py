@@ -109,9 +109,8 @@ class StreamDecoder(LMHead, nn.Module):
     def graph_capturable(self) -> bool:
         return True  # no kernel of a step is sized by the live sequence length
 
-    def held_buffers(self) -> List[Optional[torch.Tensor]]:
-        """Device memory besides the workspace that captured launches address."""
-        return [self.scratch.held()] + self.rotary.held()
+    def held_buffers(self) -> List[torch.Tensor]:
+        return super().held_buffers() + [t for t in (self.scratch.held(), *self.rotary.held()) if t is not None]
 
     def new_cache(self, batch_size: int, max_length: int, draft_tokens: int = 0, device=None) -> kv_cache.HybridCache:
         return kv_cache.HybridCache([l.mixer.cache_spec() for l in self.layers], batch_size, max_length, self.dtype,

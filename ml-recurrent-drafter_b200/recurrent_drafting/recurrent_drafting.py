@@ -132,9 +132,9 @@ class _StepGraphs:
         self.n_kernels = _lib.launches - before
         _lib.launches = before
         self.draft, self.verify, self.accept = graphs
-        # the captured kernels address these: they stay alive even if a larger request makes the model replace them
+        # the captured kernels address these: they stay alive even if another request makes the models replace them
         rows = st.kv_begin.shape[0] * beam_shape.width * beam_shape.length
-        self.buffers = (model.llm.workspace(rows, rows), getattr(model.llm, "held_buffers", lambda: [])())
+        self.buffers = (model.llm.workspace(rows, rows), model.llm.held_buffers(), draft)
         self.ready = True
 
 

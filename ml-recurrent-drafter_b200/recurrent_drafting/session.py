@@ -147,8 +147,7 @@ class DecodeGraphs:
         torch.cuda.current_stream().wait_stream(stream)
         self.n_forward = _lib.launches - before - self.n_pick
         # the captured kernels address these: they stay alive even if a larger request makes the model replace its set
-        held = getattr(session.llm, "held_buffers", lambda: [])()
-        self.buffers = (session.llm.workspace(session.batch, session.batch), session.llm._head_ws, held)
+        self.buffers = (session.llm.workspace(session.batch, session.batch), session.llm.held_buffers())
         _lib.launches = before  # capturing enqueues nothing
 
 
