@@ -24,7 +24,9 @@
 // launch has nkv chains instead of nh.
 // kDense: an explicit mask, one 64-bit word per row and key tile.  The kernel that serves these calls on the CUDA cores keeps
 // its probabilities in fp32, so here P goes to the tensor cores as the sum of two bf16 numbers, in the two buffers (a tile's P
-// then waits for PV of the tile before it).
+// then waits for PV of the tile before it).  That kernel also leaves the values of hidden keys out, whatever they are, where a
+// product with a probability of zero would make a NaN of an infinity: the softmax threads look a V tile over before its
+// product, and in a tile that holds NaN or infinities these are noted for the rows that see them and set to zero.
 // QK of tile t+1 overlaps the softmax and PV of tile t; P is double-buffered in TMEM so that the
 // softmax of tile t does not wait for PV of tile t-1 before writing P; two CTAs fit on an SM (105 KB
 // of shared memory, 256 TMEM columns each) and overlap each other's latencies.  With the shared key features a CTA holds
@@ -201,6 +203,37 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
       : "memory");
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+// Which of the two bf16 numbers in x are NaN or infinite: the top bit of each half.
+__device__ __forceinline__ uint32_t not_finite(uint32_t x) { return ((x & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+// What NaN and infinite values of V come to in a row's result, in shared memory: bit i of word w of the row's first (last) four
+// words = feature 32 w + i has received +inf (-inf); both: NaN.  Words of a row are BMQ apart.
+__device__ __noinline__ void note_specials(uint32_t* specials, const uint8_t* v, uint64_t counts) {
+  for (int j = 0; j < BNK; ++j) {
+    if (!((counts >> j) & 1)) continue;
+    for (int k = 0; k < 16; ++k) {
+      // 16-byte piece k & 7 of the key's row in box k >> 3, where the 128-byte swizzle has put it
+      const uint32_t* x = reinterpret_cast<const uint32_t*>(v + (k >> 3) * kSubTile + j * 128 + (((k & 7) ^ (j & 7)) << 4));
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t f = (x[e >> 1] >> (16 * (e & 1))) & 0xffffu;
+        if ((f & 0x7f80u) != 0x7f80u) continue;
+        const uint32_t bit = 1u << (8 * (k & 3) + e);
+        const bool nan = (f & 0x7fu) != 0;
+        if (nan || !(f & 0x8000u)) specials[(k >> 2) * BMQ] |= bit;
+        if (nan || (f & 0x8000u)) specials[(4 + (k >> 2)) * BMQ] |= bit;
+      }
+    }
+  }
+}
+// Features 32 c .. 32 c + 31 of a row of O with its specials.
+__device__ __forceinline__ void apply_specials(uint32_t* ob, const uint32_t* specials, int c) {
+  const uint32_t pos = specials[c * BMQ], neg = specials[(4 + c) * BMQ];
+  if ((pos | neg) == 0) return;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    if ((pos >> i) & 1) ob[i] = __float_as_uint(__uint_as_float(ob[i]) + INFINITY);
+    if ((neg >> i) & 1) ob[i] = __float_as_uint(__uint_as_float(ob[i]) - INFINITY);
+  }
+}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -271,6 +304,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint64_t* o_full = bars + 9;    // [2]: PV of even / odd tiles done; also frees that tile's V stage
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* odd_tile = abort_flag + 1;  // DENSE, [2]: 1 + the last even / odd tile whose V holds NaN or infinities
+  uint64_t* v_seen = bars + 13;             // DENSE: every softmax warp has looked its part of a V tile over
+  uint64_t* v_noted = bars + 14;            // DENSE: every softmax warp has noted what an odd tile holds
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int base = base_len[b];
@@ -330,6 +366,11 @@ __global__ void __launch_bounds__(kThreads, 2)
     mbar_init(s_empty, 4);
     mbar_init(p_full, 4);
     *abort_flag = 0;
+    if (DENSE) {
+      mbar_init(v_seen, 4);
+      mbar_init(v_noted, 4);
+      odd_tile[0] = odd_tile[1] = 0;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     // The first loads (Q and the first ring's worth of K and V tiles) go out here, before the TMEM
     // allocation and the block-wide barrier below: a short chain of key tiles spends a large part of its
@@ -462,9 +503,29 @@ __global__ void __launch_bounds__(kThreads, 2)
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     int site = 0;  // which wait gave up (reported in the status word)
+    uint32_t* specials = sMask + r;  // DENSE: this row's, valid once there has been an odd tile
+    int n_odd = 0;                   // odd tiles so far, the same in all softmax warps
     for (int t = 0; ok && t < n_tiles; ++t) {
       uint64_t dense = 0;  // requested ahead of the wait for the scores
       if (DENSE && live) dense = reinterpret_cast<const uint64_t*>(tree_mask)[(int64_t)(rs + qi) * mask_words + tile_of(t)];
+      uint8_t* v = sV + (t % L::kVStages) * L::kVStage;
+      uint4* mine = reinterpret_cast<uint4*>(v) + r;  // DENSE: pieces r, r + 128, ... of V are this thread's to look over
+      if (DENSE) {
+        if (!mbar_wait(&v_full[t % L::kVStages], (t / L::kVStages) & 1, abort_flag)) {
+          ok = false;
+          site = 7;
+          break;
+        }
+        uint32_t odd = 0;
+#pragma unroll
+        for (int i = 0; i < L::kVStage / 16 / BMQ; ++i) {
+          const uint4 u = mine[i * BMQ];
+          odd |= not_finite(u.x) | not_finite(u.y) | not_finite(u.z) | not_finite(u.w);
+        }
+        if (odd != 0) odd_tile[t & 1] = t + 1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(v_seen);
+      }
       if (!mbar_wait(&s_full[t & 1], (t >> 1) & 1, abort_flag)) {
         ok = false;
         site = 1;
@@ -537,6 +598,41 @@ __global__ void __launch_bounds__(kThreads, 2)
       const bool rescale = moved && (m_run != -INFINITY);
       m_run = m_new;
       const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
+      if (DENSE) {
+        if (!mbar_wait(v_seen, t & 1, abort_flag)) {
+          ok = false;
+          site = 8;
+          break;
+        }
+        if (n_odd == 0 || (rescale && alpha == 0.f)) {  // none yet, or what came before counts for nothing any more
+#pragma unroll
+          for (int w = 0; w < 8; ++w) specials[w * BMQ] = 0;
+        }
+        if (odd_tile[t & 1] == t + 1) {
+          uint64_t counts = 0;  // keys with a probability other than zero
+#pragma unroll
+          for (int i = 0; i < 64; ++i)
+            if (ex2_approx(fmaf(__uint_as_float(sb[i]), scale_log2, neg_m)) != 0.f) counts |= 1ull << i;
+          note_specials(specials, v, counts);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(v_noted);
+          if (!mbar_wait(v_noted, n_odd++ & 1, abort_flag)) {
+            ok = false;
+            site = 9;
+            break;
+          }
+#pragma unroll 1
+          for (int i = 0; i < L::kVStage / 16 / BMQ; ++i) {
+            uint4 u = mine[i * BMQ];
+            u.x &= ~((not_finite(u.x) >> 15) * 0xffffu);
+            u.y &= ~((not_finite(u.y) >> 15) * 0xffffu);
+            u.z &= ~((not_finite(u.z) >> 15) * 0xffffu);
+            u.w &= ~((not_finite(u.w) >> 15) * 0xffffu);
+            mine[i * BMQ] = u;
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the product reads what was written here
+        }
+      }
       float rowsum0 = 0.f, rowsum1 = 0.f;
       uint32_t pb[32];
 #pragma unroll
@@ -612,6 +708,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       for (int c = 0; c < HD / 32; ++c) {
         uint32_t ob[32];
         tmem_ld32(lane_addr + kColO + c * 32, ob);
+        if (DENSE && n_odd > 0) apply_specials(ob, specials, c);
         if (live) {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
@@ -631,6 +728,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       for (int c = 0; c < HD / 32; ++c) {
         uint32_t ob[32];
         tmem_ld32(lane_addr + kColO + c * 32, ob);
+        if (DENSE && n_odd > 0) apply_specials(ob, specials, c);
         if (live) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {

@@ -40,13 +40,10 @@ def _exact(shape, q, k, v, mask):
     return ((t.transpose(1, 2).reshape(B * n, nh * HD)) for t in (p @ vd, size))
 
 
-@pytest.mark.parametrize("kernel", ["tensor", "cuda"])
-@pytest.mark.parametrize("shape", SHAPES)
-def test_dense_mask(shape, kernel):
+def _attend(shape, q, k, v, mask, kernel):
     from recurrent_drafting import _lib
 
     B, nh, nkv, n, S, slots, shares = shape
-    q, k, v, mask = _problem(shape)
     out = torch.full_like(q, 9.0)
     i32 = dict(dtype=torch.int32, device="cuda")
     row_start, begin, base = torch.arange(B + 1, **i32) * n, torch.zeros(B, **i32), torch.full((B,), S, **i32)
@@ -70,7 +67,53 @@ def test_dense_mask(shape, kernel):
     if kernel == "tensor":
         _lib.load().rd_attention_plan_destroy(plan)
     assert int(status.item()) == 0
+    return out
+
+
+@pytest.mark.parametrize("kernel", ["tensor", "cuda"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_dense_mask(shape, kernel):
+    q, k, v, mask = _problem(shape)
+    out = _attend(shape, q, k, v, mask, kernel)
     want, size = _exact(shape, q, k, v, mask)
     # one rounding to bf16 (half a unit in the last place: 2^-8 of the value at most) and, of the probabilities' 17 bits, the scores' fp32 sums and the exponential,
     # 2^-15 of the sum of magnitudes
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -15 * size).all()
+
+
+# what a hidden slot holds: NaN and infinities of either sign in its value, its key, or both
+@pytest.mark.parametrize("kernel", ["tensor", "cuda"])
+@pytest.mark.parametrize("shape", [(2, 4, 1, 63, 65, 140, 1), (2, 4, 2, 150, 250, 410, 1), (1, 8, 2, 17, 700, 720, 3), (3, 2, 2, 1, 40, 41, 1)])
+def test_values_that_are_not_numbers(shape, kernel):
+    B, nh, nkv, n, S, slots, shares = shape
+    T = S + n
+    q, k, v, mask = _problem(shape, seed=11)
+    nan, inf = float("nan"), float("inf")
+    hidden = torch.zeros(B, T, dtype=torch.bool, device="cuda")
+    hidden[:, 3 : T : 29] = True  # nobody sees these
+    mask &= ~hidden[:, None]
+    at = hidden.nonzero().tolist()
+    for i, (b, j) in enumerate(at):
+        v[b, :, j, i % HD] = (nan, inf, -inf)[i % 3]
+        v[b, :, j, (i + 64) % HD] = (inf, -inf, nan)[i % 3]
+        if i % 2:
+            k[b, :, j] = (nan, inf, -inf)[i // 2 % 3]
+    v[:, :, T:] = nan  # past the live slots
+    k[:, :, T:] = inf
+    # and one that a third of the queries see: +inf, -inf and NaN in three features, both infinities in a fourth
+    seen = torch.arange(n, device="cuda") % 3 == 0
+    for b in range(B):
+        mask[b, :, 7] = mask[b, :, 9] = seen
+        v[b, 0, 7, 100], v[b, 0, 7, 5], v[b, 0, 9, 31], v[b, 0, 9, 64] = inf, -inf, nan, inf
+        v[b, 0, 7, 96], v[b, 0, 9, 96] = inf, -inf
+    out = _attend(shape, q, k, v, mask, kernel)
+    want, size = _exact(shape, q, k.nan_to_num(0, 0, 0), v.nan_to_num(0, 0, 0), mask)
+    want, size = want.view(B, n, nh, HD), size.view(B, n, nh, HD)
+    for h in range(nh // nkv):  # the query heads of key/value head 0
+        for d, x in ((100, inf), (5, -inf), (31, nan), (64, inf), (96, nan)):
+            want[:, seen, h, d] = x
+    out = out.double().view(B, n, nh, HD)
+    finite = want.isfinite()
+    assert torch.equal(out[~finite].nan_to_num(1, 2, 3), want[~finite].nan_to_num(1, 2, 3))
+    off = (out - want).abs()[finite]
+    assert (off <= (2.0 ** -8 * want.abs() + 2.0 ** -15 * size)[finite]).all()
