@@ -353,7 +353,8 @@ RD_API int rd_attention_tc_split(const void* plan, void* out, const int32_t* row
 
 /* rd_attention's mode RD_ATTN_DENSE on the same plans: mask_bits [m, words] 64-bit words, word w of new token t = its keys
  * 64 w .. 64 w + 63 (rd_mask_bits packs them from bytes; words * 64 covers base_len + new tokens of every row).  Probabilities
- * enter the second product as the sum of two bf16 numbers.  n_split and workspace as in rd_attention_tc_split. */
+ * enter the second product as the sum of three bf16 numbers (24 bits); values of hidden keys do not count, NaN or not.
+ * n_split and workspace as in rd_attention_tc_split. */
 RD_API int rd_mask_bits(const uint8_t* mask, int64_t ld, int rows, int cols, void* bits, int words, void* stream);
 RD_API int rd_attention_tc_dense(const void* plan, void* out, const int32_t* row_start, const int32_t* kv_begin,
                           const int32_t* base_len, int max_new, const void* mask_bits, int words, int n_split, void* workspace,

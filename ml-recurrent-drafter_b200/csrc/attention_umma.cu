@@ -23,10 +23,13 @@
 // then the heads that share its keys, not the one token of a single head: the keys are read once per key/value head, and the
 // launch has nkv chains instead of nh.
 // kDense: an explicit mask, one 64-bit word per row and key tile.  The kernel that serves these calls on the CUDA cores keeps
-// its probabilities in fp32, so here P goes to the tensor cores as the sum of two bf16 numbers, in the two buffers (a tile's P
-// then waits for PV of the tile before it).  That kernel also leaves the values of hidden keys out, whatever they are, where a
-// product with a probability of zero would make a NaN of an infinity: the softmax threads look a V tile over before its
-// product, and in a tile that holds NaN or infinities these are noted for the rows that see them and set to zero.
+// its probabilities in fp32, so here P goes to the tensor cores as the sum of three bf16 numbers, which hold its 24 bits: two in
+// the P buffers, the third in the columns of the scores (QK of the next tile then waits for PV of this one).  Error against 64
+// bits over 100 .. 1000 keys: 1.66e-3 with either kernel, the rounding to bf16; ahead of it 0.2e-6 .. 1.8e-6 here (two parts: 1.6e-6
+// .. 2.7e-6) and 0.2e-6 .. 0.6e-6 there.  32 heads, 4 rows of 50 tokens on 500 keys: 26 us (two parts: 25; CUDA cores: 2285).
+// That kernel also leaves the values of hidden keys out, whatever they are, where a product with a probability of zero would make
+// a NaN of an infinity: the softmax threads look a V tile over before its product, and in a tile that holds NaN or infinities these
+// are noted for the rows that see them and set to zero.
 // QK of tile t+1 overlaps the softmax and PV of tile t; P is double-buffered in TMEM so that the
 // softmax of tile t does not wait for PV of tile t-1 before writing P; two CTAs fit on an SM (105 KB
 // of shared memory, 256 TMEM columns each) and overlap each other's latencies.  With the shared key features a CTA holds
@@ -191,6 +194,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// 16 columns; complete only after tmem_st_wait().
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -443,7 +455,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
       }
       for (int t = 0; ok && t < n_tiles; ++t) {
-        if (t + 1 < n_tiles) {
+        if (!DENSE && t + 1 < n_tiles) {
           // S of tile t has been read by the softmax threads -> QK of tile t+1 may overwrite it
           if (!mbar_wait(&k_full[(t + 1) & 1], ((t + 1) >> 1) & 1, abort_flag)) {
             ok = false;
@@ -475,11 +487,21 @@ __global__ void __launch_bounds__(kThreads, 2)
           if (DENSE) {
             umma_ts(tO, tP + ks * 8, dv, idesc_pv, (t | ks) != 0);
             umma_ts(tO, tP + 32 + ks * 8, dv, idesc_pv, 1);
+            umma_ts(tO, tS + ks * 8, dv, idesc_pv, 1);
           } else {
             umma_ts(tO, tP + (t & 1) * 32 + ks * 8, dv, idesc_pv, (t | ks) != 0);
           }
         }
         umma_commit(&o_full[t & 1]);  // O holds tile t; its P buffer and V stage are free
+        if (DENSE && t + 1 < n_tiles) {
+          // the columns of the scores hold a part of P until PV of this tile is done
+          if (!mbar_wait(&k_full[(t + 1) & 1], ((t + 1) >> 1) & 1, abort_flag) || !mbar_wait(&o_full[t & 1], (t >> 1) & 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          issue_qk(t + 1);
+        }
       }
       if (!ok && atomicCAS((int*)abort_flag, 0, 1) == 0 && status) atomicExch(status, 22);
     }
@@ -537,7 +559,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       tmem_ld32(lane_addr + kColS + 32, sb + 32);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(s_empty);
+      if (!DENSE && lane == 0) mbar_arrive(s_empty);
       // visibility of the tile's 64 keys for this row as one 64-bit word
       const int j0 = tile_of(t) * BNK;
       uint64_t vis;
@@ -635,17 +657,42 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
       float rowsum0 = 0.f, rowsum1 = 0.f;
       uint32_t pb[32];
+      if constexpr (DENSE) {
+        // a half of the tile at a time, each part stored as it is formed: what the rounding to bf16 leaves is exact in fp32, and
+        // of 24 bits the third part leaves nothing
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float p0 = ex2_approx(fmaf(__uint_as_float(sb[2 * i]), scale_log2, neg_m));
-        const float p1 = ex2_approx(fmaf(__uint_as_float(sb[2 * i + 1]), scale_log2, neg_m));
-        rowsum0 += p0;
-        rowsum1 += p1;
-        pb[i] = pack_bf16(p0, p1);
-        if (DENSE) {
-          // what the rounding to bf16 left
-          sb[2 * i] = __float_as_uint(p0 - __uint_as_float(pb[i] << 16));
-          sb[2 * i + 1] = __float_as_uint(p1 - __uint_as_float(pb[i] & 0xffff0000u));
+        for (int half = 0; half < 2; ++half) {
+          uint32_t* s = sb + 32 * half;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float p0 = ex2_approx(fmaf(__uint_as_float(s[2 * i]), scale_log2, neg_m));
+            const float p1 = ex2_approx(fmaf(__uint_as_float(s[2 * i + 1]), scale_log2, neg_m));
+            rowsum0 += p0;
+            rowsum1 += p1;
+            s[2 * i] = __float_as_uint(p0);
+            s[2 * i + 1] = __float_as_uint(p1);
+          }
+#pragma unroll
+          for (int part = 0; part < 3; ++part) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float p0 = __uint_as_float(s[2 * i]), p1 = __uint_as_float(s[2 * i + 1]);
+              pb[i] = pack_bf16(p0, p1);
+              s[2 * i] = __float_as_uint(p0 - __uint_as_float(pb[i] << 16));
+              s[2 * i + 1] = __float_as_uint(p1 - __uint_as_float(pb[i] & 0xffff0000u));
+            }
+            tmem_st16(lane_addr + (part == 2 ? kColS : kColP + 32 * part) + 16 * half, pb);
+          }
+        }
+        tmem_st_wait();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float p0 = ex2_approx(fmaf(__uint_as_float(sb[2 * i]), scale_log2, neg_m));
+          const float p1 = ex2_approx(fmaf(__uint_as_float(sb[2 * i + 1]), scale_log2, neg_m));
+          rowsum0 += p0;
+          rowsum1 += p1;
+          pb[i] = pack_bf16(p0, p1);
         }
       }
       l_run = l_run * (moved ? alpha : 1.0f) + (rowsum0 + rowsum1);
@@ -668,20 +715,7 @@ __global__ void __launch_bounds__(kThreads, 2)
           tmem_st32(lane_addr + kColO + c * 32, ob);
         }
       }
-      if (DENSE) {
-        if (t >= 1 && !mbar_wait(&o_full[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag)) {
-          ok = false;
-          site = 6;
-          break;
-        }
-        tc_fence_after();
-        tmem_st32(lane_addr + kColP, pb);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) pb[i] = pack_bf16(__uint_as_float(sb[2 * i]), __uint_as_float(sb[2 * i + 1]));
-        tmem_st32(lane_addr + kColP + 32, pb);
-      } else {
-        tmem_st32(lane_addr + kColP + (t & 1) * 32, pb);
-      }
+      if (!DENSE) tmem_st32(lane_addr + kColP + (t & 1) * 32, pb);
       tc_fence_before();
       // The arrival for tile t must not be possible before the MMA thread has consumed the barrier's
       // phase for tile t-1: the thread issues QK of tile t before it looks at that phase, so without

@@ -76,8 +76,8 @@ def test_dense_mask(shape, kernel):
     q, k, v, mask = _problem(shape)
     out = _attend(shape, q, k, v, mask, kernel)
     want, size = _exact(shape, q, k, v, mask)
-    # one rounding to bf16 (half a unit in the last place: 2^-8 of the value at most) and, of the probabilities' 17 bits, the scores' fp32 sums and the exponential,
-    # 2^-15 of the sum of magnitudes
+    # one rounding to bf16 (half a unit in the last place: 2^-8 of the value at most) and, of the scores' fp32 sums and the
+    # exponential, 2^-15 of the sum of magnitudes
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -15 * size).all()
 
 
@@ -117,3 +117,26 @@ def test_values_that_are_not_numbers(shape, kernel):
     assert torch.equal(out[~finite].nan_to_num(1, 2, 3), want[~finite].nan_to_num(1, 2, 3))
     off = (out - want).abs()[finite]
     assert (off <= (2.0 ** -8 * want.abs() + 2.0 ** -15 * size)[finite]).all()
+
+
+@pytest.mark.parametrize("kernel", ["tensor", "cuda"])
+def test_probabilities_have_24_bits(kernel):
+    """Two keys of probability 1 take away the first and the second 8 bits of a third's: the rest is the result."""
+    heads = 32
+    q = torch.zeros(1, heads, HD, device="cuda")
+    q[..., 0] = 1
+    k = torch.zeros(1, heads, 4, HD, device="cuda")
+    k[0, :, 2, 0] = -torch.linspace(0.37, 7.1, heads, device="cuda").bfloat16().float()
+    k[0, :, 3, 0] = 50  # hidden
+    p = torch.exp(k[0, :, 2, 0].double() * HD ** -0.5)
+    hi = p.bfloat16().double()
+    mid = (p - hi).bfloat16().double()
+    rest = p - hi - mid
+    assert (rest.abs() > 2.0 ** -19).sum() >= 4  # with 16 bits the result is zero
+    v = torch.ones(1, heads, 4, HD, device="cuda")
+    v[0, :, 0], v[0, :, 1] = -hi.float()[:, None], -mid.float()[:, None]
+    mask = torch.tensor([[[True, True, True, False]]], device="cuda")
+    out = _attend((1, heads, heads, 1, 3, 4, 1), q.view(1, -1).bfloat16(), k.bfloat16(), v.bfloat16(), mask, kernel)
+    got = out.double().view(heads, HD) * (2 + p)[:, None]
+    # the exponential: 2 units in the last place of a number below 1, its argument half of one; three fp32 sums of numbers up to 1
+    assert ((got - rest[:, None]).abs() <= 2.0 ** -8 * rest.abs()[:, None] + 6 * 2.0 ** -24).all()
