@@ -811,13 +811,14 @@ __global__ void __launch_bounds__(HD) attention_merge_kernel(const float* partia
   for (int s = 0; s < n_split; ++s) m = fmaxf(m, p[s * (HD + 2) + HD]);
   float acc = 0.f, l = 0.f;
   for (int s = 0; s < n_split; ++s) {
-    const float ms = p[s * (HD + 2) + HD];
-    if (ms == -INFINITY) continue;  // a share without keys has written no O
+    const float ms = p[s * (HD + 2) + HD], ls = p[s * (HD + 2) + HD + 1];
+    if (ls == 0.f) continue;  // no key that the row sees: such a share may have written no O
     const float w = exp2f(ms - m);
+    if (w == 0.f && ls == ls) continue;  // too little to count, also where O holds an infinity; a NaN goes on
     acc += w * p[s * (HD + 2) + d];
-    l += w * p[s * (HD + 2) + HD + 1];
+    l += w * ls;
   }
-  out[((int64_t)tok * nh + h) * HD + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+  out[((int64_t)tok * nh + h) * HD + d] = __float2bfloat16_rn(l == 0.f ? 0.f : acc / l);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

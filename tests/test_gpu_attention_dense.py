@@ -140,3 +140,21 @@ def test_probabilities_have_24_bits(kernel):
     got = out.double().view(heads, HD) * (2 + p)[:, None]
     # the exponential: 2 units in the last place of a number below 1, its argument half of one; three fp32 sums of numbers up to 1
     assert ((got - rest[:, None]).abs() <= 2.0 ** -8 * rest.abs()[:, None] + 6 * 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("kernel", ["tensor", "cuda"])
+@pytest.mark.parametrize("shares", [1, 3])
+def test_scores_that_are_not_numbers(shares, kernel):
+    """A visible key that makes NaN of a score makes NaN of the row, also of one that sees nothing else."""
+    shape = (1, 4, 2, 9, 700, 720, shares)
+    q, k, v, mask = _problem(shape, seed=13)
+    mask[:, :, 400] = False
+    k[0, :, 400] = float("nan")
+    want, size = _exact(shape, q, k.nan_to_num(0), v, mask)
+    mask[:, 1] = False
+    mask[:, 1, 400] = mask[:, 4, 400] = True
+    want.view(9, -1)[[1, 4]] = float("nan")
+    out = _attend(shape, q, k, v, mask, kernel).double()
+    assert torch.equal(out.isnan(), want.isnan())
+    fine = ~want.isnan()
+    assert ((out - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -15 * size)[fine].all()
