@@ -352,7 +352,7 @@ RD_API int rd_attention_tc_split(const void* plan, void* out, const int32_t* row
                           int n_split, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
 
 /* rd_attention's mode RD_ATTN_DENSE on the same plans: mask_bits [m, words] 64-bit words, word w of new token t = its keys
- * 64 w .. 64 w + 63 (rd_mask_bits packs them from bytes; words * 64 covers base_len + new tokens of every row).  Probabilities
+ * 64 w .. 64 w + 63 (rd_mask_bits packs them from bytes; keys past 64 * words are hidden).  Probabilities
  * enter the second product as the sum of three bf16 numbers (24 bits); values of hidden keys do not count, NaN or not.
  * n_split and workspace as in rd_attention_tc_split. */
 RD_API int rd_mask_bits(const uint8_t* mask, int64_t ld, int rows, int cols, void* bits, int words, void* stream);

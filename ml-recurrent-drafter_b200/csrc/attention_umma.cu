@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     int n_odd = 0;                   // odd tiles so far, the same in all softmax warps
     for (int t = 0; ok && t < n_tiles; ++t) {
       uint64_t dense = 0;  // requested ahead of the wait for the scores
-      if (DENSE && live) dense = reinterpret_cast<const uint64_t*>(tree_mask)[(int64_t)(rs + qi) * mask_words + tile_of(t)];
+      if (DENSE && live && tile_of(t) < mask_words) dense = reinterpret_cast<const uint64_t*>(tree_mask)[(int64_t)(rs + qi) * mask_words + tile_of(t)];
       uint8_t* v = sV + (t % L::kVStages) * L::kVStage;
       uint4* mine = reinterpret_cast<uint4*>(v) + r;  // DENSE: pieces r, r + 128, ... of V are this thread's to look over
       if (DENSE) {

@@ -158,3 +158,32 @@ def test_scores_that_are_not_numbers(shares, kernel):
     assert torch.equal(out.isnan(), want.isnan())
     fine = ~want.isnan()
     assert ((out - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -15 * size)[fine].all()
+
+
+@pytest.mark.parametrize("shares", [1, 3])
+def test_mask_of_fewer_words_than_keys(shares):
+    """Keys past the mask's words are hidden, and no word of another row or past the last row is read."""
+    from recurrent_drafting import _lib
+
+    shape = (2, 4, 2, 9, 700, 720, shares)
+    q, k, v, mask = _problem(shape, seed=17)
+    short = mask.clone()
+    short[:, :, 5 * 64 :] = False
+    real = _lib.call
+
+    def call(name, *args):  # packs five words a row; the bits' buffer ends with those of the last row
+        if name == "rd_mask_bits":
+            rows = args[2]
+            bits = call.bits = torch.empty(rows, 5, dtype=torch.int64, device="cuda")
+            return real(name, args[0], args[1], rows, 5 * 64, _lib.ptr(bits), 5, args[6])
+        if name == "rd_attention_tc_dense":
+            args = args[:6] + (_lib.ptr(call.bits), 5) + args[8:]
+        return real(name, *args)
+
+    _lib.call = call
+    try:
+        out = _attend(shape, q, k, v, mask, "tensor")
+    finally:
+        _lib.call = real
+    want, size = _exact(shape, q, k, v, short)
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -15 * size).all()
