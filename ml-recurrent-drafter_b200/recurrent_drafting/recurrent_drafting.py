@@ -340,10 +340,6 @@ class RecurrentDrafting(torch.nn.Module):
             with text_generation.step() as rec:
                 self._step(st, cache, beam_shape, sampling_args, s_max, rec, graphs)
                 st.small_host.copy_(st.small, non_blocking=True)
-                if graphs is not None and n_steps == 2 and seq_len + Lb < max_length:
-                    # a step adds Lb tokens at most, so there will be a third one: captured while the device is at work on
-                    # this one
-                    graphs.capture(self, st, cache, beam_shape, sampling_args)
                 torch.cuda.current_stream().synchronize()
                 if int(st.small_host[2, 0]) != 0:
                     raise _lib.RedrafterError(

@@ -52,3 +52,31 @@ def test_graphs_are_not_used_where_they_do_not_apply():
     model2 = rd.RecurrentDrafting(llm2, dr2, cuda_graphs=True)
     assert model2._graphs_apply(rd.SamplingArgs(1.0, True)) and model2._graphs_apply(rd.SamplingArgs(0.8, False))
     assert not rd.RecurrentDrafting(llm2, dr2, cuda_graphs=False)._graphs_apply(rd.SamplingArgs(1.0, True))
+
+
+@pytest.mark.parametrize("eos", [False, True])
+def test_graphs_are_captured_only_when_a_third_step_is_asked_for(eos, monkeypatch):
+    """A request that ends with its second step, by an end token or because its consumer stops, pays for no capture."""
+    import recurrent_drafting as rd
+
+    llm, dr, _, _ = build_models(HD128_LLAMA, HD128_DRAFTER, 77, dtype=torch.bfloat16)
+    model = rd.RecurrentDrafting(llm, dr, cuda_graphs=True)
+    prompt = t(mb.prompts(1, 40, HD128_LLAMA["vocab_size"], 5))
+    shape = rd.modeling_drafter.BeamShape(8, 3)
+    captures = []
+    capture = rd.recurrent_drafting._StepGraphs.capture
+    monkeypatch.setattr(rd.recurrent_drafting._StepGraphs, "capture", lambda *a: captures.append(1) or capture(*a))
+
+    def steps(end):
+        return model.generate(rd.stats.Ledger(), prompt, 40 + 60, shape, rd.SamplingArgs(1.0, True), rd.SpecialTokens(0, end))
+
+    run = steps(None)
+    first, second = next(run), next(run)
+    assert not captures
+    if not eos:
+        next(run)
+        assert len(captures) == 1
+        return
+    last = int(second[0, -1])
+    assert last not in first[0, 40:].tolist()
+    assert len(list(steps(last))) == 2 and not captures
