@@ -307,10 +307,10 @@ class LlamaForCausalLM(LMHead, nn.Module):
             for name, width in (("h", H), ("xn", H), ("qkv", (nh + 2 * nkv) * hd), ("q", nh * hd), ("attn", nh * hd),
                                 ("act", self.config.intermediate_size), ("hidden", H)):
                 full[name] = torch.empty(cap_m, width, dtype=dt, device=dev)
-            # folded RMS norm: per-token sums of squares by 128-feature slice
             # shares of the projections with a residual
-            most = max(lin.shares_bytes(min(cap_m, _Linear.MAX_SHARE_ROWS)) for lin in (self._lin()["o"] + self._lin()["down"]))
+            most = max((lin.shares_bytes(min(cap_m, _Linear.MAX_SHARE_ROWS)) for lin in self._lin()["o"] + self._lin()["down"]), default=0)
             full["parts"] = torch.empty(most // 4, dtype=torch.float32, device=dev)
+            # folded RMS norm: per-token sums of squares by 128-feature slice
             full["ss"] = torch.empty(cap_m, ((H + 127) // 128 + 3) // 4 * 4, dtype=torch.float32, device=dev)
         if logit_rows > cap_l:
             cap_l = logit_rows
