@@ -289,6 +289,16 @@ def run_ours(args):
         prof.append((len(all_calls), self.weight.shape[0], self.weight.shape[1], None))
         real_qkv_rope(self, a, *pa, **kw)
 
+    real_add_residual = _Linear.add_residual
+
+    def timed_add_residual(self, a, c, residual, m_dev, *pa):
+        # leaves its rows in shares of K for few rows; where it may not, it comes down to __call__, which is counted there
+        at = len(all_calls)
+        pending = real_add_residual(self, a, c, residual, m_dev, *pa)
+        if pending is not None:
+            prof.append((at, self.weight.shape[0], self.weight.shape[1], a.shape[0] if m_dev is None else None))
+        return pending
+
     def timed_call(name, *a):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
@@ -304,6 +314,7 @@ def run_ours(args):
         next(it)
     _Linear.__call__ = timed_linear
     _Linear.qkv_rope = timed_qkv_rope
+    _Linear.add_residual = timed_add_residual
     _lib.call = timed_call
     flops = 0.0
     gemm_ms = 0.0
@@ -311,7 +322,7 @@ def run_ours(args):
     by_kernel = {}
     by_shape = {}
     n_prof_steps = 4
-    gemm_names = ("rd_gemm_bf16_tc", "rd_gemm_bf16_tc_qkv_rope", "rd_gemm_bf16_tc_argmax", "rd_gemm_bf16_tc_topk")
+    gemm_names = ("rd_gemm_bf16_tc", "rd_gemm_bf16_tc_res_shares", "rd_gemm_bf16_tc_qkv_rope", "rd_gemm_bf16_tc_argmax", "rd_gemm_bf16_tc_topk")
     for _ in range(n_prof_steps):
         prof.clear()
         all_calls.clear()
@@ -336,6 +347,7 @@ def run_ours(args):
             agg[2] += f
     _Linear.__call__ = real_linear_call
     _Linear.qkv_rope = real_qkv_rope
+    _Linear.add_residual = real_add_residual
     _lib.call = real_call
     it.close()
     model.cuda_graphs = graphs_setting
@@ -779,11 +791,17 @@ class KernelLog:
         flops = nbytes = 0.0
         if name.startswith("rd_gemm") and self.shape is not None:
             N, K, out = self.shape
+            if name == "rd_gemm_bf16_tc_res_shares" and M <= 256:
+                out = 0.0  # the norm that follows forms the rows; the shares between the two are not among what must move
             flops, nbytes = 2.0 * M * N * K, 2.0 * N * K + 2.0 * M * K + out * M * N
         elif name == "rd_stream_norm":
             nbytes = M * H * ((2 if args[1] is not None else 4 * args[7]) + (4 if args[8] is not None else 0) + 2.0)
+        elif name == "rd_stream_norm_shares":  # with few rows the last stored one is written here
+            nbytes = M * H * (4.0 * args[4] + (4 if M <= 256 else 0) + (4 if args[8] is not None else 0) + 2.0)
         elif name in ("rd_rmsnorm", "rd_embed_gather"):
             nbytes = 4.0 * M * H
+        elif name == "rd_rmsnorm_shares":
+            nbytes = (6.0 if M <= 256 else 4.0) * M * H
         elif name.startswith("rd_attention"):
             flops, nbytes = self.attention(name, args)
         elif name == "rd_head_gemm":
@@ -837,18 +855,19 @@ class KernelLog:
 
         real_call, saved = _lib.call, {}
         # bytes per output element: two, four with a fp32 result, eight where a fp32 residual is read as well; none for the arg-max
-        for method in ("__call__", "xielu", "clamped_glu", "split", "qkvg_rope", "qkv_rope", "qk_rope_norm", "argmax"):
+        for method in ("__call__", "xielu", "clamped_glu", "split", "qkvg_rope", "qkv_rope", "qk_rope_norm", "argmax", "add_residual"):
             saved[method] = getattr(Linear, method)
 
             def wrapped(lin, a, c, *pa, _real=saved[method], _m=method, **kw):
                 per = 0.0 if _m == "argmax" else 2.0
-                if _m == "__call__":
-                    per = float(c.element_size()) * (2 if kw.get("residual") is not None else 1)
+                if _m in ("__call__", "add_residual"):
+                    per = float(c.element_size()) * (2 if _m == "add_residual" or kw.get("residual") is not None else 1)
                 n = lin.weight.shape[0]
                 glu = _m == "clamped_glu" or (_m == "__call__" and pa and pa[0] == _lib.EPI_SWIGLU)
                 self.shape = (n // 2 * 2, lin.weight.shape[1], per * (0.5 if glu else 1.0))
-                _real(lin, a, c, *pa, **kw)
+                result = _real(lin, a, c, *pa, **kw)
                 self.shape = None
+                return result
 
             setattr(Linear, method, wrapped)
 
