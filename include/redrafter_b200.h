@@ -179,7 +179,9 @@ RD_API int rd_gemm_bf16_tc(const void* plan, int out_dtype, void* C, int64_t ldc
 
 /* C = A W^T + R (RD_EPI_RES), or, for few rows, the shares that a norm kernel adds up (rd_rmsnorm_shares,
  * rd_stream_norm_shares): up to 256 live rows of at most 1024, K is cut among CTA pairs that the weight tiles alone would leave idle, and
- * C is not written.  parts: rd_gemm_shares_bytes(m_max, N, K) bytes, 16-byte aligned; 0 means that no row count is cut. */
+ * C is not written.  parts: rd_gemm_shares_bytes(m_max, N, K) bytes, 16-byte aligned; 0 means that no row count is cut.
+ * Shares change the order of a row's fp32 additions: the last bits of a result depend on the side of 256 live rows and of 1024
+ * rows of capacity on which the call lies. */
 RD_API int64_t rd_gemm_shares_bytes(int m_max, int N, int K);
 RD_API int rd_gemm_bf16_tc_res_shares(const void* plan, int out_dtype, void* C, int64_t ldc, const void* R, int64_t ldr,
                                const int32_t* m_dev, float* parts, int64_t parts_bytes, int32_t* status, void* stream);
