@@ -1,6 +1,6 @@
 // C = epilogue(A * W^T) on CUDA cores with fp32 accumulation, for fp32 models (exact-fp32 parity
 // with a CPU run is only possible without tensor cores) and as the cross-check of the tcgen05
-// path.  Two kernels with 256 threads: 64x64 tiles, and 32x32 tiles where 64x64 tiles would be fewer than the GPU can hold.  Both add
+// path.  Two kernels with 256 threads: 64x64 tiles, and 32x32 tiles where launch() finds them to finish first.  Both add
 // an output's products in ascending order of K, so they give the same bits.
 #include "rd_common.cuh"
 
@@ -175,23 +175,37 @@ template <typename T, typename OutT>
 int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* bias, const void* R,
            int64_t ldr, int m_max, const int32_t* m_dev, int N, int K, int epilogue, float act0, float act1, cudaStream_t s) {
   dim3 grid((N + BN - 1) / BN, (m_max + BM - 1) / BM);
-  // Two 64x64 tiles fit on an SM at a time.  Where there are fewer than that the small tiles finish first however they are dealt;
-  // with more, the large ones read their operands half as often.
-  const bool small = (int64_t)grid.x * grid.y < 2 * 148;
+  // Both kernels keep several blocks on an SM (48 registers, 256 threads: five), but what an SM's blocks take adds up: K = 2048, one
+  // B200, us of a launch by itself with 1 / 2 / 3 / 4 small tiles per SM: 59 / 100 / 145 / 190, with 1 / 2 large ones 133 / 240 (123 / 223
+  // where half of their rows are empty).  So small tiles as long as there are at most two of them for each large one that an SM would
+  // have: 64 x 4736 100 and not 133, but 64 x 6144 133 and not 145, 512 x 2304 221 and not 371.  K = 256 and 688 lie the same way.
+  // From two large tiles per SM on there are only these, although few rows would gain (20 x 18944: 223, small ones 180).
+  constexpr int kSMs = 148;
+  const auto per_sm = [](int64_t blocks) { return (blocks + kSMs - 1) / kSMs; };
   const dim3 small_grid((N + SN - 1) / SN, (m_max + SM - 1) / SM);
+  const int64_t n_large = (int64_t)grid.x * grid.y, n_small = (int64_t)small_grid.x * small_grid.y;
+  const bool small = n_large < 2 * kSMs && per_sm(n_small) <= 2 * per_sm(n_large);
+  // Launched programmatically only while two such launches have an SM for each block: blocks that are placed beside those of the
+  // launch before crowd on some SMs.  In a row, K = 2048: 64 blocks 53 us (ordinary launches 54), 128 blocks 107 (56), 288 blocks
+  // 202 (97); K = 256: 64 blocks 8.1 (10.5), 256 blocks 25.5 (14.9).
+  const bool chained = 2 * n_small <= kSMs;
   const auto row_vec = [](const void* p, int64_t ld) { return ((uintptr_t)p | (uintptr_t)(ld * sizeof(T))) % (4 * sizeof(T)) == 0; };
   const int vec_a = row_vec(A, lda), vec_w = row_vec(W, ldw);
 #define RD_LAUNCH_EPI(E)                                                                                              \
   case E:                                                                                                             \
-    if (small) {                                                                                                      \
+    if (small && chained) {                                                                                           \
       cudaError_t err = rd::launch_chained(gemm_simt_small_kernel<T, OutT, E>, small_grid, dim3(256), 0, s, 1, (const T*)A, lda, \
                                            (const T*)W, ldw, (OutT*)C, ldc, (const T*)bias, (const OutT*)R, ldr, m_max, m_dev, N, K, \
                                            act0, act1, vec_a, vec_w);                                                \
       RD_CHECK_CHAINED(err);                                                                                          \
-      break;                                                                                                          \
+    } else if (small) {                                                                                               \
+      gemm_simt_small_kernel<T, OutT, E><<<small_grid, 256, 0, s>>>((const T*)A, lda, (const T*)W, ldw, (OutT*)C, ldc,  \
+                                                                    (const T*)bias, (const OutT*)R, ldr, m_max, m_dev, N, K, act0, act1, \
+                                                                    vec_a, vec_w);                                    \
+    } else {                                                                                                          \
+      gemm_simt_kernel<T, OutT, E><<<grid, 256, 0, s>>>((const T*)A, lda, (const T*)W, ldw, (OutT*)C, ldc, (const T*)bias, \
+                                                        (const OutT*)R, ldr, m_max, m_dev, N, K, act0, act1);         \
     }                                                                                                                 \
-    gemm_simt_kernel<T, OutT, E><<<grid, 256, 0, s>>>((const T*)A, lda, (const T*)W, ldw, (OutT*)C, ldc, (const T*)bias, \
-                                                      (const OutT*)R, ldr, m_max, m_dev, N, K, act0, act1);           \
     break;
   switch (epilogue) {
     RD_LAUNCH_EPI(RD_EPI_NONE)
