@@ -174,6 +174,13 @@ RD_API int rd_gemm(int dtype, int out_dtype, const void* A, int64_t lda, const v
  * Free with rd_gemm_plan_destroy.  Returns NULL on failure. */
 RD_API void* rd_gemm_plan_create(const void* A, int64_t lda, int m_max, const void* W, int64_t ldw, int N, int K);
 RD_API void rd_gemm_plan_destroy(void* plan);
+/* Launches of this plan may read W before the kernels ahead of them in the stream have finished.  For calls that follow, in one
+ * chain of this library's launches, an rd_embed_gather, rd_stream_norm with ids or rd_drafter_prepare: these let what comes after
+ * them start only when all that came before them is complete, so that W is as the stream's earlier work left it. */
+RD_API void rd_gemm_plan_early(void* plan);
+/* 1 if plans of this size are served by the kernel for few tokens (up to 256, fewer for matrices of few features; K a multiple of
+ * 64): one wave of CTAs, each with a slab of weight rows, all of K and all tokens.  A row's sums then run over K in one piece. */
+RD_API int rd_gemm_few_rows(int m_max, int N, int K);
 RD_API int rd_gemm_bf16_tc(const void* plan, int out_dtype, void* C, int64_t ldc, const void* bias, const void* R,
                     int64_t ldr, const int32_t* m_dev, int epilogue, int32_t* status, void* stream);
 

@@ -11,8 +11,8 @@ template <typename T>
 __global__ void drafter_prepare_kernel(const T* embed, const int64_t* beams,
                                        const int32_t* parent, const T* ctx, T* a,
                                        T* x, int W, int Lb, int H, int k, int vec, int additive) {
-  rd::pdl_launch_dependents();
   rd::pdl_wait();
+  rd::pdl_launch_dependents();  // what follows may read weights ahead of its own wait (rd_gemm_plan_early)
   const int r = blockIdx.x;
   const int b = r / W;
   const int64_t tok = beams[(int64_t)r * Lb + k];

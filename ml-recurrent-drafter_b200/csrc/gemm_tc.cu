@@ -28,7 +28,7 @@
 //              tile's main loop through the second accumulator buffer; the peer's epilogue frees the
 //              accumulator with remote mbarrier arrives.
 // gemm_tc_kernel is the single-CTA form of the same design (cta_group::1, 128 weight rows per tile,
-// four stages) for matrices with fewer than 256 output features.
+// four stages) for matrices with fewer than 256 output features.  gemm_rows_kernel (gemm_rows.cuh) serves few tokens.
 // Tiles are walked weight-tile-major so that the CTAs running at the same time share W tiles
 // through L2; GEMMs with few weight tiles cut the tokens finer so that every CTA pair has a tile.
 //
@@ -80,11 +80,25 @@ struct TokMaps {
   CUtensorMap m[4];
 };
 
+constexpr int kRowMaps = 9;  // token boxes of gemm_rows_kernel: 16, 32, 64, 96 .. 256 rows
+struct RowMaps {
+  CUtensorMap m[kRowMaps];
+};
+struct RowsShape {
+  int rows, kb;   // weight rows of a CTA (0: the plan is not for this kernel); k-blocks of 64 per load
+  int a_rows;     // the most tokens that a stage has to hold
+  int tmem_cols;
+  int early;      // weights may be requested before the dependency wait
+};
+
 struct GemmPlan {
   CUtensorMap map_a;    // activations [m_max, K], box 64 x 128 (single-CTA kernel)
   TokMaps maps_a;       // the same tensor in boxes of 64 x 32/64/96/128: the pair kernel fetches only the rows its chunk fills
   CUtensorMap map_w;  // weights [N, K], box 64 x 128
   int m_max, N, K;
+  RowsShape rows;
+  CUtensorMap map_rows_w;  // [k-blocks][N][64], box kb x rows
+  RowMaps maps_rows_a;     // [k-blocks][m_max][64], boxes of kb x 16 / 32 / 64 .. tokens as far as m_max needs them
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -97,17 +111,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
 }
 // One attempt: the hardware may suspend the thread until the phase completes or a time limit of its
 // own expires, so a waiter wakes as soon as the barrier flips instead of at its next poll.
@@ -129,7 +132,7 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 // Bounded wait (kWaitLimitNs).  Returns false when it gave up or when another role already aborted.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_test(bar, parity)) return true;
+  if (mbar_try(bar, parity)) return true;  // most waits end here, without the clock's latency
   const uint64_t t0 = global_ns();
   for (;;) {
     if (mbar_try(bar, parity)) return true;
@@ -668,39 +671,48 @@ __device__ __forceinline__ void norm_scale_stage(const EpiArgs& e, float* s_scal
 // epilogue warps exchange their transposed blocks through the scratch and meet at a named barrier.
 // Values are rounded to bf16 first, as a separate projection would have stored them, so the result
 // equals projection -> rope bit for bit.  After the exchange four lanes share a token row (8 features
-// each), so the cos/sin reads and the stores of an instruction cover 8 rows, not 32.
-__device__ __forceinline__ void epilogue_rope_block(const float* v, const EpiArgs& e, float* scr_all, int quarter, int lane,
-                                                    int head, int tok0, int tok_limit, const int* s_pos, const int* s_dst,
-                                                    const float* s_scale, float* ss_red) {
-  float* scr = scr_all + quarter * 32 * kScrLd;
+// each), so the cos/sin reads and the stores of an instruction cover 8 rows, not 32.  PUT = false: the exchange area already
+// holds all four quarters, as rope_round leaves them.
+// The cos/sin rows of a 32-token block, requested ahead of where they are needed: four lanes share a token row.
+struct RopeRows {
+  float4 v[4][4];
+  __device__ __forceinline__ void request(const EpiArgs& e, const int* s_pos, int quarter, int lane, int tok0, int tok_limit, bool is_v) {
+    if (is_v) return;
+    const int row0 = lane >> 2, d0 = quarter * 32 + (lane & 3) * 8;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      if (tok0 + row0 + 8 * p < tok_limit) {
+        const int pos = s_pos[tok0 + row0 + 8 * p];
+        const float* c = e.cos_t + (int64_t)pos * 128 + d0;
+        const float* sn = e.sin_t + (int64_t)pos * 128 + d0;
+        v[p][0] = ldg_f4(c), v[p][1] = ldg_f4(c + 4), v[p][2] = ldg_f4(sn), v[p][3] = ldg_f4(sn + 4);
+      }
+    }
+  }
+};
+
+__device__ __forceinline__ void rope_round(float* v, const EpiArgs& e, const float* s_scale) {
+  // folded RMS norm: the projection of the normalised row is the projection of the row times its scale; scaled and
+  // rounded after the exchange, where a lane holds one token's values.  Normed heads are rounded once, at the end.
+  if (s_scale != nullptr || e.head_norm) return;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __bfloat162float(__float2bfloat16_rn(v[i]));
+}
+template <bool PUT>
+__device__ __forceinline__ void epilogue_rope_block(float* v, const EpiArgs& e, float* scr_all, int quarter, int lane,
+                                                    int head, int tok0, int tok_limit, const int* s_dst, const RopeRows& rows,
+                                                    const float* s_scale, float* ss_red, int quarter_stride = 32 * kScrLd) {
+  float* scr = scr_all + quarter * quarter_stride;
   const bool is_v = head >= e.nh + e.nkv;
   const int sub = lane & 3, row0 = lane >> 2;
   const int d0 = quarter * 32 + sub * 8;
   const float sign = d0 < e.rot_half ? -1.0f : 1.0f;  // rotate_half: (-x2, x1)
   // this lane's eight features are paired with those at pd (unrotated features with themselves: their sines are 0)
   const int pd = d0 < e.rot_half ? d0 + e.rot_half : (d0 < 2 * e.rot_half ? d0 - e.rot_half : d0);
-  // the cos/sin rows of the block's tokens are requested first (volatile asm keeps them here): their latency
-  // runs under the transposition and the exchange below
-  float4 cs[4][4];
-  if (!is_v) {
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      if (tok0 + row0 + 8 * p < tok_limit) {
-        const int pos = s_pos[row0 + 8 * p];
-        const float* c = e.cos_t + (int64_t)pos * 128 + d0;
-        const float* sn = e.sin_t + (int64_t)pos * 128 + d0;
-        cs[p][0] = ldg_f4(c), cs[p][1] = ldg_f4(c + 4), cs[p][2] = ldg_f4(sn), cs[p][3] = ldg_f4(sn + 4);
-      }
-    }
-  }
-  if (s_scale != nullptr || e.head_norm) {
-    // folded RMS norm: the projection of the normalised row is the projection of the row times its scale; scaled and
-    // rounded after the exchange, where a lane holds one token's values.  Normed heads are rounded once, at the end.
+  if (PUT) {
+    rope_round(v, e, s_scale);
 #pragma unroll
     for (int i = 0; i < 32; ++i) scr[i * kScrLd + lane] = v[i];
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) scr[i * kScrLd + lane] = __bfloat162float(__float2bfloat16_rn(v[i]));
   }
   asm volatile("bar.sync 1, 128;" ::: "memory");
   float o[4][8];
@@ -733,7 +745,7 @@ __device__ __forceinline__ void epilogue_rope_block(const float* v, const EpiArg
       for (int j = 0; j < 8; ++j) o[p][j] = __bfloat162float(__float2bfloat16_rn(o[p][j] * sc));
     }
     if (!is_v) {
-      const float* oth = scr_all + (pd >> 5) * 32 * kScrLd + r * kScrLd + (pd & 31);
+      const float* oth = scr_all + (pd >> 5) * quarter_stride + r * kScrLd + (pd & 31);
       float4 b0 = *reinterpret_cast<const float4*>(oth), b1 = *reinterpret_cast<const float4*>(oth + 4);
       if (s_scale != nullptr) {
         b0.x = __bfloat162float(__float2bfloat16_rn(b0.x * sc)), b0.y = __bfloat162float(__float2bfloat16_rn(b0.y * sc));
@@ -742,7 +754,7 @@ __device__ __forceinline__ void epilogue_rope_block(const float* v, const EpiArg
         b1.z = __bfloat162float(__float2bfloat16_rn(b1.z * sc)), b1.w = __bfloat162float(__float2bfloat16_rn(b1.w * sc));
       }
       if (tok0 + r < tok_limit) {
-        const float4 c0 = cs[p][0], c1 = cs[p][1], s0 = cs[p][2], s1 = cs[p][3];
+        const float4 c0 = rows.v[p][0], c1 = rows.v[p][1], s0 = rows.v[p][2], s1 = rows.v[p][3];
         // two rounded products and one rounded sum, as the separate rope kernel computes them
         o[p][0] = __fadd_rn(__fmul_rn(o[p][0], c0.x), __fmul_rn(sign * b0.x, s0.x));
         o[p][1] = __fadd_rn(__fmul_rn(o[p][1], c0.y), __fmul_rn(sign * b0.y, s0.y));
@@ -1003,8 +1015,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         } else if (EPI == kEpiQkvRope && rope_head >= epi.nh + 2 * epi.nkv) {
           epilogue_gate_block(v, epi, lane, n_warp0 - (epi.nh + 2 * epi.nkv) * 128, tok_base + c, tok_limit);
         } else if (EPI == kEpiQkvRope) {
-          epilogue_rope_block(v, epi, scratch, quarter, lane, rope_head, tok_base + c, tok_limit, s_pos + c, s_dst + c,
-                              norm_in ? s_scale + c : nullptr, ss_red + ((c >> 5) & 1) * 128);
+          // requested first (volatile asm keeps them here): their latency runs under the transposition and the exchange
+          RopeRows cs;
+          cs.request(epi, s_pos - tok_base, quarter, lane, tok_base + c, tok_limit, rope_head >= epi.nh + epi.nkv);
+          epilogue_rope_block<true>(v, epi, scratch, quarter, lane, rope_head, tok_base + c, tok_limit, s_dst + c, cs,
+                                    norm_in ? s_scale + c : nullptr, ss_red + ((c >> 5) & 1) * 128);
         } else if (EPI == kEpiArgmax) {
           epilogue_argmax_block(v, epi, scr, lane, n_warp0, tok_base + c, tok_limit, N);
         } else if (EPI == kEpiSplit && n_warp0 >= epi.n_split) {
@@ -1337,8 +1352,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         } else if (EPI == kEpiQkvRope && rope_head >= epi.nh + 2 * epi.nkv) {
           epilogue_gate_block(v, epi, lane, n_warp0 - (epi.nh + 2 * epi.nkv) * 128, tok_base + c, tok_limit);
         } else if (EPI == kEpiQkvRope) {
-          epilogue_rope_block(v, epi, scratch, quarter, lane, rope_head, tok_base + c, tok_limit, s_pos + c, s_dst + c,
-                              norm_in ? s_scale + c : nullptr, ss_red + ((c >> 5) & 1) * 128);
+          // requested first (volatile asm keeps them here): their latency runs under the transposition and the exchange
+          RopeRows cs;
+          cs.request(epi, s_pos - tok_base, quarter, lane, tok_base + c, tok_limit, rope_head >= epi.nh + epi.nkv);
+          epilogue_rope_block<true>(v, epi, scratch, quarter, lane, rope_head, tok_base + c, tok_limit, s_dst + c, cs,
+                                    norm_in ? s_scale + c : nullptr, ss_red + ((c >> 5) & 1) * 128);
         } else if (EPI == kEpiArgmax) {
           epilogue_argmax_block(v, epi, scr, lane, n_warp0, tok_base + c, tok_limit, N);
         } else if (EPI == kEpiResShares && shares > 1) {
@@ -1373,6 +1391,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * kMaxChunk) : "memory");
   }
 }
+
+#include "gemm_rows.cuh"
 
 // Second half of the fused LM-head argmax: the partial results are 64-bit keys whose unsigned order is
 // (logit descending, id ascending), so the merge is a plain maximum.  A block serves 8 tokens with 32
@@ -1436,6 +1456,18 @@ bool make_map(CUtensorMap* map, const void* base, int64_t ld_elems, int rows, in
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same matrix as k-blocks of 64 features: box of `kb` blocks x `box_rows` rows.  cols is a multiple of 64.
+bool make_map_blocks(CUtensorMap* map, const void* base, int64_t ld_elems, int rows, int cols, int box_rows, int kb) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)BK, (cuuint64_t)rows, (cuuint64_t)(cols / BK)};
+  cuuint64_t strides[2] = {(cuuint64_t)ld_elems * 2, (cuuint64_t)BK * 2};
+  cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, (cuuint32_t)kb};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <typename Kern>
 int launch_cluster2(Kern kern, int grid, int smem_bytes, cudaStream_t s, const GemmPlan* p, const EpiArgs& e, const int32_t* m_dev,
                     int32_t* status) {
@@ -1466,9 +1498,48 @@ int multiprocessors() {
   return sm_count;
 }
 
+// Slabs of gemm_rows_kernel for m_max tokens; rows 0 where it does not serve.  One wave of slabs has to cover the matrix, and K has to be
+// whole k-blocks.  Slabs of 96 rows are left out: QKV projections of 96 heads need whole heads, and the others finish as soon
+// with 128.  A narrow slab's products cost the same as a wide one's and every CTA loads all tokens, so with many tokens other splits win:
+// 4096 x 11008 with its norm, 64 tokens 25.4 us here and 25.6 in shares of K, 110 tokens 39 and 27; 6144 x 4096, 110 tokens 16.0
+// here and 17.8 in pairs.
+RowsShape rows_shape(int m_max, int N, int K) {
+  RowsShape s{};
+  if (m_max > kMaxChunk || K % BK != 0) return s;
+  int rows = ((N + multiprocessors() - 1) / multiprocessors() + 31) / 32 * 32;
+  if (rows == 96) rows = 128;
+  if (rows > 256 || m_max > (rows == 32 ? 64 : (rows == 64 ? 128 : kMaxChunk))) return s;
+  s.a_rows = row_map_rows(row_map_index(m_max));
+  // the more k-blocks a step has the less its own cost counts, as long as four steps fit
+  for (s.kb = rows == 32 ? 4 : (rows <= 160 ? 2 : 1); s.kb > (rows < BM ? 2 : 1) && rows_stages(rows, s.a_rows, s.kb) < 4;) s.kb /= 2;
+  for (s.tmem_cols = 32; s.tmem_cols < (rows > BM ? 2 : 1) * max(s.a_rows, 32);) s.tmem_cols *= 2;
+  s.rows = rows;
+  return s;
+}
+
+template <int EPI, bool OUT_F32>
+int launch_rows(const GemmPlan* p, const EpiArgs& e, const int32_t* m_dev, int32_t* status, cudaStream_t s) {
+  auto kern = gemm_rows_kernel<EPI, OUT_F32>;
+  static bool smem_set = false;
+  if (!smem_set) {
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem);
+    RD_CHECK_CHAINED(err);
+    smem_set = true;
+  }
+  const int cluster = EPI == kEpiQkvRope ? BM / p->rows.rows : 1;
+  const int grid = EPI == kEpiQkvRope ? (p->N + BM - 1) / BM * cluster : (p->N + p->rows.rows - 1) / p->rows.rows;
+  cudaError_t err = rd::launch_chained(kern, dim3(grid), dim3(kRowsThreads), kRowsSmem, s, cluster, p->maps_rows_a, p->map_rows_w, e,
+                                       p->rows, p->m_max, m_dev, p->N, p->K, status);
+  RD_CHECK_CHAINED(err);
+  return RD_OK;
+}
+
 template <int EPI>
 int launch_out(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t* m_dev, int32_t* status, cudaStream_t s) {
   const int sm_count = multiprocessors();
+  // the folded RMS norms need 128 features in a CTA, rotary heads a cluster of whole slabs
+  if (EPI != kEpiResShares && p->rows.rows > 0 && !e.gamma && !e.ss_in && (EPI != kEpiQkvRope || p->rows.rows <= BM))
+    return out_dtype == RD_F32 ? launch_rows<EPI, true>(p, e, m_dev, status, s) : launch_rows<EPI, false>(p, e, m_dev, status, s);
   // upper bound of the tile count with the finest chunking the kernel may choose (64 tokens)
   const int chunks = (p->m_max + 63) / 64;
   if (p->N >= 2 * BM && g_use_pairs) {
@@ -1548,12 +1619,24 @@ extern "C" void* rd_gemm_plan_create(const void* A, int64_t lda, int m_max, cons
   p->K = K;
   bool ok = make_map(&p->map_a, A, lda, m_max, K, 128) && make_map(&p->map_w, W, ldw, N, K, BM);
   for (int i = 0; ok && i < 4; ++i) ok = make_map(&p->maps_a.m[i], A, lda, m_max, K, (i + 1) * kTokBox);
+  p->rows = rows_shape(m_max, N, K);
+  if (p->rows.rows > 0) {
+    ok = ok && make_map_blocks(&p->map_rows_w, W, ldw, N, K, p->rows.rows, p->rows.kb);
+    for (int i = 0; ok && i <= row_map_index(m_max); ++i)
+      ok = make_map_blocks(&p->maps_rows_a.m[i], A, lda, m_max, K, row_map_rows(i), p->rows.kb);
+  }
   if (!ok) {
     delete p;
     return nullptr;
   }
   return p;
 }
+
+extern "C" void rd_gemm_plan_early(void* plan) {
+  if (plan) static_cast<GemmPlan*>(plan)->rows.early = 1;
+}
+
+extern "C" int rd_gemm_few_rows(int m_max, int N, int K) { return m_max >= 1 && N >= 1 && rows_shape(m_max, N, K).rows > 0 ? 1 : 0; }
 
 extern "C" void rd_gemm_plan_destroy(void* plan) { delete static_cast<GemmPlan*>(plan); }
 

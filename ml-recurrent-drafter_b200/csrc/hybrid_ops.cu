@@ -22,8 +22,11 @@ __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
   extern __shared__ float smem[];
   float* row = smem;              // [H]
   float* part_sum = smem + H;     // [groups * parts]
-  rd::pdl_launch_dependents();
+  // the first kernel of a step: what follows may read weights ahead of its own wait (rd_gemm_plan_early)
+  const bool first = table != nullptr;
+  if (!first) rd::pdl_launch_dependents();
   rd::pdl_wait();
+  if (first) rd::pdl_launch_dependents();
   const int t = blockIdx.x;
   const int M = rd::live_rows(m_dev, m_max);
   if (t >= M) return;

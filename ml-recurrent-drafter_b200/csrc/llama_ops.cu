@@ -8,8 +8,8 @@ namespace {
 template <typename T>
 __global__ void embed_gather_kernel(const T* table, const int64_t* ids, T* out,
                                     int m_max, const int32_t* m_dev, int H, int vec) {
-  rd::pdl_launch_dependents();
   rd::pdl_wait();
+  rd::pdl_launch_dependents();  // what follows may read weights ahead of its own wait (rd_gemm_plan_early)
   const int t = blockIdx.x;
   if (t >= rd::live_rows(m_dev, m_max)) return;
   const T* src = table + ids[t] * (int64_t)H;

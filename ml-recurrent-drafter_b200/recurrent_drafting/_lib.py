@@ -57,6 +57,8 @@ SIGNATURES = {
     "rd_gemm_bf16_tc_slicemax": (_I, [_P, _I, _P, _L, _P, _P, _L, _P, _P]),
     "rd_vocab_topk_sliced": (_I, [_I, _P, _L, _I, _P, _I, _I, _F, _I, _F, _P, _L, _P, _P, _P, _P, _P]),
     "rd_embed_gather": (_I, [_I, _P, _P, _P, _I, _P, _I, _P]),
+    "rd_gemm_plan_early": (None, [_P]),
+    "rd_gemm_few_rows": (_I, [_I, _I, _I]),
     "rd_gemm_shares_bytes": (_L, [_I, _I, _I]),
     "rd_gemm_bf16_tc_res_shares": (_I, [_P, _I, _P, _L, _P, _L, _P, _P, _L, _P, _P]),
     "rd_rmsnorm_shares": (_I, [_I, _P, _P, _P, _I, _P, _P, _I, _P, _I, _F, _P]),

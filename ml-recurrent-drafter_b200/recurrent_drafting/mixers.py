@@ -39,6 +39,11 @@ class StepContext:
     parts: Optional[torch.Tensor] = None  # where the projections with a residual may leave their rows in shares of K
     pending: Optional[PendingRows] = None  # the rows that the last such projection left there: the next norm forms them
 
+    def add_residual(self, lin: Linear, a: torch.Tensor, out: torch.Tensor, residual: torch.Tensor) -> None:
+        """out = a W^T + residual, or, where shares pay, their rows in `parts` for the next norm."""
+        parts = None if lin.few_rows(self.m_max) else self.parts
+        self.pending = lin.add_residual(a, out, residual, self.m_dev, self.m_max, self.status, parts, early=True)
+
 
 @dataclass(frozen=True)
 class Visibility:
@@ -246,14 +251,14 @@ class GroupedAttention(_Mixer):
             self._attend_128(ctx, state, q, gate, mixed)
         else:
             self._attend(ctx, state, q, gate, mixed)
-        ctx.pending = self.lin[1].add_residual(mixed, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
+        ctx.add_residual(self.lin[1], mixed, out, residual)
 
     def _project(self, ctx: StepContext, state, xn):
         """Projection, then rotation, norm and cache append.  Returns the queries' rows and the gates."""
         c, st = self.cfg, _lib.stream()
         code, ld = _lib.dtype_code(self.w_in.dtype), row_stride(self.w_in.shape[0])
         proj = rows_of(ctx.ws["proj"], ld)
-        self.lin[0](xn, proj, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        self.lin[0](xn, proj, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status, early=True)
         cos, sin = self.rotary.get(c.rot_dims, c.rot_base, ctx.n_pos, xn.device)
         common = (_lib.ptr(proj), ld, _lib.ptr(state.keys), _lib.ptr(state.values), _lib.ptr(ctx.tok_row), _lib.ptr(ctx.tok_pos),
                   _lib.ptr(ctx.tok_slot), _lib.ptr(cos), _lib.ptr(sin), ctx.n_pos, ctx.m_max, _lib.ptr(ctx.m_dev), c.heads, c.kv_heads, c.dim)
@@ -279,11 +284,11 @@ class GroupedAttention(_Mixer):
         cos, sin = self.rotary.get(c.rot_dims, c.rot_base, ctx.n_pos, xn.device, head=128)
         if not self.gated:
             self.lin[0].qk_rope_norm(xn, q, state.keys, state.values, ctx.tok_row, ctx.tok_pos, ctx.tok_slot, cos, sin, c.heads, c.kv_heads,
-                                     c.rot_dims, self.unit_norm_eps, ctx.m_dev, ctx.m_max, ctx.status)
+                                     c.rot_dims, self.unit_norm_eps, ctx.m_dev, ctx.m_max, ctx.status, early=True)
             return q, None
         gate = rows_of(ctx.ws["head_gate"], row_stride(c.heads))
         self.lin[0].qkvg_rope(xn, q, state.keys, state.values, gate, ctx.tok_row, ctx.tok_pos, ctx.tok_slot, cos, sin, c.heads, c.kv_heads,
-                              c.rot_dims, ctx.m_dev, ctx.m_max, ctx.status)
+                              c.rot_dims, ctx.m_dev, ctx.m_max, ctx.status, early=True)
         return q, gate
 
     def _tensor_core_prompt(self, ctx: StepContext, q: torch.Tensor) -> bool:
@@ -385,9 +390,9 @@ class LatentAttention(_Mixer):
         c, ws = self.cfg, ctx.ws
         q, dkv = rows_of(ws["proj"], row_stride(self.n_split)), rows_of(ws["latent"], row_stride(self.width))
         mixed = rows_of(ws["mixed"], c.heads * c.vdim)
-        self.lin[0].split(xn, q, dkv, self.n_split, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        self.lin[0].split(xn, q, dkv, self.n_split, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status, early=True)
         (self._expanded if self._expands(ctx) else self._absorbed)(ctx, state, q, dkv, mixed)
-        ctx.pending = self.lin[1].add_residual(mixed, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
+        ctx.add_residual(self.lin[1], mixed, out, residual)
 
     def _append(self, ctx: StepContext, state, q, dkv, q_rot: torch.Tensor, rot_head: int) -> None:
         """Latents and key parts to the cache; the queries' rotated features to q_rot (rows as q_rot's, heads rot_head apart)."""
@@ -530,14 +535,14 @@ class MatrixMemory(_Mixer):
             proj = rows_of(ws["proj"], ld)
             gates = rows_of(ws["gates"], 2 * c.heads)
         mixed = rows_of(ws["mixed"], c.heads * c.vdim)
-        self.lin[0].split(xn, proj, gates, self.n_split, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        self.lin[0].split(xn, proj, gates, self.n_split, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status, early=True)
         if tree:
             self._tree(ctx, state, proj, gates, mixed)
         elif self._chunked(ctx):
             self._chunk(ctx, state, proj, gates, mixed)
         else:
             self._scan(ctx.batch, ctx.row_start, ctx.base_len, ctx.max_new, state, proj, gates, mixed)
-        ctx.pending = self.lin[1].add_residual(mixed, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
+        ctx.add_residual(self.lin[1], mixed, out, residual)
 
     def _chunked(self, ctx: StepContext) -> bool:
         """Prompts of a bf16 model; portions of a few tokens are run one after the other."""
@@ -598,7 +603,7 @@ class _FeedForward(nn.Module):
     def run(self, ctx: StepContext, xn: torch.Tensor, residual: torch.Tensor, out: torch.Tensor) -> None:
         act = rows_of(ctx.ws["act"], row_stride(self.ff))
         self._activate(ctx, xn, act)
-        ctx.pending = self.lin[1].add_residual(act, out, residual, ctx.m_dev, ctx.m_max, ctx.status, ctx.parts)
+        ctx.add_residual(self.lin[1], act, out, residual)
 
 
 class DenseFeedForward(_FeedForward):
@@ -627,7 +632,7 @@ class DenseFeedForward(_FeedForward):
         self.coeff = (softplus(p), 0.5 + softplus(q))
 
     def _activate(self, ctx: StepContext, xn: torch.Tensor, act: torch.Tensor) -> None:
-        self.lin[0].xielu(xn, act, *self.coeff, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        self.lin[0].xielu(xn, act, *self.coeff, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status, early=True)
 
 
 class ClampedGatedFeedForward(_FeedForward):
@@ -646,4 +651,4 @@ class ClampedGatedFeedForward(_FeedForward):
         return {"gate": self.up.detach()[0::2], "up": self.up.detach()[1::2], "down": self.down.detach()}
 
     def _activate(self, ctx: StepContext, xn: torch.Tensor, act: torch.Tensor) -> None:
-        self.lin[0].clamped_glu(xn, act, self.limit, self.alpha, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status)
+        self.lin[0].clamped_glu(xn, act, self.limit, self.alpha, m_dev=ctx.m_dev, m_max=ctx.m_max, status=ctx.status, early=True)

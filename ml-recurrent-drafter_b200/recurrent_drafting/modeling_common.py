@@ -15,6 +15,7 @@ class Linear:
         self.bias = bias
         self._plans: Dict[Tuple, int] = {}
         self._shares_bytes: Dict[int, int] = {}  # by row capacity
+        self._few_rows: Dict[int, bool] = {}
 
     MAX_SHARE_ROWS = 1024  # row capacities above this are never cut (rd_gemm_shares_bytes)
     MAX_PLANS = 32  # distinct (activation buffer, row capacity) pairs remembered per weight
@@ -43,14 +44,18 @@ class Linear:
             and self.weight.data_ptr() % 16 == 0
         )
 
-    def _plan(self, a: torch.Tensor, lda: int, m_max: int) -> int:
+    def _plan(self, a: torch.Tensor, lda: int, m_max: int, early: bool = False) -> int:
+        """early: the weight may be read before the kernels ahead in the stream have finished (rd_gemm_plan_early); for calls in a
+        chain of launches that begins with an embedding or a drafter's staging kernel and writes no weight."""
         n, k = self.weight.shape
-        key = (a.data_ptr(), lda, m_max)
+        key = (a.data_ptr(), lda, m_max, early)
         plan = self._plans.get(key)
         if plan is None:
             plan = _lib.load().rd_gemm_plan_create(_lib.ptr(a), lda, m_max, _lib.ptr(self.weight), self.weight.stride(0), n, k)
             if not plan:
                 raise _lib.RedrafterError("rd_gemm_plan_create failed (TMA descriptor could not be encoded)")
+            if early:
+                _lib.load().rd_gemm_plan_early(plan)
             if len(self._plans) >= self.MAX_PLANS:
                 self.drop_plans()
             self._plans[key] = plan
@@ -58,12 +63,12 @@ class Linear:
 
     def qkv_rope(self, a: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, tok_row, tok_pos,
                  tok_slot, cos: torch.Tensor, sin: torch.Tensor, nh: int, nkv: int, hd: int, m_dev, m_max: int,
-                 status: Optional[torch.Tensor], norm=None) -> None:
+                 status: Optional[torch.Tensor], norm=None, early: bool = False) -> None:
         """This weight as the packed QKV projection with rotary embedding and cache append in the
         GEMM epilogue (rd_gemm_bf16_tc_qkv_rope); tensor-core path only."""
         if not self._tc_ok(a, a.stride(0)):
             raise _lib.RedrafterError("the fused QKV projection needs the tensor-core GEMM path (bf16, aligned operands)")
-        plan = self._plan(a, a.stride(0), m_max)
+        plan = self._plan(a, a.stride(0), m_max, early)
         if norm is not None:
             # `a` holds gamma-scaled, not normalised rows: the 1 / rms of each row is applied in the epilogue
             ss, dim, eps = norm
@@ -78,25 +83,25 @@ class Linear:
 
     def qkvg_rope(self, a: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, gate_out: torch.Tensor,
                   tok_row, tok_pos, tok_slot, cos: torch.Tensor, sin: torch.Tensor, nh: int, nkv: int, rot_dims: int, m_dev,
-                  m_max: int, status: Optional[torch.Tensor]) -> None:
+                  m_max: int, status: Optional[torch.Tensor], early: bool = False) -> None:
         """This weight as the packed q, k, v and head-gate projection of heads of 128 features, with rotary embedding on
         rot_dims of them and the cache append in the epilogue (rd_gemm_bf16_tc_qkvg_rope); tensor-core path only."""
         if not self._tc_ok(a, a.stride(0)):
             raise _lib.RedrafterError("the fused QKV projection needs the tensor-core GEMM path (bf16, aligned operands)")
-        plan = self._plan(a, a.stride(0), m_max)
+        plan = self._plan(a, a.stride(0), m_max, early)
         _lib.call("rd_gemm_bf16_tc_qkvg_rope", plan, _lib.ptr(m_dev), _lib.ptr(q_out), _lib.ptr(k_cache), _lib.ptr(v_cache),
                   _lib.ptr(gate_out), gate_out.stride(0), _lib.ptr(tok_row), _lib.ptr(tok_pos), _lib.ptr(tok_slot), _lib.ptr(cos),
                   _lib.ptr(sin), cos.shape[0], nh, nkv, 128, rot_dims, k_cache.shape[2], _lib.ptr(status), _lib.stream())
 
     def qk_rope_norm(self, a: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, tok_row, tok_pos, tok_slot,
                      cos: torch.Tensor, sin: torch.Tensor, nh: int, nkv: int, rot_dims: int, eps: float, m_dev, m_max: int,
-                     status: Optional[torch.Tensor]) -> None:
+                     status: Optional[torch.Tensor], early: bool = False) -> None:
         """This weight as the packed q and k projection of heads of 128 features whose values are the keys: rotary embedding
         on rot_dims features, division by the head's root mean square and the append of keys and values in the epilogue
         (rd_gemm_bf16_tc_qk_rope_norm); tensor-core path only."""
         if not self._tc_ok(a, a.stride(0)):
             raise _lib.RedrafterError("the fused QK projection needs the tensor-core GEMM path (bf16, aligned operands)")
-        plan = self._plan(a, a.stride(0), m_max)
+        plan = self._plan(a, a.stride(0), m_max, early)
         _lib.call("rd_gemm_bf16_tc_qk_rope_norm", plan, _lib.ptr(m_dev), _lib.ptr(q_out), _lib.ptr(k_cache), _lib.ptr(v_cache),
                   _lib.ptr(tok_row), _lib.ptr(tok_pos), _lib.ptr(tok_slot), _lib.ptr(cos), _lib.ptr(sin), cos.shape[0], nh, nkv, 128,
                   rot_dims, k_cache.shape[2], eps, _lib.ptr(status), _lib.stream())
@@ -124,19 +129,30 @@ class Linear:
             self._shares_bytes[rows] = need
         return need
 
+    def few_rows(self, m_max: int) -> bool:
+        """Calls for this many rows go through the kernel for few tokens, which has no use for shares (rd_gemm_few_rows)."""
+        if m_max > 256:
+            return False
+        got = self._few_rows.get(m_max)
+        if got is None:
+            n, k = self.weight.shape
+            got = self.weight.dtype == torch.bfloat16 and bool(_lib.load().rd_gemm_few_rows(m_max, n, k))
+            self._few_rows[m_max] = got
+        return got
+
     def add_residual(self, a: torch.Tensor, c: torch.Tensor, residual: torch.Tensor, m_dev, m_max: int, status: Optional[torch.Tensor],
-                     parts: Optional[torch.Tensor] = None) -> Optional["PendingRows"]:
+                     parts: Optional[torch.Tensor] = None, early: bool = False) -> Optional["PendingRows"]:
         """c = a W^T + residual.  With `parts` given (fp32), few rows are left there in shares of K instead: then the result
         says what the norm that follows has to add up (rd_gemm_bf16_tc_res_shares)."""
         n, k = self.weight.shape
         if parts is not None and self._tc_ok(a, a.stride(0)):
             need = self.shares_bytes(m_max)
             if 0 < need <= parts.numel() * 4 and (c.data_ptr() | residual.data_ptr()) % 16 == 0 and c.stride(0) == residual.stride(0) == n:
-                plan = self._plan(a, a.stride(0), m_max)
+                plan = self._plan(a, a.stride(0), m_max, early)
                 _lib.call("rd_gemm_bf16_tc_res_shares", plan, _lib.dtype_code(c.dtype), _lib.ptr(c), n, _lib.ptr(residual), n, _lib.ptr(m_dev),
                           _lib.ptr(parts), parts.numel() * 4, _lib.ptr(status), _lib.stream())
                 return PendingRows(residual, parts, k)
-        self(a, c, _lib.EPI_RES, residual=residual, m_dev=m_dev, m_max=m_max, status=status)
+        self(a, c, _lib.EPI_RES, residual=residual, m_dev=m_dev, m_max=m_max, status=status, early=early)
         return None
 
     def swiglu_normed(self, a: torch.Tensor, c: torch.Tensor, ss: torch.Tensor, dim: int, eps: float, m_dev, m_max: int,
@@ -160,7 +176,7 @@ class Linear:
                   _lib.ptr(status), _lib.stream())
 
     def with_slice_max(self, a: torch.Tensor, c: torch.Tensor, slice_max: torch.Tensor, m_dev=None, m_max: Optional[int] = None,
-                       status: Optional[torch.Tensor] = None) -> bool:
+                       status: Optional[torch.Tensor] = None, early: bool = False) -> bool:
         """c = a W^T plus the per-(32 outputs, row) maxima of c in slice_max [N/32, >= m_max]
         (rd_gemm_bf16_tc_slicemax).  Returns False, doing nothing, when the shapes rule it out."""
         n, k = self.weight.shape
@@ -169,18 +185,18 @@ class Linear:
         if not (self._tc_ok(a, a.stride(0)) and n % 32 == 0 and c.data_ptr() % 16 == 0 and (c.stride(0) * esz) % 16 == 0
                 and slice_max.shape[0] * 32 == n and slice_max.stride(0) >= m_max):
             return False
-        plan = self._plan(a, a.stride(0), m_max)
+        plan = self._plan(a, a.stride(0), m_max, early)
         _lib.call("rd_gemm_bf16_tc_slicemax", plan, _lib.dtype_code(c.dtype), _lib.ptr(c), c.stride(0), _lib.ptr(m_dev),
                   _lib.ptr(slice_max), slice_max.stride(0), _lib.ptr(status), _lib.stream())
         return True
 
     def xielu(self, a: torch.Tensor, c: torch.Tensor, pos: float, neg: float, m_dev=None, m_max: Optional[int] = None,
-              status: Optional[torch.Tensor] = None) -> None:
+              status: Optional[torch.Tensor] = None, early: bool = False) -> None:
         """c = xIELU(a W^T) with the activation in the epilogue."""
         n, k = self.weight.shape
         m_max = a.shape[0] if m_max is None else m_max
         if self._tc_ok(a, a.stride(0)):
-            plan = self._plan(a, a.stride(0), m_max)
+            plan = self._plan(a, a.stride(0), m_max, early)
             _lib.call("rd_gemm_bf16_tc_xielu", plan, _lib.ptr(c), c.stride(0), _lib.ptr(m_dev), pos, neg, _lib.ptr(status),
                       _lib.stream())
         else:
@@ -188,13 +204,13 @@ class Linear:
                       self.weight.stride(0), _lib.ptr(c), c.stride(0), m_max, _lib.ptr(m_dev), n, k, pos, neg, _lib.stream())
 
     def clamped_glu(self, a: torch.Tensor, c: torch.Tensor, limit: float, alpha: float, m_dev=None, m_max: Optional[int] = None,
-                    status: Optional[torch.Tensor] = None) -> None:
+                    status: Optional[torch.Tensor] = None, early: bool = False) -> None:
         """c = g sigmoid(alpha g) (u + 1) of the interleaved (gate, up) rows of this weight, g and u cut at limit, in the
         epilogue."""
         n, k = self.weight.shape
         m_max = a.shape[0] if m_max is None else m_max
         if self._tc_ok(a, a.stride(0)):
-            plan = self._plan(a, a.stride(0), m_max)
+            plan = self._plan(a, a.stride(0), m_max, early)
             _lib.call("rd_gemm_bf16_tc_clamped_glu", plan, _lib.ptr(c), c.stride(0), _lib.ptr(m_dev), limit, alpha, _lib.ptr(status),
                       _lib.stream())
         else:
@@ -202,12 +218,12 @@ class Linear:
                       self.weight.stride(0), _lib.ptr(c), c.stride(0), m_max, _lib.ptr(m_dev), n, k, limit, alpha, _lib.stream())
 
     def split(self, a: torch.Tensor, c: torch.Tensor, c_hi: torch.Tensor, n_split: int, m_dev=None,
-              m_max: Optional[int] = None, status: Optional[torch.Tensor] = None) -> None:
+              m_max: Optional[int] = None, status: Optional[torch.Tensor] = None, early: bool = False) -> None:
         """Output features [0, n_split) of a W^T to c in its dtype, the rest to c_hi in fp32."""
         n, k = self.weight.shape
         m_max = a.shape[0] if m_max is None else m_max
         if self._tc_ok(a, a.stride(0)):
-            plan = self._plan(a, a.stride(0), m_max)
+            plan = self._plan(a, a.stride(0), m_max, early)
             _lib.call("rd_gemm_bf16_tc_split", plan, _lib.ptr(c), c.stride(0), _lib.ptr(c_hi), c_hi.stride(0), n_split,
                       _lib.ptr(m_dev), _lib.ptr(status), _lib.stream())
             return
@@ -218,7 +234,8 @@ class Linear:
 
     def __call__(self, a: torch.Tensor, c: torch.Tensor, epilogue: int = _lib.EPI_NONE, residual=None,
                  m_dev: Optional[torch.Tensor] = None, lda: Optional[int] = None, ldc: Optional[int] = None,
-                 ldr: Optional[int] = None, m_max: Optional[int] = None, status: Optional[torch.Tensor] = None) -> None:
+                 ldr: Optional[int] = None, m_max: Optional[int] = None, status: Optional[torch.Tensor] = None,
+                 early: bool = False) -> None:
         n, k = self.weight.shape
         m_max = a.shape[0] if m_max is None else m_max
         lda = a.stride(0) if lda is None else lda
@@ -231,7 +248,7 @@ class Linear:
             residual is None or (residual.data_ptr() % 16 == 0 and (ldr * esz) % 16 == 0)
         )
         if self._tc_ok(a, lda) and aligned:
-            plan = self._plan(a, lda, m_max)
+            plan = self._plan(a, lda, m_max, early)
             _lib.call("rd_gemm_bf16_tc", plan, out_code, _lib.ptr(c), ldc, _lib.ptr(self.bias), _lib.ptr(residual),
                       ldr or 0, _lib.ptr(m_dev), epilogue, _lib.ptr(status), _lib.stream())
         else:

@@ -285,23 +285,23 @@ class Drafter(torch.nn.Module):
             q_k = ws["q_first"] if shared else ws["q"][k]
             # recurrent update, written into the state half of x
             if lin["rnn"] is not None:
-                lin["rnn"](a_k, x_k[:, H:], _lib.EPI_BIAS_SILU, ldc=x_k.stride(0))
+                lin["rnn"](a_k, x_k[:, H:], _lib.EPI_BIAS_SILU, ldc=x_k.stride(0), early=True)
             else:
                 x_k[:, H:].copy_(a_k[:, H:])  # the prepare kernel already formed embedding + parent state
             cur = x_k
             yi = 0
             if lin["proj"] is not None:
-                lin["proj"](cur, ys[yi], _lib.EPI_BIAS)
+                lin["proj"](cur, ys[yi], _lib.EPI_BIAS, early=True)
                 cur, yi = ys[yi], yi + 1
             for res in lin["res"]:
                 nxt = ys[yi % 3]
-                res(cur, nxt, _lib.EPI_BIAS_SILU_RES, residual=cur)
+                res(cur, nxt, _lib.EPI_BIAS_SILU_RES, residual=cur, early=True)
                 cur, yi = nxt, yi + 1
             smax = ws["slice_max"] if os.environ.get("RD_FUSED_HEAD", "1") != "0" else None
-            if smax is not None and not shared and lin["vocab"].with_slice_max(cur, logits_k, smax):
+            if smax is not None and not shared and lin["vocab"].with_slice_max(cur, logits_k, smax, early=True):
                 vocab_topk(logits_k, q_k, subtract_max=True, slice_max=smax)
             else:
-                lin["vocab"](cur, logits_k)
+                lin["vocab"](cur, logits_k, early=True)
                 vocab_topk(logits_k, q_k, subtract_max=True)
             if shared:
                 q = ws["q"][0]

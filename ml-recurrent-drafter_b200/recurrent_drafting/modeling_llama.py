@@ -376,6 +376,10 @@ class LlamaForCausalLM(LMHead, nn.Module):
                 _lib.call("rd_rmsnorm_shares", code, _lib.ptr(h), _lib.ptr(pending.residual), _lib.ptr(pending.parts), pending.k,
                           _lib.ptr(weight), _lib.ptr(y), m_max, md, H, self.eps, st)
 
+        def add_residual(lin_l, a):
+            return lin_l.add_residual(a, h, h, m_dev, m_max, self.gemm_status, None if lin_l.few_rows(m_max) else parts, early=True)
+
+        # `early`: everything below follows the embedding kernel, and nothing in it writes a weight
         pending = None
         for l in range(self.n_layers):
             if not fused_norm or l == 0:
@@ -384,9 +388,9 @@ class LlamaForCausalLM(LMHead, nn.Module):
             if fused_rope:
                 # rotary embedding and the cache append ride on the projection's epilogue
                 lin["qkv"][l].qkv_rope(xn, q, kc, vc, tok_row, tok_pos, tok_slot, cos, sin, nh, nkv, hd, m_dev, m_max,
-                                       self.gemm_status, norm=(ss, H, self.eps) if fused_norm and l > 0 else None)
+                                       self.gemm_status, norm=(ss, H, self.eps) if fused_norm and l > 0 else None, early=True)
             else:
-                lin["qkv"][l](xn, qkv, _lib.EPI_NONE, m_dev=m_dev, m_max=m_max, status=self.gemm_status)
+                lin["qkv"][l](xn, qkv, _lib.EPI_NONE, m_dev=m_dev, m_max=m_max, status=self.gemm_status, early=True)
                 _lib.call("rd_rope_kv_write", code, _lib.ptr(qkv), _lib.ptr(q), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(tok_row),
                           _lib.ptr(tok_pos), _lib.ptr(tok_slot), _lib.ptr(cos), _lib.ptr(sin), cos.shape[0], m_max, md, nh, nkv,
                           hd, max_len, st)
@@ -400,10 +404,10 @@ class LlamaForCausalLM(LMHead, nn.Module):
                 else:
                     lin["down"][l](act, h, _lib.EPI_RES, residual=h, m_dev=m_dev, m_max=m_max, status=self.gemm_status)
                 continue
-            pending = lin["o"][l].add_residual(attn, h, h, m_dev, m_max, self.gemm_status, parts)
+            pending = add_residual(lin["o"][l], attn)
             norm(self.ln2[l], xn, pending)
-            lin["gu"][l](xn, act, _lib.EPI_SWIGLU, m_dev=m_dev, m_max=m_max, status=self.gemm_status)
-            pending = lin["down"][l].add_residual(act, h, h, m_dev, m_max, self.gemm_status, parts)
+            lin["gu"][l](xn, act, _lib.EPI_SWIGLU, m_dev=m_dev, m_max=m_max, status=self.gemm_status, early=True)
+            pending = add_residual(lin["down"][l], act)
         norm(self.norm, ws["hidden"], pending)
         return ws["hidden"]
 
