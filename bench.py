@@ -291,10 +291,10 @@ def run_ours(args):
 
     real_add_residual = _Linear.add_residual
 
-    def timed_add_residual(self, a, c, residual, m_dev, *pa):
+    def timed_add_residual(self, a, c, residual, m_dev, *pa, **kw):
         # leaves its rows in shares of K for few rows; where it may not, it comes down to __call__, which is counted there
         at = len(all_calls)
-        pending = real_add_residual(self, a, c, residual, m_dev, *pa)
+        pending = real_add_residual(self, a, c, residual, m_dev, *pa, **kw)
         if pending is not None:
             prof.append((at, self.weight.shape[0], self.weight.shape[1], a.shape[0] if m_dev is None else None))
         return pending

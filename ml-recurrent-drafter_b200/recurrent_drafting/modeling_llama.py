@@ -428,20 +428,20 @@ class LlamaForCausalLM(LMHead, nn.Module):
         assert S + q_len <= cache_tensor.shape[4]
         M = B * q_len
         i32 = dict(dtype=torch.int32, device=dev)
-        tok_row = torch.arange(B, **i32).repeat_interleave(q_len)
-        tok_slot = (S + torch.arange(q_len, **i32)).repeat(B)
-        tok_pos = position_ids.reshape(-1).clamp(min=0).to(torch.int32)
-        row_start = torch.arange(B + 1, **i32) * q_len
+        tok_row = torch.arange(B, **i32)[:, None].expand(B, q_len).reshape(-1)
+        tok_slot = torch.arange(S, S + q_len, **i32).repeat(B)
+        row_start = torch.arange(0, M + 1, q_len, **i32)
         kv_begin = torch.zeros(B, **i32)
         base_len = torch.full((B,), S, **i32)
+        tok_pos = position_ids.reshape(-1).clamp(min=0).to(torch.int32)
         dense = attention_mask.to(torch.uint8).contiguous()
-        ws = self.workspace(M, M)
+        ws = self.workspace(M, 1)
         n_pos = max(4096, int(S + q_len) + 1)
         hidden = self.backbone(ws, cache_tensor, M, None, input_ids.reshape(-1).contiguous(), tok_row, tok_pos, tok_slot,
                                row_start, kv_begin, base_len, B, q_len, S + q_len, _lib.ATTN_DENSE, dense_mask=dense,
                                n_pos=n_pos)
-        logits = self.lm_logits(hidden, ws["logits"])
+        V = self.config.vocab_size
+        logits = self.lm_logits(hidden, torch.empty(M, V, dtype=torch.float32, device=dev))  # the caller's: no copy out of the workspace
         for k, v in past_key_values:
             k.length = v.length = S + q_len
-        V = self.config.vocab_size
-        return CausalLMOutput(logits=logits.view(B, q_len, V).clone(), hidden_states=hidden.view(B, q_len, -1).clone())
+        return CausalLMOutput(logits=logits.view(B, q_len, V), hidden_states=hidden.view(B, q_len, -1).clone())
