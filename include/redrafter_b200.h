@@ -114,6 +114,14 @@ RD_API int rd_tree_pack_reference_layout(int B, int W, int Lb, const int32_t* un
  * (embedding + parent state, rounded once to the model type) and the caller copies it into x[r, H:2H]. */
 RD_API int rd_drafter_prepare(int dtype, const void* embed, const int64_t* beams, const int32_t* parent, const void* ctx,
                        void* a, void* x, int B, int W, int Lb, int H, int k, int additive, void* stream);
+/* rd_drafter_prepare of iteration 0 from the rows' start tokens init_tok[B], which become token 0 of every beam in beams. */
+RD_API int rd_drafter_begin(int dtype, const void* embed, const int64_t* init_tok, int64_t* beams, const void* ctx, void* a, void* x, int B,
+                     int W, int Lb, int H, int additive, void* stream);
+/* What the first iteration computed once for a batch row becomes that of all its beams: the sparse lists [B, 64] of rd_vocab_topk ->
+ * [B*W, 64], and the state x[b*W, H:2H] -> x[b*W+w, H:2H] (:170-177: the beams of a row start with one token and state). */
+RD_API int rd_drafter_spread(int dtype, const float* first_val, const int32_t* first_idx, const int32_t* first_cnt,
+                      const float* first_masked, float* val, int32_t* idx, int32_t* cnt, float* masked, void* x, int B, int W, int H,
+                      void* stream);
 
 /* Per-row top-k warp + log-softmax of a (rows, V) logits matrix, sparse output.  Replaces
  * maintain_logits, warp_logits and log_softmax (modeling_drafter.py:63-99, 201-203) and, for the
@@ -175,7 +183,7 @@ RD_API int rd_gemm(int dtype, int out_dtype, const void* A, int64_t lda, const v
 RD_API void* rd_gemm_plan_create(const void* A, int64_t lda, int m_max, const void* W, int64_t ldw, int N, int K);
 RD_API void rd_gemm_plan_destroy(void* plan);
 /* Launches of this plan may read W before the kernels ahead of them in the stream have finished.  For calls that follow, in one
- * chain of this library's launches, an rd_embed_gather, rd_stream_norm with ids or rd_drafter_prepare: these let what comes after
+ * chain of this library's launches, an rd_embed_gather, rd_stream_norm with ids, rd_drafter_begin or rd_drafter_prepare: these let what comes after
  * them start only when all that came before them is complete, so that W is as the stream's earlier work left it. */
 RD_API void rd_gemm_plan_early(void* plan);
 /* 1 if plans of this size are served by the kernel for few tokens (up to 256, fewer for matrices of few features; K a multiple of

@@ -270,12 +270,15 @@ class Drafter(torch.nn.Module):
         code = _lib.dtype_code(self.dtype)
         st = _lib.stream()
         a, x = ws["a"], ws["x"]
-        ws["beams"][0][:, :, 0] = init_token[:, None]
-        ctx = prompt_state.contiguous()
+        ctx, start = prompt_state.contiguous(), init_token.contiguous()
         for k in range(Lb - 1):
             bin_, bout = ws["beams"][k % 2], ws["beams"][(k + 1) % 2]
-            _lib.call("rd_drafter_prepare", code, _lib.ptr(embeddings.weight), _lib.ptr(bin_), _lib.ptr(ws["parent"]),
-                      _lib.ptr(ctx), _lib.ptr(a), _lib.ptr(x), B, W, Lb, H, k, 0 if cfg.rnn else 1, st)
+            if k == 0:
+                _lib.call("rd_drafter_begin", code, _lib.ptr(embeddings.weight), _lib.ptr(start), _lib.ptr(bin_), _lib.ptr(ctx), _lib.ptr(a),
+                          _lib.ptr(x), B, W, Lb, H, 0 if cfg.rnn else 1, st)
+            else:
+                _lib.call("rd_drafter_prepare", code, _lib.ptr(embeddings.weight), _lib.ptr(bin_), _lib.ptr(ws["parent"]),
+                          _lib.ptr(ctx), _lib.ptr(a), _lib.ptr(x), B, W, Lb, H, k, 0 if cfg.rnn else 1, st)
             # In the first iteration every beam of a row holds the same token, state and context
             # (modeling_drafter.py:170-177), so the W rows of a batch row are identical: compute row 0
             # of each (a view with row stride W) and copy its results to the others.
@@ -305,13 +308,8 @@ class Drafter(torch.nn.Module):
                 vocab_topk(logits_k, q_k, subtract_max=True)
             if shared:
                 q = ws["q"][0]
-                K = q.val.shape[1]
-                q.val.view(B, W, K).copy_(q_k.val.view(B, 1, K).expand(B, W, K))
-                q.idx.view(B, W, K).copy_(q_k.idx.view(B, 1, K).expand(B, W, K))
-                q.cnt.view(B, W).copy_(q_k.cnt.view(B, 1).expand(B, W))
-                q.masked.view(B, W).copy_(q_k.masked.view(B, 1).expand(B, W))
-                xs = x.view(B, W, 2 * H)
-                xs[:, 1:, H:].copy_(xs[:, :1, H:].expand(B, W - 1, H))
+                _lib.call("rd_drafter_spread", code, _lib.ptr(q_k.val), _lib.ptr(q_k.idx), _lib.ptr(q_k.cnt), _lib.ptr(q_k.masked),
+                          _lib.ptr(q.val), _lib.ptr(q.idx), _lib.ptr(q.cnt), _lib.ptr(q.masked), _lib.ptr(x), B, W, H, st)
             _lib.call("rd_beam_select", B, W, Lb, k, V, _lib.ptr(ws["q"][k].val), _lib.ptr(ws["q"][k].idx),
                       _lib.ptr(ws["q"][k].cnt), _lib.ptr(ws["score"][k % 2]), _lib.ptr(ws["score"][(k + 1) % 2]),
                       _lib.ptr(bin_), _lib.ptr(bout), _lib.ptr(ws["anc"][k % 2]), _lib.ptr(ws["anc"][(k + 1) % 2]),
