@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint64_t* v_full = bars + 3;    // [2]
   uint64_t* s_full = bars + 5;    // [2]: QK^T of even / odd tiles done; also frees that tile's K stage
   uint64_t* s_empty = bars + 7;
-  uint64_t* p_full = bars + 8;
+  uint64_t* p_full = bars + 15;   // [2]: even / odd tiles
   uint64_t* o_full = bars + 9;    // [2]: PV of even / odd tiles done; also frees that tile's V stage
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(kThreads, 2)
       mbar_init(&o_full[s], 1);
     }
     mbar_init(s_empty, 4);
-    mbar_init(p_full, 4);
+    mbar_init(&p_full[0], 4);
+    mbar_init(&p_full[1], 4);
     *abort_flag = 0;
     if (DENSE) {
       mbar_init(v_seen, 4);
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(kThreads, 2)
           issue_qk(t + 1);
         }
         // P of tile t is in TMEM (and O has been rescaled where needed); V of tile t has landed
-        if (!mbar_wait(p_full, t & 1, abort_flag)) {
+        if (!mbar_wait(&p_full[t & 1], (t >> 1) & 1, abort_flag)) {
           ok = false;
           break;
         }
@@ -522,6 +523,8 @@ __global__ void __launch_bounds__(kThreads, 2)
       const int p = mode == RD_ATTN_CAUSAL ? base + qi : (live ? win.tok_pos[rs + qi] : base);
       first_seen = rd_win::first_visible(win.mask_kind, win.window, p);
     }
+    // keys before this one are visible to all queries (before windows): the cached prefix, and those up to the first query
+    const int all_see = mode == RD_ATTN_CAUSAL ? base + q0 + 1 : base;
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     int site = 0;  // which wait gave up (reported in the status word)
@@ -565,8 +568,8 @@ __global__ void __launch_bounds__(kThreads, 2)
       uint64_t vis;
       if (DENSE) {
         vis = dense;
-      } else if (j0 + BNK <= base) {
-        vis = ~0ull;  // the whole tile lies in the cached prefix
+      } else if (j0 + BNK <= all_see) {
+        vis = ~0ull;  // every query of this CTA sees the whole tile
       } else {
         const int off = j0 - base;  // index of the tile's first key among the new tokens (may be negative)
         uint64_t nb;                // visibility of new tokens [max(off,0), ...) aligned to bit max(-off,0)
@@ -597,20 +600,22 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
       // Running max over the RAW scores (the scale is positive), masked keys set to -inf first.
       // exp2 then takes one FFMA per element: p = 2^(s*scale - m*scale).
-      float mx = -INFINITY;
-      if (__all_sync(0xffffffffu, vis == ~0ull)) {
-#pragma unroll
-        for (int i = 0; i < 64; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(sb[i]), __uint_as_float(sb[i + 1])));
-      } else {
+      if (!__all_sync(0xffffffffu, vis == ~0ull)) {
         const uint32_t vlo = (uint32_t)vis, vhi = (uint32_t)(vis >> 32);
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           if (!((vlo >> i) & 1u)) sb[i] = 0xff800000u;
           if (!((vhi >> i) & 1u)) sb[32 + i] = 0xff800000u;
         }
-#pragma unroll
-        for (int i = 0; i < 64; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(sb[i]), __uint_as_float(sb[i + 1])));
       }
+      float part[4];  // four chains: one of 64 waits for itself
+#pragma unroll
+      for (int i = 0; i < 4; ++i) part[i] = fmaxf(__uint_as_float(sb[i]), __uint_as_float(sb[4 + i]));
+#pragma unroll
+      for (int i = 8; i < 64; i += 8)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[j] = fmaxf(part[j], fmaxf(__uint_as_float(sb[i + j]), __uint_as_float(sb[i + 4 + j])));
+      const float mx = fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3]));
       // Lazy running max (in log2 units): it only moves when the tile's max exceeds it by more than
       // kMaxSlack, so P stays <= 2^kMaxSlack and O is rescaled rarely; l and O use the same max.
       const float mx2 = mx * scale_log2;
@@ -696,7 +701,6 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
       }
       l_run = l_run * (moved ? alpha : 1.0f) + (rowsum0 + rowsum1);
-      // P buffer t&1 was last read by PV of tile t-2, seen complete before this warp's arrival for tile t-1
       if (__any_sync(0xffffffffu, rescale)) {
         // O must be quiescent while it is rescaled: PV of tile t-1 has to be complete
         if (!mbar_wait(&o_full[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag)) {
@@ -717,18 +721,12 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
       if (!DENSE) tmem_st32(lane_addr + kColP + (t & 1) * 32, pb);
       tc_fence_before();
-      // The arrival for tile t must not be possible before the MMA thread has consumed the barrier's
-      // phase for tile t-1: the thread issues QK of tile t before it looks at that phase, so without
-      // this wait a fast softmax could complete two phases between two of its polls, and a parity
-      // wait cannot tell phase t-1 from phase t+1.  PV of tile t-1 complete implies it was consumed
-      // (and that no warp's arrival for tile t can be counted into the phase of tile t-1).
-      if (t >= 1 && !mbar_wait(&o_full[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag)) {
-        ok = false;
-        site = 4;
-        break;
-      }
+      // A parity wait cannot tell a phase from the one after next, so this barrier's phase of tile t - 2 has to have been consumed.
+      // It has: the scores of tile t were issued after that, and their barrier says that PV of tile t - 2 is done as well,
+      // which was issued before them and read this P buffer.  (With one barrier for all tiles every tile waited for PV of the one
+      // before it here, some 140 cycles of 1950.)
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&p_full[t & 1]);
     }
     if (ok && n_tiles > 0) {
       ok = mbar_wait(&o_full[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, abort_flag);
