@@ -10,125 +10,169 @@
 namespace {
 
 constexpr int kNormMaxThreads = 1024;
+constexpr int kNormWarmTokens = 64;
 
 // One block per token.  The row is formed in fp32 (embedding gather, or the weighted sum of `n_hist` stored
 // rows), written to x when asked for, kept in shared memory, and normalised in groups of H / groups
 // features: each group over its own sqrt(mean of squares + eps), the whole times w.
-template <typename T, int VEC, bool SHARES>
+// A row's stored rows are some 16 KB each, so few tokens pay for trips to memory one after the other: eight stored rows and the weight
+// are requested together.  warm: launches of few tokens run the body once on shared memory ahead of the dependency wait,
+// because its instructions come from L2 or memory the first time.  6 tokens of 4096 features, 2 .. 9 stored rows, in a decode step: 6.8
+// -> 6.1 us a launch; 8 tokens, one stored row 5.6 -> 4.8.
+template <typename T, int VEC, bool SHARES, bool FEW>
 __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
-    const T* table, const int64_t* ids, float embed_scale, float* hist,
-    int64_t hist_stride, const float* coeff, int n_hist, float* x_out, const T* w,
-    T* y, int m_max, const int32_t* m_dev, int H, int groups, int parts, float eps, rd::Shares<float> sh) {
+    const T* table, const int64_t* ids, float embed_scale, float* hist_,
+    int64_t hist_stride_, const float* coeff_, int n_hist_, float* x_out_, const T* w_,
+    T* y, int m_max, const int32_t* m_dev, int H, int groups, int parts, float eps, int warm, rd::Shares<float> sh) {
   extern __shared__ float smem[];
   float* row = smem;              // [H]
   float* part_sum = smem + H;     // [groups * parts]
+  const int tid = threadIdx.x, n_thr = blockDim.x;
+  constexpr int U = FEW ? 8 : 4;  // many tokens: more blocks on an SM instead
   // the first kernel of a step: what follows may read weights ahead of its own wait (rd_gemm_plan_early)
   const bool first = table != nullptr;
   if (!first) rd::pdl_launch_dependents();
-  rd::pdl_wait();
-  if (first) rd::pdl_launch_dependents();
-  const int t = blockIdx.x;
-  const int M = rd::live_rows(m_dev, m_max);
-  if (t >= M) return;
-  const int tid = threadIdx.x, n_thr = blockDim.x;
-  const bool shares = SHARES && rd::live_shares(sh.count, M) > 1;
-  if (table != nullptr) {
-    const T* src = table + ids[t] * (int64_t)H;
-    for (int d = tid * VEC; d < H; d += n_thr * VEC) {
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) row[d + e] = rd::Num<T>::to_f(src[d + e]) * embed_scale;
+#pragma unroll 1
+  for (int live = FEW && warm ? 0 : 1; live < 2; ++live) {
+    // without a live token: every row is the one in shared memory
+    float* stand_in = smem + ((H + groups * parts + 3) & ~3);  // [max(H, U)]
+    float *src = stand_in, *x_out = x_out_ ? stand_in : nullptr;
+    const float* coeff = coeff_ ? stand_in : nullptr;
+    int64_t hist_stride = 0;
+    int n_hist = coeff_ ? U : 1, t = 0;
+    const T* w = reinterpret_cast<const T*>(stand_in);
+    T* dst = reinterpret_cast<T*>(stand_in);
+    bool shares = SHARES;
+    rd::Shares<float> from{stand_in, stand_in, sh.count, 0};
+    if (live) {
+      rd::pdl_wait();
+      if (first) rd::pdl_launch_dependents();
+      t = blockIdx.x;
+      const int M = rd::live_rows(m_dev, m_max);
+      if (t >= M) return;
+      shares = SHARES && rd::live_shares(sh.count, M) > 1;
+      from = sh;
+      src = hist_ + (int64_t)t * H;
+      hist_stride = hist_stride_;
+      n_hist = n_hist_;
+      coeff = coeff_;
+      x_out = x_out_ ? x_out_ + (int64_t)t * H : nullptr;
+      w = w_;
+      dst = y + (int64_t)t * H;
     }
-  } else {
-    float* src = hist + (int64_t)t * H;
-    for (int d = tid * VEC; d < H; d += n_thr * VEC) {
-      float acc[VEC];
+    T g0[VEC];  // the weight of this thread's first features
+    if (tid * VEC < H) {
+      if constexpr (VEC == 4 && sizeof(T) == 2)
+        *reinterpret_cast<uint2*>(g0) = *reinterpret_cast<const uint2*>(w + tid * VEC);
+      else if constexpr (VEC == 4)
+        *reinterpret_cast<float4*>(g0) = *reinterpret_cast<const float4*>(w + tid * VEC);
+      else
+        g0[0] = w[tid];
+    }
+    if (live && table != nullptr) {
+      const T* e = table + ids[t] * (int64_t)H;
+      for (int d = tid * VEC; d < H; d += n_thr * VEC) {
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
-      if (shares) {
-        // the last stored row is still in shares: formed here, by the thread that reads it below
-        float f[VEC];
-        rd::add_shares<VEC>(sh, t, H, d, f);
-        float* dst = src + (int64_t)(n_hist - 1) * hist_stride + d;
-        if constexpr (VEC == 4)
-          *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
-        else
-          *dst = f[0];
+        for (int k = 0; k < VEC; ++k) row[d + k] = rd::Num<T>::to_f(e[d + k]) * embed_scale;
       }
-      if (coeff == nullptr) {
-        if constexpr (VEC == 4) {
-          *reinterpret_cast<float4*>(acc) = *reinterpret_cast<const float4*>(src + d);
-        } else {
-          acc[0] = src[d];
+    } else {
+      for (int d = tid * VEC; d < H; d += n_thr * VEC) {
+        float acc[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
+        if (shares) {
+          // the last stored row is still in shares: formed here, by the thread that reads it below
+          float f[VEC];
+          rd::add_shares<VEC>(from, t, H, d, f);
+          float* last = src + (int64_t)(n_hist - 1) * hist_stride + d;
+          if constexpr (VEC == 4)
+            *reinterpret_cast<float4*>(last) = make_float4(f[0], f[1], f[2], f[3]);
+          else
+            *last = f[0];
         }
-      } else {
-#pragma unroll 4
-        for (int j = 0; j < n_hist; ++j) {
-          const float c = coeff[j];
+        if (coeff == nullptr) {
           if constexpr (VEC == 4) {
-            const float4 f = *reinterpret_cast<const float4*>(src + (int64_t)j * hist_stride + d);
-            acc[0] = fmaf(c, f.x, acc[0]);
-            acc[1] = fmaf(c, f.y, acc[1]);
-            acc[2] = fmaf(c, f.z, acc[2]);
-            acc[3] = fmaf(c, f.w, acc[3]);
+            *reinterpret_cast<float4*>(acc) = *reinterpret_cast<const float4*>(src + d);
           } else {
-            acc[0] = fmaf(c, src[(int64_t)j * hist_stride + d], acc[0]);
+            acc[0] = src[d];
+          }
+        } else {
+          for (int j0 = 0; j0 < n_hist; j0 += U) {
+            float f[U][VEC], c[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const bool in = j0 + u < n_hist;
+              c[u] = in ? coeff[j0 + u] : 0.f;
+              if constexpr (VEC == 4)
+                *reinterpret_cast<float4*>(f[u]) = in ? *reinterpret_cast<const float4*>(src + (int64_t)(j0 + u) * hist_stride + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+              else
+                f[u][0] = in ? src[(int64_t)(j0 + u) * hist_stride + d] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              if (j0 + u >= n_hist) break;
+#pragma unroll
+              for (int e = 0; e < VEC; ++e) acc[e] = fmaf(c[u], f[u][e], acc[e]);
+            }
           }
         }
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) row[d + e] = acc[e];
       }
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) row[d + e] = acc[e];
     }
-  }
-  __syncthreads();
-  if (x_out != nullptr) {
-    float* dst = x_out + (int64_t)t * H;
+    __syncthreads();
+    if (x_out != nullptr) {
+      for (int d = tid * VEC; d < H; d += n_thr * VEC) {
+        if constexpr (VEC == 4)
+          *reinterpret_cast<float4*>(x_out + d) = *reinterpret_cast<const float4*>(row + d);
+        else
+          x_out[d] = row[d];
+      }
+    }
+    // sums of squares: every group is cut into `parts` interleaved shares, one warp each
+    const int warp = tid >> 5, lane = tid & 31;
+    const int gsize = H / groups;
+    for (int u = warp; u < groups * parts; u += (n_thr / 32)) {
+      const float* g = row + (u / parts) * gsize;
+      float ss = 0.f;
+      for (int d = (u % parts) * 32 + lane; d < gsize; d += 32 * parts) ss = fmaf(g[d], g[d], ss);
+      ss = rd::warp_sum(ss);
+      if (lane == 0) part_sum[u] = ss;
+    }
+    __syncthreads();
+    // one scale per group, left in the place of its first share
+    for (int g = tid; g < groups; g += n_thr) {
+      float tot = 0.f;
+      for (int p = 0; p < parts; ++p) tot += part_sum[g * parts + p];
+      part_sum[g * parts] = 1.0f / sqrtf(tot / (float)gsize + eps);
+    }
+    __syncthreads();
+    const bool whole = gsize % VEC == 0;  // a vector lies in one group
     for (int d = tid * VEC; d < H; d += n_thr * VEC) {
-      if constexpr (VEC == 4)
-        *reinterpret_cast<float4*>(dst + d) = *reinterpret_cast<const float4*>(row + d);
-      else
-        dst[d] = row[d];
-    }
-  }
-  // sums of squares: every group is cut into `parts` interleaved shares, one warp each
-  const int warp = tid >> 5, lane = tid & 31;
-  const int gsize = H / groups;
-  for (int u = warp; u < groups * parts; u += (n_thr / 32)) {
-    const float* g0 = row + (u / parts) * gsize;
-    float ss = 0.f;
-    for (int d = (u % parts) * 32 + lane; d < gsize; d += 32 * parts) ss = fmaf(g0[d], g0[d], ss);
-    ss = rd::warp_sum(ss);
-    if (lane == 0) part_sum[u] = ss;
-  }
-  __syncthreads();
-  // one scale per group, left in the place of its first share
-  for (int g = tid; g < groups; g += n_thr) {
-    float tot = 0.f;
-    for (int p = 0; p < parts; ++p) tot += part_sum[g * parts + p];
-    part_sum[g * parts] = 1.0f / sqrtf(tot / (float)gsize + eps);
-  }
-  __syncthreads();
-  T* dst = y + (int64_t)t * H;
-  const bool whole = gsize % VEC == 0;  // a vector lies in one group
-  for (int d = tid * VEC; d < H; d += n_thr * VEC) {
-    T o[VEC], g[VEC];
-    if constexpr (VEC == 4 && sizeof(T) == 2)
-      *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(w + d);
-    else if constexpr (VEC == 4)
-      *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(w + d);
-    else
-      g[0] = w[d];
-    float rs = part_sum[(d / gsize) * parts];
+      T o[VEC], g[VEC];
+      if (d == tid * VEC) {
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) {
-      if (!whole) rs = part_sum[((d + e) / gsize) * parts];
-      o[e] = rd::Num<T>::from_f(row[d + e] * rs * rd::Num<T>::to_f(g[e]));
+        for (int e = 0; e < VEC; ++e) g[e] = g0[e];
+      } else if constexpr (VEC == 4 && sizeof(T) == 2)
+        *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(w + d);
+      else if constexpr (VEC == 4)
+        *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(w + d);
+      else
+        g[0] = w[d];
+      float rs = part_sum[(d / gsize) * parts];
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        if (!whole) rs = part_sum[((d + e) / gsize) * parts];
+        o[e] = rd::Num<T>::from_f(row[d + e] * rs * rd::Num<T>::to_f(g[e]));
+      }
+      if constexpr (VEC == 4 && sizeof(T) == 2)
+        *reinterpret_cast<uint2*>(dst + d) = *reinterpret_cast<const uint2*>(o);
+      else if constexpr (VEC == 4)
+        *reinterpret_cast<float4*>(dst + d) = *reinterpret_cast<const float4*>(o);
+      else
+        dst[d] = o[0];
     }
-    if constexpr (VEC == 4 && sizeof(T) == 2)
-      *reinterpret_cast<uint2*>(dst + d) = *reinterpret_cast<const uint2*>(o);
-    else if constexpr (VEC == 4)
-      *reinterpret_cast<float4*>(dst + d) = *reinterpret_cast<const float4*>(o);
-    else
-      dst[d] = o[0];
+    __syncthreads();  // the row and the sums are used again
   }
 }
 
@@ -245,23 +289,31 @@ static int stream_norm_launch(int dtype, const void* table, const int64_t* ids, 
   const bool vec = H % 4 == 0 && bits % 16 == 0 && hist_stride % 4 == 0;
   int threads = ((vec ? H / 4 : H) + 31) / 32 * 32;
   // few tokens: the row's loads all in flight at once; many tokens: small blocks, several per SM
-  const int most = m_max <= 2 * 148 ? kNormMaxThreads : 256;
+  const bool few = m_max <= 2 * 148;
+  const int most = few ? kNormMaxThreads : 256;
   threads = threads > most ? most : threads;
   const int warps = threads / 32;
   const int parts = groups >= warps ? 1 : (warps + groups - 1) / groups;
-  const size_t smem = ((size_t)H + (size_t)groups * parts) * sizeof(float);
+  size_t smem = ((size_t)H + (size_t)groups * parts) * sizeof(float);
   RD_REQUIRE(smem <= 200 * 1024, RD_ERR_SIZE);
+  // few tokens find room beside the kernel before, whose grid leaves some SMs free
+  const size_t with_stand_in = (((size_t)H + (size_t)groups * parts + 3) / 4 * 4 + (H < 8 ? 8 : H)) * sizeof(float);
+  const int warm = !table && m_max <= kNormWarmTokens && with_stand_in <= 64 * 1024;
+  if (warm) smem = with_stand_in;
   cudaError_t err = cudaSuccess;
   RD_DISPATCH_T(dtype, {
-    auto kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true> : stream_norm_kernel<T, 1, true>)
-                             : (vec ? stream_norm_kernel<T, 4, false> : stream_norm_kernel<T, 1, false>);
+    auto few_kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true, true> : stream_norm_kernel<T, 1, true, true>)
+                                 : (vec ? stream_norm_kernel<T, 4, false, true> : stream_norm_kernel<T, 1, false, true>);
+    auto many_kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true, false> : stream_norm_kernel<T, 1, true, false>)
+                                  : (vec ? stream_norm_kernel<T, 4, false, false> : stream_norm_kernel<T, 1, false, false>);
+    auto kern = few ? few_kern : many_kern;
     if (smem > 48 * 1024) {
       err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       RD_CHECK_CHAINED(err);
     }
     err = rd::launch_chained(kern, dim3(m_max), dim3(threads), smem, (cudaStream_t)stream, 1, (const T*)table, ids,
                              embed_scale, hist, hist_stride, coeff, n_hist, x_out, (const T*)weight, (T*)y, m_max, m_dev, H,
-                             groups, parts, eps, sh);
+                             groups, parts, eps, warm, sh);
   });
   RD_CHECK_CHAINED(err);
   return RD_OK;
