@@ -291,17 +291,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
   }
-  rd::pdl_wait();  // row_start, Q and the new K/V rows come from the kernels before this one
-  const int rs = row_start[b];
-  const int n_new = row_start[b + 1] - rs;
   const int q0 = (bx / n_split) * BMQ;
   const int split = bx % n_split;  // this CTA's share of the key tiles (1 share = the whole row)
-  if (q0 >= n_new) return;
   extern __shared__ __align__(1024) uint8_t smem[];  // the swizzled boxes start at multiples of 1024
-  if ((smem_u32(smem) & 1023) != 0) {
-    if (status && threadIdx.x == 0) atomicExch(status, 24);
-    return;
-  }
   uint8_t* sQ = smem;
   uint8_t* sK = smem + L::kQBytes;
   uint8_t* sV = sK + L::kKStages * L::kKStage;
@@ -319,9 +311,35 @@ __global__ void __launch_bounds__(kThreads, 2)
   volatile int* odd_tile = abort_flag + 1;  // DENSE, [2]: 1 + the last even / odd tile whose V holds NaN or infinities
   uint64_t* v_seen = bars + 13;             // DENSE: every softmax warp has looked its part of a V tile over
   uint64_t* v_noted = bars + 14;            // DENSE: every softmax warp has noted what an odd tile holds
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&k_full[s], 1);
+      mbar_init(&v_full[s], 1);
+      mbar_init(&s_full[s], 1);
+      mbar_init(&o_full[s], 1);
+      mbar_init(&p_full[s], 4);
+    }
+    mbar_init(s_empty, 4);
+    *abort_flag = 0;
+    if (DENSE) {
+      mbar_init(v_seen, 4);
+      mbar_init(v_noted, 4);
+      odd_tile[0] = odd_tile[1] = 0;
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  rd::pdl_wait();  // row_start, Q and the new K/V rows come from the kernels before this one
+  // asked for together: one trip to memory before the first tile can be, not three
+  const int rs = row_start[b], row_end = row_start[b + 1], base = base_len[b], first_slot = kv_begin[b];
+  const int n_new = row_end - rs;
+  if (q0 >= n_new) return;
+  if ((smem_u32(smem) & 1023) != 0) {
+    if (status && threadIdx.x == 0) atomicExch(status, 24);
+    return;
+  }
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int base = base_len[b];
   const int hk = h / group;
   const int kv_end = (mode == RD_ATTN_CAUSAL) ? base + min(n_new, q0 + BMQ) : base + n_new;
   int all_tiles = (kv_end + BNK - 1) / BNK;
@@ -350,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int u = t_begin + t;
     return (WIN && u >= kept_tiles) ? u - kept_tiles + first_tile : u;
   };
-  const int kv_row0 = b * at.row_b + hk * at.row_h + kv_begin[b];  // matrix row of key 0
+  const int kv_row0 = b * at.row_b + hk * at.row_h + first_slot;  // matrix row of key 0
   auto load_k = [&](int t, uint64_t* bar) {
     const int row = kv_row0 + tile_of(t) * BNK;
     uint8_t* dst = sK + (t & 1) * L::kKStage;
@@ -368,23 +386,6 @@ __global__ void __launch_bounds__(kThreads, 2)
   };
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&v_full[s], 1);
-      mbar_init(&s_full[s], 1);
-      mbar_init(&o_full[s], 1);
-    }
-    mbar_init(s_empty, 4);
-    mbar_init(&p_full[0], 4);
-    mbar_init(&p_full[1], 4);
-    *abort_flag = 0;
-    if (DENSE) {
-      mbar_init(v_seen, 4);
-      mbar_init(v_noted, 4);
-      odd_tile[0] = odd_tile[1] = 0;
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     // The first loads (Q and the first ring's worth of K and V tiles) go out here, before the TMEM
     // allocation and the block-wide barrier below: a short chain of key tiles spends a large part of its
     // life waiting for this first data.

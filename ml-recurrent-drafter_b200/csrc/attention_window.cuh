@@ -74,8 +74,8 @@ struct Query {
 template <typename T>
 struct RowKeys {
   const T *k, *v, *tail;
-  __device__ __forceinline__ void init(const Args& a, int b, int g) {
-    const int64_t begin = a.kv_begin[b];
+  __device__ __forceinline__ void init(const Args& a, int b, int g) { init(a, b, g, a.kv_begin[b]); }
+  __device__ __forceinline__ void init(const Args& a, int b, int g, int64_t begin) {
     k = (const T*)a.k + b * a.k_batch + g * a.k_head + begin * a.k_row;
     v = (const T*)a.v + b * a.v_batch + g * a.v_head + begin * a.v_row;
     tail = a.tail_dim > 0 ? (const T*)a.k_tail + b * a.tail_batch + begin * a.tail_row : nullptr;

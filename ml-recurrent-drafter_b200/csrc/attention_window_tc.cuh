@@ -246,8 +246,9 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_window_decode_kernel
   const int group = a.nh / a.nkv;
   const int hk = blockIdx.y % a.nkv, row_tile = blockIdx.y / a.nkv;
   const int rank = (int)cluster.block_rank(), n_ranks = (int)cluster.num_blocks();
-  const int rs = a.row_start[b];
-  const int n_new = a.row_start[b + 1] - rs;
+  // asked for together: one trip to memory before the first tile can be, not three
+  const int rs = a.row_start[b], row_end = a.row_start[b + 1], base = a.base_len[b], first_slot = a.kv_begin[b];
+  const int n_new = row_end - rs;
   const int n_rows = group * n_new - row_tile * kRows;  // rows of this tile and after
   if (n_rows <= 0) return;                              // the same for the whole cluster
   extern __shared__ __align__(128) uint8_t smem[];
@@ -257,9 +258,9 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_window_decode_kernel
   float* part_ml = reinterpret_cast<float*>(smem + Y::kQ + (Y::kRing > Y::kPart ? Y::kRing : Y::kPart));  // [4][kRows][2]
   float* cta_o = part_ml + 4 * kRows * 2;          // [kRows][kOld]
   float* cta_ml = cta_o + kRows * Y::kOld;         // [kRows][2]
+  __shared__ float row_sink[kRows], row_gate[kRows];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t4 = lane & 3;
-  const int base = a.base_len[b];
   // row r of the tile: head hk * group + (row / n_new), new token row % n_new, row = row_tile * 16 + r
   auto head_of = [&](int r) { return hk * group + (row_tile * kRows + r) / n_new; };
   auto tok_of = [&](int r) { return (row_tile * kRows + r) % n_new; };
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_window_decode_kernel
   const int per = (n_all + n_ranks - 1) / n_ranks;
   const int t_begin = min(rank * per, n_all), n_tiles = min(per, n_all - t_begin);
   RowKeys<__nv_bfloat16> keys;
-  keys.init(a, b, hk);
+  keys.init(a, b, hk, first_slot);
   constexpr int CQ = DQ / 8, CV = DV / 8;
   for (int idx = tid; idx < kRows * CQ; idx += kDecodeThreads) {
     const int r = idx / CQ, c = idx % CQ;
@@ -290,6 +291,10 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_window_decode_kernel
   };
   load(0);
   load(1);
+  // what the output needs of a row's head, on its way while the keys are worked on
+  const bool has_row = tid < min(n_rows, kRows);
+  const float my_sink = has_row && a.sink != nullptr ? a.sink[head_of(tid)] : 0.f;
+  const float my_gate = has_row && a.gate != nullptr ? __bfloat162float(((const __nv_bfloat16*)a.gate)[(int64_t)(rs + tok_of(tid)) * a.ld_gate + head_of(tid)]) : 0.f;
   float o[DV / 8][4];
 #pragma unroll
   for (int i = 0; i < DV / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
@@ -392,6 +397,10 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_window_decode_kernel
       cta_ml[r * 2 + 1] = l;
     }
   }
+  if (has_row) {
+    row_sink[tid] = my_sink;
+    row_gate[tid] = a.gate != nullptr ? sigmoid_exact(my_gate) : 1.0f;
+  }
   cluster.sync();
   // the ranks share the rows of the output
   for (int idx = rank * kDecodeThreads + tid; idx < min(n_rows, kRows) * DV; idx += n_ranks * kDecodeThreads) {
@@ -407,8 +416,8 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_window_decode_kernel
       l = fmaf(f, ml[r * 2 + 1], l);
     }
     const int t = rs + tok_of(r), h = head_of(r);
-    float f = finish_softmax(m, l, a.sink, h);
-    if (a.gate != nullptr) f *= sigmoid_exact(__bfloat162float(((const __nv_bfloat16*)a.gate)[(int64_t)t * a.ld_gate + h]));
+    float f = finish_softmax(m, l, a.sink != nullptr ? row_sink + r : nullptr, 0);
+    if (a.gate != nullptr) f *= row_gate[r];
     ((__nv_bfloat16*)a.out)[((int64_t)t * a.nh + h) * a.vdim + d] = __float2bfloat16_rn(acc * f);
   }
   cluster.sync();  // peers have read this CTA's partial
@@ -440,11 +449,12 @@ int launch_decode(const Args& a, cudaStream_t s) {
     set = true;
   }
   const int row_tiles = ((a.nh / a.nkv) * a.max_new + kRows - 1) / kRows;
-  // a cluster's CTAs share the key tiles of a row: enough of them to fill the GPU twice, at least two tiles each
+  // a cluster's CTAs share the key tiles of a row: as many as run at the same time, at least two tiles each.  Two rounds of them cost more
+  // than shorter shares give: 8 rows, 8 key/value heads, up to 18 tiles, 512 CTAs 30 us, 256 CTAs 17.9.
   const int64_t visible = (int64_t)a.window + a.max_new + a.keep_first + 2 * kBN;
   const int tiles = (int)((visible < a.max_kv ? visible : a.max_kv) + kBN - 1) / kBN;
   int ranks = 1;
-  while (ranks < 8 && (int64_t)a.B * a.nkv * row_tiles * ranks < 2 * 148 && tiles / (ranks * 2) >= 2) ranks *= 2;
+  while (ranks < 8 && (int64_t)a.B * a.nkv * row_tiles * ranks * 2 <= 2 * 148 && tiles / (ranks * 2) >= 2) ranks *= 2;
   cudaError_t err = rd::launch_chained(kern, dim3(ranks, a.nkv * row_tiles, a.B), dim3(kDecodeThreads), smem, s, ranks, a);
   RD_CHECK_CHAINED(err);
   return RD_OK;

@@ -45,7 +45,7 @@ constexpr int kScanThreads = 256;
 // squares is exchanged through distributed shared memory.  The state slice stays in shared memory when the
 // row brings several tokens (smem_state), otherwise it passes through registers once.
 template <typename T, int VEC>
-__global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArgs a, int smem_state) {
+__global__ void __launch_bounds__(kScanThreads, 4) mlstm_scan_kernel(const MlstmArgs a, int smem_state) {
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) float smem[];
   rd::pdl_launch_dependents();
@@ -53,10 +53,7 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
   const int b = blockIdx.z, h = blockIdx.y;
   const int rank = (int)cluster.block_rank(), n_ranks = (int)cluster.num_blocks();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rs = a.row_start[b];
-  const int n_tok = a.path ? min(a.count[b] + 1, a.Lb) : a.row_start[b + 1] - rs;
-  if (n_tok <= 0) return;  // the same for every CTA of the cluster
-  const int32_t* path = a.path ? a.path + ((int64_t)b * a.W + a.seq[b]) * a.Lb : nullptr;
+  const int rs = a.row_start[b], row_end = a.row_start[b + 1], base = a.base_len[b];
   const int dim = a.dim, vdim = a.vdim;
   const int c0 = rank * a.slice;
   const int cols = max(0, min(a.slice, vdim - c0));
@@ -65,6 +62,28 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
   const int rows_par = kScanThreads / lanes_c;               // threads along the rows
   const int tc = tid % lanes_c, tr = tid / lanes_c;
   const bool active = tc < col_units && tr < rows_par;
+  float* S_g = a.S + ((int64_t)b * a.nh + h) * dim * vdim + c0;
+  // One token: this thread's first eight rows of the state are asked for before anything else is known (a row that starts from
+  // the zero state drops them), not after the token's q and k have come; so are the gate and the norm's weight below.  Four CTAs on an
+  // SM, because those that start beside the kernel before crowd the SMs that it leaves free: 6 rows, 8 heads of 256 x 512, one B200,
+  // 22.5 -> 20.4 us (three CTAs 23.5).
+  constexpr int U = 8;
+  float s[U][VEC];
+  auto read_state = [&](int r0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + u * rows_par;
+      const float* from = S_g + (int64_t)r * vdim + tc * VEC;
+      if constexpr (VEC == 4)
+        *reinterpret_cast<float4*>(s[u]) = r < dim ? *reinterpret_cast<const float4*>(from) : make_float4(0.f, 0.f, 0.f, 0.f);
+      else
+        s[u][0] = r < dim ? *from : 0.f;
+    }
+  };
+  if (!smem_state && active) read_state(tr);
+  const int n_tok = a.path ? min(a.count[b] + 1, a.Lb) : row_end - rs;
+  if (n_tok <= 0) return;  // the same for every CTA of the cluster
+  const int32_t* path = a.path ? a.path + ((int64_t)b * a.W + a.seq[b]) * a.Lb : nullptr;
 
   const int dim4 = (dim + 3) & ~3;         // keeps the state slice on a 16-byte boundary
   float* q_s = smem;                       // [dim]
@@ -75,8 +94,7 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
   float* ssq = warp_red + 8;               // [2]: this CTA's sum of squares, double-buffered over the tokens
   float* S_s = ssq + 2 + 6;                // [dim][slice] when smem_state
 
-  const bool fresh = a.base_len[b] == 0;
-  float* S_g = a.S + ((int64_t)b * a.nh + h) * dim * vdim + c0;
+  const bool fresh = base == 0;
   float* n_g = a.n + ((int64_t)b * a.nh + h) * dim;
   for (int d = tid; d < dim; d += kScanThreads) n_s[d] = fresh ? 0.f : n_g[d];
   float m = fresh ? 0.f : a.m[(int64_t)b * a.nh + h];
@@ -98,6 +116,11 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
       q_s[d] = rd::Num<T>::to_f(qp[d]) * qscale;
       k_s[d] = rd::Num<T>::to_f(kp[d]);
     }
+    // of this thread's output column
+    const int col = h * vdim + c0 + tid;
+    const bool has_col = a.out != nullptr && tid < cols;
+    const T g_raw = has_col ? row[(int64_t)2 * a.nh * dim + (int64_t)a.nh * vdim + col] : rd::Num<T>::from_f(0.f);
+    const T w_raw = has_col ? ((const T*)a.norm_w)[col] : rd::Num<T>::from_f(0.f);
     const float zi = soft_cap(a.gates[(int64_t)t * a.ld_gates + h] + bi, a.cap);
     const float zf = log_sigmoid(soft_cap(a.gates[(int64_t)t * a.ld_gates + a.nh + h] + bf, a.cap));
     const float m_new = fmaxf(zf + m, zi);
@@ -116,42 +139,30 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
         float* sp = S_s + tc * VEC;
         for (int r = tr; r < dim; r += rows_par) {
           const float kk = k_s[r], qq = q_s[r];
-          float s[VEC];
+          float x[VEC];
           if constexpr (VEC == 4) {
-            *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(sp + r * a.slice);
+            *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(sp + r * a.slice);
           } else {
-            s[0] = sp[r * a.slice];
+            x[0] = sp[r * a.slice];
           }
 #pragma unroll
           for (int e = 0; e < VEC; ++e) {
-            s[e] = fmaf(fa, s[e], kk * v[e]);
-            o[e] = fmaf(s[e], qq, o[e]);
+            x[e] = fmaf(fa, x[e], kk * v[e]);
+            o[e] = fmaf(x[e], qq, o[e]);
           }
           if constexpr (VEC == 4) {
-            *reinterpret_cast<float4*>(sp + r * a.slice) = *reinterpret_cast<const float4*>(s);
+            *reinterpret_cast<float4*>(sp + r * a.slice) = *reinterpret_cast<const float4*>(x);
           } else {
-            sp[r * a.slice] = s[0];
+            sp[r * a.slice] = x[0];
           }
         }
       } else {
+        // Eight rows are read before the first of them is written: a load may not pass a store that could be to the same
+        // place, so reading and writing row by row was one trip to memory after the other (30 us).
         const bool zero = fresh && it == 0;
         float* sp = S_g + tc * VEC;
-        // Eight rows are read before the first of them is written: a load may not pass a store that could be to the same
-        // place, so reading and writing row by row was one trip to memory after the other.  6 rows, 8 heads of 256 x 512, one
-        // B200: 30 -> 23.5 us.
-        constexpr int U = 8;
         for (int r0 = tr; r0 < dim; r0 += rows_par * U) {
-          float s[U][VEC];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int r = r0 + u * rows_par;
-            const bool read = r < dim && !zero;
-            if constexpr (VEC == 4) {
-              *reinterpret_cast<float4*>(s[u]) = read ? *reinterpret_cast<const float4*>(sp + (int64_t)r * vdim) : make_float4(0.f, 0.f, 0.f, 0.f);
-            } else {
-              s[u][0] = read ? sp[(int64_t)r * vdim] : 0.f;
-            }
-          }
+          if (it > 0 || r0 > tr) read_state(r0);
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const int r = r0 + u * rows_par;
@@ -159,7 +170,7 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
             const float kk = k_s[r], qq = q_s[r];
 #pragma unroll
             for (int e = 0; e < VEC; ++e) {
-              s[u][e] = fmaf(fa, s[u][e], kk * v[e]);
+              s[u][e] = fmaf(fa, zero ? 0.f : s[u][e], kk * v[e]);
               o[e] = fmaf(s[u][e], qq, o[e]);
             }
             if constexpr (VEC == 4) {
@@ -212,9 +223,7 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
       for (int r = 0; r < n_ranks; ++r) tot += *cluster.map_shared_rank(&ssq[it & 1], r);
       if (tid < cols) {
         const float rms = 1.0f / sqrtf(tot / (float)vdim + a.eps);
-        const int col = h * vdim + c0 + tid;
-        const float g = rd::Num<T>::to_f(row[(int64_t)2 * a.nh * dim + (int64_t)a.nh * vdim + col]);
-        const float y = oc * rms * rd::Num<T>::to_f(((const T*)a.norm_w)[col]) / (1.0f + expf(-g));
+        const float y = oc * rms * rd::Num<T>::to_f(w_raw) / (1.0f + expf(-rd::Num<T>::to_f(g_raw)));
         ((T*)a.out)[(int64_t)t * a.nh * vdim + col] = rd::Num<T>::from_f(y);
       }
     } else {
