@@ -368,6 +368,13 @@ RD_API int rd_attention_tc_split(const void* plan, void* out, const int32_t* row
                           const int32_t* base_len, int max_new, int mode, const uint32_t* tree_mask, int mask_words,
                           int n_split, void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
 
+/* rd_attention_tc_masked in mode RD_ATTN_CAUSAL with the keys that a row sees cut into shares; n_split and workspace as
+ * rd_attention_tc_split.  Not for plans with shared key features. */
+RD_API int rd_attention_tc_masked_split(const void* plan, void* out, const int32_t* row_start, const int32_t* kv_begin,
+                           const int32_t* base_len, int max_new, float scale, int mask_kind, int window, int keep_first, const void* gate,
+                           int64_t ld_gate, const float* sink, int n_split, void* workspace, int64_t workspace_bytes, int32_t* status,
+                           void* stream);
+
 /* rd_attention's mode RD_ATTN_DENSE on the same plans: mask_bits [m, words] 64-bit words, word w of new token t = its keys
  * 64 w .. 64 w + 63 (rd_mask_bits packs them from bytes; keys past 64 * words are hidden).  Probabilities
  * enter the second product as the sum of three bf16 numbers (24 bits); values of hidden keys do not count, NaN or not.

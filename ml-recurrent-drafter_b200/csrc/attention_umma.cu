@@ -21,7 +21,10 @@
 //               one of its rows' running max moved.
 // kHeads: one new token per row and several query heads to a key/value head (a decode step).  The rows of a CTA's query tile are
 // then the heads that share its keys, not the one token of a single head: the keys are read once per key/value head, and the
-// launch has nkv chains instead of nh.
+// launch has nkv chains instead of nh.  With windows its P goes to the tensor cores in two bf16 parts, which hold 16 of its bits (both P
+// buffers; a tile's are written when PV of the tile before is done): the warp-level kernel that serves the other short calls has
+// a maximum of its own in every warp and with it fewer roundings.  Error against 64 bits, 6 rows of 320 keys: 2.2e-4, all of it the
+// output's rounding (one part 3.0e-4, that kernel 2.3e-4).
 // kDense: an explicit mask, one 64-bit word per row and key tile.  The kernel that serves these calls on the CUDA cores keeps
 // its probabilities in fp32, so here P goes to the tensor cores as the sum of three bf16 numbers, which hold its 24 bits: two in
 // the P buffers, the third in the columns of the scores (QK of the next tile then waits for PV of this one).  Error against 64
@@ -62,8 +65,9 @@ struct Layout {
   static constexpr int kMaskBytes = QB == 2 ? BMQ * kMaxMaskWords * 4 : 0;  // the tile's bitmask rows (tree mode)
   static constexpr int kBytes = kQBytes + kKStages * kKStage + kVStages * kVStage + kMaskBytes + 256;
 };
-// TMEM columns
 constexpr float kMaxSlack = 6.0f;  // log2 units the tile max may exceed the running max without moving it
+constexpr float kTinyPart = 0x1p-60f;  // the second part of a probability is at least this, unless that one is smaller
+// TMEM columns
 constexpr uint32_t kColS = 0;     // S: 64 fp32 columns
 constexpr uint32_t kColP = 64;    // P: two buffers of 64 bf16 = 32 columns each
 constexpr uint32_t kColO = 128;   // O: 128 fp32 columns, accumulated over the tiles
@@ -274,6 +278,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                           int n_split, float* partial, const WindowArgs win) {
   using L = Layout<QB>;
   constexpr bool DENSE = FORM == kDense, HEADS = FORM == kHeads;
+  constexpr bool PARTS = WIN && HEADS;  // P in two parts
   const int group = nh / nkv;
   // A causal query tile visits the more keys the later it lies.  CTAs start in the order of their index, so the last tiles of all
   // heads come first and the launch does not end on a few long ones (8192 tokens, 32 heads, one B200: 790 -> 584 us a layer; the
@@ -490,6 +495,9 @@ __global__ void __launch_bounds__(kThreads, 2)
             umma_ts(tO, tP + ks * 8, dv, idesc_pv, (t | ks) != 0);
             umma_ts(tO, tP + 32 + ks * 8, dv, idesc_pv, 1);
             umma_ts(tO, tS + ks * 8, dv, idesc_pv, 1);
+          } else if (PARTS) {
+            umma_ts(tO, tP + ks * 8, dv, idesc_pv, (t | ks) != 0);
+            umma_ts(tO, tP + 32 + ks * 8, dv, idesc_pv, 1);
           } else {
             umma_ts(tO, tP + (t & 1) * 32 + ks * 8, dv, idesc_pv, (t | ks) != 0);
           }
@@ -698,7 +706,15 @@ __global__ void __launch_bounds__(kThreads, 2)
           const float p1 = ex2_approx(fmaf(__uint_as_float(sb[2 * i + 1]), scale_log2, neg_m));
           rowsum0 += p0;
           rowsum1 += p1;
-          pb[i] = pack_bf16(p0, p1);
+          if (PARTS) {
+            // cut, not rounded: what is left is exact in fp32 and, kept off zero, leaves an infinite value's product infinite
+            const uint32_t c0 = __float_as_uint(p0), c1 = __float_as_uint(p1);
+            pb[i] = __byte_perm(c0, c1, 0x7632);
+            sb[2 * i] = __float_as_uint(fmaxf(p0 - __uint_as_float(c0 & 0xffff0000u), fminf(p0, kTinyPart)));
+            sb[2 * i + 1] = __float_as_uint(fmaxf(p1 - __uint_as_float(c1 & 0xffff0000u), fminf(p1, kTinyPart)));
+          } else {
+            pb[i] = pack_bf16(p0, p1);
+          }
         }
       }
       l_run = l_run * (moved ? alpha : 1.0f) + (rowsum0 + rowsum1);
@@ -720,7 +736,21 @@ __global__ void __launch_bounds__(kThreads, 2)
           tmem_st32(lane_addr + kColO + c * 32, ob);
         }
       }
-      if (!DENSE) tmem_st32(lane_addr + kColP + (t & 1) * 32, pb);
+      if (PARTS) {
+        // both P buffers hold this tile's: PV of the tile before has to be done
+        if (t > 0 && !mbar_wait(&o_full[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag)) {
+          ok = false;
+          site = 4;
+          break;
+        }
+        tc_fence_after();
+        tmem_st32(lane_addr + kColP, pb);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pb[i] = pack_bf16(__uint_as_float(sb[2 * i]), __uint_as_float(sb[2 * i + 1]));
+        tmem_st32(lane_addr + kColP + 32, pb);
+      } else if (!DENSE) {
+        tmem_st32(lane_addr + kColP + (t & 1) * 32, pb);
+      }
       tc_fence_before();
       // A parity wait cannot tell a phase from the one after next, so this barrier's phase of tile t - 2 has to have been consumed.
       // It has: the scores of tile t were issued after that, and their barrier says that PV of tile t - 2 is done as well,
@@ -754,8 +784,12 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
     } else if (ok) {
       tc_fence_after();
-      float inv = WIN ? rd_win::finish_softmax(m_run, l_run, win.sink, h) : (l_run > 0.f ? 1.0f / l_run : 0.f);
-      if (WIN && win.gate != nullptr && live) inv /= 1.0f + __expf(-__bfloat162float(win.gate[(int64_t)(rs + qi) * win.ld_gate + h]));
+      float inv = WIN ? rd_win::finish_softmax(m_run, l_run, live ? win.sink : nullptr, hq) : (l_run > 0.f ? 1.0f / l_run : 0.f);
+      if (WIN && win.gate != nullptr && live) {
+        const float gate = __bfloat162float(win.gate[(int64_t)(rs + qi) * win.ld_gate + hq]);
+        if (HEADS) inv *= rd_win::sigmoid_exact(gate);
+        else inv /= 1.0f + __expf(-gate);
+      }
       uint4* dst = reinterpret_cast<uint4*>(out + ((int64_t)(rs + qi) * nh + hq) * HD);
 #pragma unroll 1
       for (int c = 0; c < HD / 32; ++c) {
@@ -805,8 +839,10 @@ __global__ void __launch_bounds__(256) mask_bits_kernel(const uint8_t* mask, int
 constexpr int kMergeWarps = 8;
 constexpr int kMergeAhead = 4;  // shares whose O is asked for at once
 
+template <bool WIN>
 __global__ void __launch_bounds__(kMergeWarps * 32) attention_merge_kernel(const float* partial, __nv_bfloat16* out,
-                                                                          const int32_t* row_start, int B, int nh, int n_split) {
+                                                                          const int32_t* row_start, int B, int nh, int n_split,
+                                                                          const WindowArgs win) {
   rd::pdl_launch_dependents();
   rd::pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -825,6 +861,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) attention_merge_kernel(const
     }
   };
   request(0);
+  const int h = WIN ? (int)(row % nh) : 0;
+  const float gate = WIN && win.gate != nullptr ? __bfloat162float(win.gate[row / nh * win.ld_gate + h]) : 0.f;
   float m = ml.x;
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
@@ -850,6 +888,13 @@ __global__ void __launch_bounds__(kMergeWarps * 32) attention_merge_kernel(const
     }
   }
   __nv_bfloat16* to = out + row * HD + 2 * lane;
+  if (WIN) {
+    float f = rd_win::finish_softmax(m, l, win.sink, h);
+    if (win.gate != nullptr) f *= rd_win::sigmoid_exact(gate);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) *reinterpret_cast<__nv_bfloat162*>(to + 64 * i) = __floats2bfloat162_rn(acc[i].x * f, acc[i].y * f);
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
     *reinterpret_cast<__nv_bfloat162*>(to + 64 * i) =
@@ -948,15 +993,16 @@ static int attention_tc_launch(const void* plan, void* out, const int32_t* row_s
   RD_REQUIRE(!p->tail || (win && n_split == 1 && mode == RD_ATTN_CAUSAL), RD_ERR_UNSUPPORTED);
   // Heads as rows wherever a group has more than one and there is one token: 24 rows of some 350 keys, 32 heads on 8, one B200:
   // 31 -> 11 us a layer.
-  const bool heads = !p->tail && !win && mode == RD_ATTN_CAUSAL && max_new == 1 && p->nh > p->nkv && p->nh / p->nkv <= BMQ;
-  const int which = p->tail ? 2 : (win ? 1 : (mode == RD_ATTN_DENSE ? 3 : (heads ? 4 : 0)));
+  const bool heads = !p->tail && mode == RD_ATTN_CAUSAL && max_new == 1 && p->nh > p->nkv && p->nh / p->nkv <= BMQ;
+  const int which = p->tail ? 2 : win ? (heads ? 5 : 1) : mode == RD_ATTN_DENSE ? 3 : heads ? 4 : 0;
   auto kern = which == 2   ? attention_umma_kernel<true, 3, kPlain>
               : which == 1 ? attention_umma_kernel<true, 2, kPlain>
               : which == 3 ? attention_umma_kernel<false, 2, kDense>
               : which == 4 ? attention_umma_kernel<false, 2, kHeads>
+              : which == 5 ? attention_umma_kernel<true, 2, kHeads>
                            : attention_umma_kernel<false, 2, kPlain>;
   const int smem = p->tail ? Layout<3>::kBytes : Layout<2>::kBytes;
-  static bool smem_set[5] = {false, false, false, false, false};  // set once each, so that steady-state launches are pure launches
+  static bool smem_set[6] = {};  // set once each, so that steady-state launches are pure launches
   if (!smem_set[which]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     RD_CHECK_CHAINED(e);
@@ -971,8 +1017,9 @@ static int attention_tc_launch(const void* plan, void* out, const int32_t* row_s
   if (n_split > 1) {
     const int64_t blocks = ((int64_t)p->m_max * p->nh + kMergeWarps - 1) / kMergeWarps;
     RD_REQUIRE(blocks <= 0x7fffffff, RD_ERR_SIZE);
-    err = rd::launch_chained(attention_merge_kernel, dim3((unsigned)blocks), dim3(kMergeWarps * 32), 0, (cudaStream_t)stream, 1,
-                             (const float*)workspace, (__nv_bfloat16*)out, row_start, p->B, p->nh, n_split);
+    err = rd::launch_chained(win ? attention_merge_kernel<true> : attention_merge_kernel<false>, dim3((unsigned)blocks), dim3(kMergeWarps * 32), 0,
+                             (cudaStream_t)stream, 1, (const float*)workspace, (__nv_bfloat16*)out, row_start, p->B, p->nh, n_split,
+                             win ? *win : WindowArgs{});
     RD_CHECK_CHAINED(err);
   }
   RD_CHECK_LAUNCH();
@@ -1030,4 +1077,15 @@ extern "C" int rd_attention_tc_masked(const void* plan, void* out, const int32_t
   const WindowArgs win{mask_kind, window, keep_first, (const __nv_bfloat16*)gate, ld_gate, tok_pos, sink};
   return attention_tc_launch(plan, out, row_start, kv_begin, base_len, max_new, mode, tree_mask, mask_words, 1, nullptr, 0, status,
                              stream, &win, scale);
+}
+
+extern "C" int rd_attention_tc_masked_split(const void* plan, void* out, const int32_t* row_start, const int32_t* kv_begin,
+                                            const int32_t* base_len, int max_new, float scale, int mask_kind, int window, int keep_first,
+                                            const void* gate, int64_t ld_gate, const float* sink, int n_split, void* workspace,
+                                            int64_t workspace_bytes, int32_t* status, void* stream) {
+  RD_REQUIRE(mask_kind == RD_MASK_WINDOW || mask_kind == RD_MASK_CHUNK, RD_ERR_UNSUPPORTED);
+  RD_REQUIRE(scale > 0.f && window >= 1 && keep_first >= 0, RD_ERR_SIZE);
+  const WindowArgs win{mask_kind, window, keep_first, (const __nv_bfloat16*)gate, ld_gate, nullptr, sink};
+  return attention_tc_launch(plan, out, row_start, kv_begin, base_len, max_new, RD_ATTN_CAUSAL, nullptr, 0, n_split, workspace,
+                             workspace_bytes, status, stream, &win, scale);
 }

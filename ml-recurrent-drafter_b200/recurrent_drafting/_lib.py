@@ -75,6 +75,7 @@ SIGNATURES = {
     "rd_attention_plan_destroy": (None, [_P]),
     "rd_attention_tc": (_I, [_P, _P, _P, _P, _P, _I, _I, _P, _I, _P, _P]),
     "rd_attention_tc_masked": (_I, [_P, _P, _P, _P, _P, _I, _I, _P, _P, _I, _F, _I, _I, _I, _P, _L, _P, _P, _P]),
+    "rd_attention_tc_masked_split": (_I, [_P, _P, _P, _P, _P, _I, _F, _I, _I, _I, _P, _L, _P, _I, _P, _L, _P, _P]),
     "rd_attention_split_workspace_bytes": (_L, [_I, _I, _I]),
     "rd_attention_tc_split": (_I, [_P, _P, _P, _P, _P, _I, _I, _P, _I, _I, _P, _L, _P, _P]),
     "rd_argmax_rows": (_I, [_P, _L, _I, _P, _I, _P, _P, _P]),
@@ -180,7 +181,7 @@ def check(rc: int, what: str) -> None:
 
 # kernels enqueued per entry point where that is not one; `launches` counts the kernels this process has enqueued
 # through call() (a replayed CUDA graph adds the number of kernels captured in it, see count_replay)
-KERNELS_PER_CALL = {"rd_tree_pack": 2, "rd_gemm_bf16_tc_argmax": 2, "rd_attention_tc_split": 2, "rd_cache_unpack": 2,
+KERNELS_PER_CALL = {"rd_tree_pack": 2, "rd_gemm_bf16_tc_argmax": 2, "rd_attention_tc_split": 2, "rd_attention_tc_masked_split": 2, "rd_cache_unpack": 2,
                     "rd_cache_unpack_static": 2, "rd_mlstm_chunk": 3, "rd_mlstm_tree": 2}
 launches = 0
 

@@ -39,15 +39,15 @@ ATTN_MAX_SPLIT = 16
 DENSE_MAX_KEYS = 220 * 1024 // 32 - 128
 
 
-def key_range_shares(batch: int, n_heads: int, max_new: int, max_kv: int, n_sm: int = 148) -> int:
+def key_range_shares(batch: int, n_heads: int, max_new: int, max_kv: int, n_sm: int = 148, min_tiles: int = 4) -> int:
     """How many CTAs should share the key range of one (row, head) in the tcgen05 attention
     (rd_attention_tc_split).  One, unless the launch has fewer (row, head, query tile) chains than
-    the GPU can hold at two CTAs per SM: then enough shares to fill it, each with at least four key
+    the GPU can hold at two CTAs per SM: then enough shares to fill it, each with at least min_tiles key
     tiles of 64."""
     chains = batch * n_heads * ((max_new + 127) // 128)
     slots = 2 * n_sm
     if chains >= slots // 2:
         return 1
     by_fill = slots // chains
-    by_length = max(1, ((max_kv + 63) // 64) // 4)
+    by_length = max(1, ((max_kv + 63) // 64) // min_tiles)
     return max(1, min(ATTN_MAX_SPLIT, by_fill, by_length))

@@ -10,7 +10,7 @@ from typing import Callable, Dict, List, Optional, Tuple
 import torch
 from torch import nn
 
-from . import _lib, kv_cache
+from . import _lib, attention, kv_cache
 from .modeling_common import Linear, PendingRows
 
 
@@ -199,9 +199,9 @@ class GroupedAttention(_Mixer):
     their root mean square after the rotation (unit_norm_eps), a sink of score 0 in the softmax (zero_sink)."""
 
     def __init__(self, cfg, width: int, rotary: RotaryTables, visible: Visibility, gated: bool = False, values_are_keys: bool = False,
-                 unit_norm_eps: Optional[float] = None, zero_sink: bool = False):
+                 unit_norm_eps: Optional[float] = None, zero_sink: bool = False, scratch: Optional["Scratch"] = None):
         super().__init__()
-        self.cfg, self.rotary, self.visible = cfg, rotary, visible
+        self.cfg, self.rotary, self.visible, self.scratch = cfg, rotary, visible, scratch
         self.gated, self.values_are_keys, self.unit_norm_eps, self.zero_sink = gated, values_are_keys, unit_norm_eps, zero_sink
         c = cfg
         if values_are_keys and c.vdim != c.dim:
@@ -247,7 +247,7 @@ class GroupedAttention(_Mixer):
             q, gate = self._project_128(ctx, state, xn)
         else:
             q, gate = self._project(ctx, state, xn)
-        if self._tensor_core_prompt(ctx, q):
+        if self._tensor_core(ctx, q):
             self._attend_128(ctx, state, q, gate, mixed)
         else:
             self._attend(ctx, state, q, gate, mixed)
@@ -291,12 +291,15 @@ class GroupedAttention(_Mixer):
                               c.rot_dims, ctx.m_dev, ctx.m_max, ctx.status, early=True)
         return q, gate
 
-    def _tensor_core_prompt(self, ctx: StepContext, q: torch.Tensor) -> bool:
-        """Prompts and draft trees of the tcgen05 attention; few tokens take the kernel that shares keys among a group's heads."""
+    def _tensor_core(self, ctx: StepContext, q: torch.Tensor) -> bool:
+        """What the tcgen05 attention serves: prompts, draft trees, and single tokens of grouped heads, which share a tile.  Other calls of a
+        few tokens take the kernel that shares keys among a group's heads and a cluster's CTAs (single tokens, 32 heads on 8, one B200, back to
+        back: 6 rows of 320 keys 12.9 us there and 8.8 here, 24 rows 18.8 and 15.8, 8 rows of 1120 keys 16.1 and 16.9, 1 row of 1900 keys
+        11.3 and 9.9; in a decode step 6 rows of 320 keys 17.2 and 10.5)."""
         c, v = self.cfg, self.visible
         tree = ctx.mode == _lib.ATTN_TREE
         return (q.dtype == torch.bfloat16 and c.dim == 128 and c.vdim == 128 and q.stride(0) == c.heads * 128 and c.scale > 0
-                and (c.heads // c.kv_heads) * ctx.max_new > 32
+                and ((c.heads // c.kv_heads) * ctx.max_new > 32 or (ctx.max_new == 1 and not tree and c.heads > c.kv_heads))
                 and not (tree and (v.kind != _lib.MASK_WINDOW or v.size < _lib.MAX_BEAM_LENGTH or ctx.mask_words > 16)))
 
     def _attend(self, ctx: StepContext, state, q, gate, mixed) -> None:
@@ -312,10 +315,21 @@ class GroupedAttention(_Mixer):
         key = (q.data_ptr(), ctx.m_max, state.keys.data_ptr(), state.values.data_ptr(), ctx.batch, max_len)
         plan = self._plans.get(key, "rd_attention_plan_create", _lib.ptr(q), ctx.m_max, _lib.ptr(state.keys), _lib.ptr(state.values),
                                ctx.batch, c.heads, c.kv_heads, 128, max_len)
+        gate_ld = gate.stride(0) if gate is not None else 0
+        if ctx.max_new == 1 and ctx.mode == _lib.ATTN_CAUSAL and self.scratch is not None:
+            # of the keys that a row can see; its window and the kept tokens each begin anywhere in a tile.  A tile takes some 1.3 us and a
+            # merge 2: shares of two tiles are 3 to 20 % faster than shares of four (1 row of 340 keys 8.0 us and 10.5), but for 3 % at 8 rows of 320
+            shares = attention.key_range_shares(ctx.batch, c.kv_heads, 1, min(ctx.max_kv, v.size + v.keep_first + 128), min_tiles=2)
+            if shares > 1:
+                need = _lib.load().rd_attention_split_workspace_bytes(ctx.m_max, c.heads, shares)
+                parts = self.scratch.get(need, q.device)
+                _lib.call("rd_attention_tc_masked_split", plan, _lib.ptr(mixed), _lib.ptr(ctx.row_start), _lib.ptr(ctx.kv_begin),
+                          _lib.ptr(ctx.base_len), 1, c.scale, v.kind, v.size, v.keep_first, _lib.ptr(gate), gate_ld, _lib.ptr(self.sink), shares,
+                          _lib.ptr(parts), parts.numel(), _lib.ptr(ctx.status), _lib.stream())
+                return
         _lib.call("rd_attention_tc_masked", plan, _lib.ptr(mixed), _lib.ptr(ctx.row_start), _lib.ptr(ctx.kv_begin), _lib.ptr(ctx.base_len),
                   ctx.max_new, ctx.mode, _lib.ptr(ctx.tok_pos), _lib.ptr(ctx.tree_mask), ctx.mask_words, c.scale, v.kind, v.size,
-                  v.keep_first, _lib.ptr(gate), gate.stride(0) if gate is not None else 0, _lib.ptr(self.sink), _lib.ptr(ctx.status),
-                  _lib.stream())
+                  v.keep_first, _lib.ptr(gate), gate_ld, _lib.ptr(self.sink), _lib.ptr(ctx.status), _lib.stream())
 
     def commit_draft(self, state: kv_cache.LayerKeyValues, kv_begin, fp, n_accepted, seq_in_beam, beam_shape) -> None:
         self._commit_planes((state.keys, state.values), kv_begin, fp, n_accepted, seq_in_beam, beam_shape)

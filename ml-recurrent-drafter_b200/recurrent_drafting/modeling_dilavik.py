@@ -16,7 +16,7 @@ class DecoderLayer(StreamLayer):
         H, c = model_cfg.hidden_size, cfg.mixer
         if cfg.type == "attention":
             visible = mixers.Visibility(_lib.MASK_WINDOW, c.window, c.keep_first)
-            mixer = mixers.GroupedAttention(c, H, rotary, visible, gated=True)
+            mixer = mixers.GroupedAttention(c, H, rotary, visible, gated=True, scratch=scratch)
         else:
             mixer = mixers.MatrixMemory(c, H, model_cfg.norm_eps, scratch)
         super().__init__(H, mixer, mixers.DenseFeedForward(H, cfg.ff) if cfg.ff is not None else None)

@@ -22,7 +22,7 @@ class NulunexForCausalLM(StreamDecoder):
         mixer: torch.nn.Module
         if cfg.type == "attention":
             mixer = mixers.GroupedAttention(c, H, self.rotary, mixers.Visibility(_lib.MASK_CHUNK, c.chunk), values_are_keys=True,
-                                            unit_norm_eps=eps, zero_sink=True)
+                                            unit_norm_eps=eps, zero_sink=True, scratch=self.scratch)
         else:
             mixer = mixers.LatentAttention(c, H, eps, self.rotary, self.scratch, mixers.Visibility(_lib.MASK_WINDOW, c.window))
         mlp: Optional[torch.nn.Module] = None
