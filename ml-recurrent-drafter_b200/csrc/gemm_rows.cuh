@@ -159,6 +159,12 @@ __device__ __forceinline__ bool rows_epilogue(const EpiArgs& epi, const RowsShap
     auto finish = [&](float* v, int n_warp0, int c, bool vec_ok, float bias, const ResidualRegs<OUT_F32, kOut>& res) {
       if (EPI == kEpiArgmax) {
         epilogue_argmax_block(v, epi, scr, lane, n_warp0, c, M, N);
+      } else if (EPI == kEpiResShares) {
+        EpiArgs part = epi;
+        part.C = epi.parts + (int64_t)blockIdx.y * epi.part_rows * N;
+        part.ldc = N;
+        epilogue_block<RD_EPI_NONE, true>(v, part, scr, lane, n_warp0, c, M, N, N % 4 == 0 && n_warp0 + 32 <= N, ResidualRegs<true, 32>(), nullptr,
+                                          make_uint4(0u, 0u, 0u, 0u), ss_red);
       } else if (EPI == kEpiSplit && n_warp0 >= epi.n_split) {
         epilogue_hi_block(v, epi, lane, n_warp0, c, M, N);
       } else {
@@ -262,7 +268,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int steps = (K / BK + sh.kb - 1) / sh.kb;
+  int steps = (K / BK + sh.kb - 1) / sh.kb, step0 = 0;
+  if (EPI == kEpiResShares) {  // of this CTA's share
+    step0 = (int)blockIdx.y * steps / (int)gridDim.y;
+    steps = ((int)blockIdx.y + 1) * steps / (int)gridDim.y - step0;
+  }
   const int row0 = blockIdx.x * sh.rows;
   rd::pdl_launch_dependents();
   // weight loads before the dependency wait: as many stages as there are with the most tokens
@@ -280,7 +290,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       for (int i = 0; i < ahead; ++i) {
         mbar_expect_tx_if(&full[i], w_bytes, 1);
-        tma_load_3d(smem + i * w_bytes, &map_w, &full[i], 0, row0, i * sh.kb, 1);
+        tma_load_3d(smem + i * w_bytes, &map_w, &full[i], 0, row0, (step0 + i) * sh.kb, 1);
       }
     }
     __syncwarp();
@@ -318,7 +328,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
             break;
           }
           mbar_expect_tx_if(&full[stage], w_bytes, 1);
-          tma_load_3d(smem + stage * w_bytes, &map_w, &full[stage], 0, row0, i * sh.kb, 1);
+          tma_load_3d(smem + stage * w_bytes, &map_w, &full[stage], 0, row0, (step0 + i) * sh.kb, 1);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;
@@ -340,7 +350,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
             break;
           }
           mbar_expect_tx_if(&full[stage], a_bytes, on);
-          tma_load_3d(sA + stage * a_bytes, &maps_a.m[a_map], &full[stage], 0, 0, i * sh.kb, on);
+          tma_load_3d(sA + stage * a_bytes, &maps_a.m[a_map], &full[stage], 0, 0, (step0 + i) * sh.kb, on);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;

@@ -96,9 +96,9 @@ struct GemmPlan {
   TokMaps maps_a;       // the same tensor in boxes of 64 x 32/64/96/128: the pair kernel fetches only the rows its chunk fills
   CUtensorMap map_w;  // weights [N, K], box 64 x 128
   int m_max, N, K;
-  RowsShape rows;
-  CUtensorMap map_rows_w;  // [k-blocks][N][64], box kb x rows
-  RowMaps maps_rows_a;     // [k-blocks][m_max][64], boxes of kb x 16 / 32 / 64 .. tokens as far as m_max needs them
+  RowsShape rows, cut;     // of whole projections; of those in shares of K
+  CUtensorMap map_rows_w, map_cut_w;  // [k-blocks][N][64], box kb x rows
+  RowMaps maps_rows_a, maps_cut_a;    // [k-blocks][m_max][64], boxes of kb x 16 / 32 / 64 .. tokens as far as m_max needs them
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -1511,6 +1511,16 @@ int multiprocessors() {
   return sm_count;
 }
 
+RowsShape rows_shape_of(int m_max, int rows) {
+  RowsShape s{};
+  s.a_rows = row_map_rows(row_map_index(m_max));
+  // the more k-blocks a step has the less its own cost counts, as long as four steps fit
+  for (s.kb = rows == 32 ? 4 : (rows <= 160 ? 2 : 1); s.kb > (rows < BM ? 2 : 1) && rows_stages(rows, s.a_rows, s.kb) < 4;) s.kb /= 2;
+  for (s.tmem_cols = 32; s.tmem_cols < (rows > BM ? 2 : 1) * max(s.a_rows, 32);) s.tmem_cols *= 2;
+  s.rows = rows;
+  return s;
+}
+
 // Slabs of gemm_rows_kernel for m_max tokens; rows 0 where it does not serve.  One wave of slabs has to cover the matrix, and K has to be
 // whole k-blocks.  Slabs of 96 rows are left out: QKV projections of 96 heads need whole heads, and the others finish as soon
 // with 128.  A narrow slab's products cost the same as a wide one's and every CTA loads all tokens, so with many tokens other splits win:
@@ -1522,12 +1532,19 @@ RowsShape rows_shape(int m_max, int N, int K) {
   int rows = ((N + multiprocessors() - 1) / multiprocessors() + 31) / 32 * 32;
   if (rows == 96) rows = 128;
   if (rows > 256 || m_max > (rows == 32 ? 64 : (rows == 64 ? 128 : kMaxChunk))) return s;
-  s.a_rows = row_map_rows(row_map_index(m_max));
-  // the more k-blocks a step has the less its own cost counts, as long as four steps fit
-  for (s.kb = rows == 32 ? 4 : (rows <= 160 ? 2 : 1); s.kb > (rows < BM ? 2 : 1) && rows_stages(rows, s.a_rows, s.kb) < 4;) s.kb /= 2;
-  for (s.tmem_cols = 32; s.tmem_cols < (rows > BM ? 2 : 1) * max(s.a_rows, 32);) s.tmem_cols *= 2;
-  s.rows = rows;
-  return s;
+  return rows_shape_of(m_max, rows);
+}
+
+// Slabs of projections in shares of K (rd::share_count, which counts tiles of 256 rows for the pairs: slabs of half of that and shares
+// fill no more than a wave).  The pair kernel would serve them too, but it reads a share through the same number of SMs only after the kernel
+// before has finished.  Such a slab also beats slabs of all of K where those are narrow: 128 CTAs of 32 rows load the tokens 128 times, 32
+// slabs in 4 shares 32 times, and a narrow slab's products cost the tensor core as much.  With the norm that follows, bf16, one B200,
+// us (in pairs; whole): 4096 x 4096, 1 token 10.1 (12.5; 11.3), 64 tokens 13.0 (13.6; 14.0), 128 tokens 13.4 (16.1); 4096 x 11008,
+// 1 token 19.2 (22.2; 21.3), 64 tokens 22.3 (24.5; 25.8), 128 tokens 25.2 (27.8), 225 tokens 33.6 (33.9); 2048 x 5632, 1 token 9.0
+// (10.4; 11.7), 128 tokens 11.6 (14.4).
+RowsShape cut_shape(int m_max, int N, int K) {
+  if (m_max > kMaxChunk || K % BK != 0 || rd::share_count(m_max, N, K, rd_gemm_pairs()) <= 1) return RowsShape{};
+  return rows_shape_of(m_max, BM);
 }
 
 template <int EPI, bool OUT_F32>
@@ -1539,10 +1556,13 @@ int launch_rows(const GemmPlan* p, const EpiArgs& e, const int32_t* m_dev, int32
     RD_CHECK_CHAINED(err);
     smem_set = true;
   }
-  const int cluster = EPI == kEpiQkvRope ? BM / p->rows.rows : 1;
-  const int grid = EPI == kEpiQkvRope ? (p->N + BM - 1) / BM * cluster : (p->N + p->rows.rows - 1) / p->rows.rows;
-  cudaError_t err = rd::launch_chained(kern, dim3(grid), dim3(kRowsThreads), kRowsSmem, s, cluster, p->maps_rows_a, p->map_rows_w, e,
-                                       p->rows, p->m_max, m_dev, p->N, p->K, status);
+  constexpr bool kCut = EPI == kEpiResShares;
+  const RowsShape& sh = kCut ? p->cut : p->rows;
+  const int cluster = EPI == kEpiQkvRope ? BM / sh.rows : 1;
+  const int grid = EPI == kEpiQkvRope ? (p->N + BM - 1) / BM * cluster : (p->N + sh.rows - 1) / sh.rows;
+  cudaError_t err = rd::launch_chained(kern, dim3(grid, kCut ? e.shares : 1), dim3(kRowsThreads), kRowsSmem, s, cluster,
+                                       kCut ? p->maps_cut_a : p->maps_rows_a, kCut ? p->map_cut_w : p->map_rows_w, e, sh, p->m_max, m_dev, p->N,
+                                       p->K, status);
   RD_CHECK_CHAINED(err);
   return RD_OK;
 }
@@ -1551,7 +1571,8 @@ template <int EPI>
 int launch_out(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t* m_dev, int32_t* status, cudaStream_t s) {
   const int sm_count = multiprocessors();
   // the folded RMS norms need 128 features in a CTA, rotary heads a cluster of whole slabs
-  if (EPI != kEpiResShares && p->rows.rows > 0 && !e.gamma && !e.ss_in && (EPI != kEpiQkvRope || p->rows.rows <= BM))
+  if (EPI == kEpiResShares ? p->cut.rows > 0
+                           : p->rows.rows > 0 && !e.gamma && !e.ss_in && (EPI != kEpiQkvRope || p->rows.rows <= BM))
     return out_dtype == RD_F32 ? launch_rows<EPI, true>(p, e, m_dev, status, s) : launch_rows<EPI, false>(p, e, m_dev, status, s);
   // upper bound of the tile count with the finest chunking the kernel may choose (64 tokens)
   const int chunks = (p->m_max + 63) / 64;
@@ -1633,11 +1654,14 @@ extern "C" void* rd_gemm_plan_create(const void* A, int64_t lda, int m_max, cons
   bool ok = make_map(&p->map_a, A, lda, m_max, K, 128) && make_map(&p->map_w, W, ldw, N, K, BM);
   for (int i = 0; ok && i < 4; ++i) ok = make_map(&p->maps_a.m[i], A, lda, m_max, K, (i + 1) * kTokBox);
   p->rows = rows_shape(m_max, N, K);
-  if (p->rows.rows > 0) {
-    ok = ok && make_map_blocks(&p->map_rows_w, W, ldw, N, K, p->rows.rows, p->rows.kb);
-    for (int i = 0; ok && i <= row_map_index(m_max); ++i)
-      ok = make_map_blocks(&p->maps_rows_a.m[i], A, lda, m_max, K, row_map_rows(i), p->rows.kb);
-  }
+  p->cut = cut_shape(m_max, N, K);
+  auto row_maps = [&](const RowsShape& sh, CUtensorMap* w, RowMaps* a) {
+    if (sh.rows == 0) return;
+    ok = ok && make_map_blocks(w, W, ldw, N, K, sh.rows, sh.kb);
+    for (int i = 0; ok && i <= row_map_index(m_max); ++i) ok = make_map_blocks(&a->m[i], A, lda, m_max, K, row_map_rows(i), sh.kb);
+  };
+  row_maps(p->rows, &p->map_rows_w, &p->maps_rows_a);
+  row_maps(p->cut, &p->map_cut_w, &p->maps_cut_a);
   if (!ok) {
     delete p;
     return nullptr;
@@ -1646,7 +1670,7 @@ extern "C" void* rd_gemm_plan_create(const void* A, int64_t lda, int m_max, cons
 }
 
 extern "C" void rd_gemm_plan_early(void* plan) {
-  if (plan) static_cast<GemmPlan*>(plan)->rows.early = 1;
+  if (plan) static_cast<GemmPlan*>(plan)->rows.early = static_cast<GemmPlan*>(plan)->cut.early = 1;
 }
 
 extern "C" int rd_gemm_few_rows(int m_max, int N, int K) { return m_max >= 1 && N >= 1 && rows_shape(m_max, N, K).rows > 0 ? 1 : 0; }

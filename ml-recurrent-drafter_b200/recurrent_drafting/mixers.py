@@ -41,8 +41,7 @@ class StepContext:
 
     def add_residual(self, lin: Linear, a: torch.Tensor, out: torch.Tensor, residual: torch.Tensor) -> None:
         """out = a W^T + residual, or, where shares pay, their rows in `parts` for the next norm."""
-        parts = None if lin.few_rows(self.m_max) else self.parts
-        self.pending = lin.add_residual(a, out, residual, self.m_dev, self.m_max, self.status, parts, early=True)
+        self.pending = lin.add_residual(a, out, residual, self.m_dev, self.m_max, self.status, self.parts, early=True)
 
 
 @dataclass(frozen=True)

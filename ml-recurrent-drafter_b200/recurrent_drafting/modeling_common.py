@@ -15,7 +15,6 @@ class Linear:
         self.bias = bias
         self._plans: Dict[Tuple, int] = {}
         self._shares_bytes: Dict[int, int] = {}  # by row capacity
-        self._few_rows: Dict[int, bool] = {}
 
     MAX_SHARE_ROWS = 1024  # row capacities above this are never cut (rd_gemm_shares_bytes)
     MAX_PLANS = 32  # distinct (activation buffer, row capacity) pairs remembered per weight
@@ -128,17 +127,6 @@ class Linear:
             need = _lib.load().rd_gemm_shares_bytes(rows, n, k) if self.weight.dtype == torch.bfloat16 else 0
             self._shares_bytes[rows] = need
         return need
-
-    def few_rows(self, m_max: int) -> bool:
-        """Calls for this many rows go through the kernel for few tokens, which has no use for shares (rd_gemm_few_rows)."""
-        if m_max > 256:
-            return False
-        got = self._few_rows.get(m_max)
-        if got is None:
-            n, k = self.weight.shape
-            got = self.weight.dtype == torch.bfloat16 and bool(_lib.load().rd_gemm_few_rows(m_max, n, k))
-            self._few_rows[m_max] = got
-        return got
 
     def add_residual(self, a: torch.Tensor, c: torch.Tensor, residual: torch.Tensor, m_dev, m_max: int, status: Optional[torch.Tensor],
                      parts: Optional[torch.Tensor] = None, early: bool = False) -> Optional["PendingRows"]:

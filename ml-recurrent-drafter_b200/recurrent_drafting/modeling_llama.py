@@ -377,7 +377,7 @@ class LlamaForCausalLM(LMHead, nn.Module):
                           _lib.ptr(weight), _lib.ptr(y), m_max, md, H, self.eps, st)
 
         def add_residual(lin_l, a):
-            return lin_l.add_residual(a, h, h, m_dev, m_max, self.gemm_status, None if lin_l.few_rows(m_max) else parts, early=True)
+            return lin_l.add_residual(a, h, h, m_dev, m_max, self.gemm_status, parts, early=True)
 
         # `early`: everything below follows the embedding kernel, and nothing in it writes a weight
         pending = None

@@ -37,7 +37,7 @@ def test_sums_and_residual(m, live, n, k, early):
 
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     lin = _linear(n, k, g)
-    assert lin.few_rows(m)
+    assert _lib.load().rd_gemm_few_rows(m, n, k) == 1
     a = torch.randn(m, k, generator=g, device="cuda").bfloat16()
     r = torch.randn(m, n, generator=g, device="cuda")
     rows = m if live is None else live
@@ -67,7 +67,7 @@ def test_epilogues(m, n, early):
     k = 512
     g = torch.Generator(device="cuda").manual_seed(m + n)
     lin, head = _linear(n, k, g, bias=True), _linear(n, k, g)
-    assert lin.few_rows(m)
+    assert _lib.load().rd_gemm_few_rows(m, n, k) == 1
     a = torch.randn(m, k, generator=g, device="cuda").bfloat16()
     r = torch.randn(m, n, generator=g, device="cuda").bfloat16()
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
@@ -119,13 +119,15 @@ def test_epilogues(m, n, early):
 def test_rotary_heads(nh, nkv, m, live, kind, early):
     """Rotation, head norm, gates and cache append against the kernel for more tokens: a row's values may differ by the rounding to bf16
     where the two add up in another order."""
+    from recurrent_drafting import _lib
     from recurrent_drafting.modeling_llama import rope_tables
 
     k, max_len, B, n_pos = 512, 90, 2, 128
     g = torch.Generator(device="cuda").manual_seed(nh + nkv + m)
     heads = nh + (1 if kind == "norm" else 2) * nkv
     lin = _linear(heads * 128 + (nh if kind == "qkvg" else 0), k, g)
-    assert lin.few_rows(m) and not lin.few_rows(300)
+    served = [_lib.load().rd_gemm_few_rows(rows, lin.weight.shape[0], k) for rows in (m, 300)]
+    assert served == [1, 0]
     cos, sin = rope_tables(128, n_pos, 10000.0, "cuda")
     rows = m if live is None else live
     i32 = dict(dtype=torch.int32, device="cuda")
