@@ -294,7 +294,7 @@ class GroupedAttention(_Mixer):
         """What the tcgen05 attention serves: prompts, draft trees, and single tokens of grouped heads, which share a tile.  Other calls of a
         few tokens take the kernel that shares keys among a group's heads and a cluster's CTAs (single tokens, 32 heads on 8, one B200, back to
         back: 6 rows of 320 keys 12.9 us there and 8.8 here, 24 rows 18.8 and 15.8, 8 rows of 1120 keys 16.1 and 16.9, 1 row of 1900 keys
-        11.3 and 9.9; in a decode step 6 rows of 320 keys 17.2 and 10.5)."""
+        11.3 and 9.9; in a decode step 6 rows of 320 keys 17.2 and 13.4 with the merge, 13.8 in one share)."""
         c, v = self.cfg, self.visible
         tree = ctx.mode == _lib.ATTN_TREE
         return (q.dtype == torch.bfloat16 and c.dim == 128 and c.vdim == 128 and q.stride(0) == c.heads * 128 and c.scale > 0
