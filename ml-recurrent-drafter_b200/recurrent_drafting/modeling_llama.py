@@ -428,12 +428,13 @@ class LlamaForCausalLM(LMHead, nn.Module):
         assert S + q_len <= cache_tensor.shape[4]
         M = B * q_len
         i32 = dict(dtype=torch.int32, device=dev)
-        tok_row = torch.arange(B, **i32)[:, None].expand(B, q_len).reshape(-1)
+        # contiguous(): one row's reshape is a view of a single element
+        tok_row = torch.arange(B, **i32)[:, None].expand(B, q_len).reshape(-1).contiguous()
         tok_slot = torch.arange(S, S + q_len, **i32).repeat(B)
         row_start = torch.arange(0, M + 1, q_len, **i32)
         kv_begin = torch.zeros(B, **i32)
         base_len = torch.full((B,), S, **i32)
-        tok_pos = position_ids.reshape(-1).clamp(min=0).to(torch.int32)
+        tok_pos = position_ids.reshape(-1).clamp(min=0).to(torch.int32).contiguous()
         dense = attention_mask.to(torch.uint8).contiguous()
         ws = self.workspace(M, 1)
         n_pos = max(4096, int(S + q_len) + 1)
