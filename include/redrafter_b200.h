@@ -187,13 +187,14 @@ RD_API void rd_gemm_plan_destroy(void* plan);
  * them start only when all that came before them is complete, so that W is as the stream's earlier work left it. */
 RD_API void rd_gemm_plan_early(void* plan);
 /* 1 if plans of this size are served by the kernel for few tokens (up to 256, fewer for matrices of few features; K a multiple of
- * 64): one wave of CTAs, each with a slab of weight rows, all of K and all tokens.  A row's sums then run over K in one piece. */
+ * 64): one wave of CTAs, each with a slab of weight rows, all of K and all tokens.  A row's sums then run over K in one piece
+ * (rd_gemm_bf16_tc_res_shares has its own slabs). */
 RD_API int rd_gemm_few_rows(int m_max, int N, int K);
 RD_API int rd_gemm_bf16_tc(const void* plan, int out_dtype, void* C, int64_t ldc, const void* bias, const void* R,
                     int64_t ldr, const int32_t* m_dev, int epilogue, int32_t* status, void* stream);
 
 /* C = A W^T + R (RD_EPI_RES), or, for few rows, the shares that a norm kernel adds up (rd_rmsnorm_shares,
- * rd_stream_norm_shares): up to 256 live rows of at most 1024, K is cut among CTA pairs that the weight tiles alone would leave idle, and
+ * rd_stream_norm_shares): up to 256 live rows of at most 1024, K is cut among CTAs that the weight tiles alone would leave idle, and
  * C is not written.  parts: rd_gemm_shares_bytes(m_max, N, K) bytes, 16-byte aligned; 0 means that no row count is cut.
  * Shares change the order of a row's fp32 additions: the last bits of a result depend on the side of 256 live rows and of 1024
  * rows of capacity on which the call lies. */

@@ -5,7 +5,8 @@
 // them through few SMs (one pair per 256 features: 96 of 148 SMs for 12288 features, 32 for 4096) and only once the kernel before has
 // finished.  Here
 //   * every CTA owns `rows` weight rows (32 .. 256, the fewest that let one wave cover the matrix), all of K and all tokens: one
-//     tile per CTA, no shares of K, and the sums of a row in the order of gemm_tc_pair_kernel;
+//     tile per CTA, and the sums of a row in the order of gemm_tc_pair_kernel.  Projections whose norm adds shares of K (kEpiResShares) have
+//     slabs of 128 rows instead and a share a CTA (cut_shape has the rule and the figures);
 //   * a load is a box of `rows` weight rows x KB k-blocks of 64 (a three-dimensional map: feature within a k-block, row, k-block), and
 //     a step of the MMA loop is such a load: with few columns the thread that issues the products, not the tensor core, sets the
 //     pace (a wait, a commit and the loop's own instructions cost it some 150 cycles a step, a product 23 to 39);
@@ -16,7 +17,7 @@
 //     and 2 to 4 for an epilogue that needs 0.6.
 // Back to back in a stream, bf16, one B200, us (the pair kernel's, o and down with the norm that adds their shares, beside): 22016 x
 // 4096, 1 token 30.7 (36.8), 110 tokens 36.5 (42.6); 12288 x 4096, 1 token 17.7 (27), 110 tokens 22.6 (31); 6144 x 4096, 24 tokens
-// 11.8 (17.8); 4096 x 4096 11.6 (12.4); 4096 x 11008 21.6 (22.1); 32000 x 4096, 1 token 41.5 (47).  In a decode step of 32 such layers
+// 11.8 (17.8); whole, 4096 x 4096 11.6 (12.4); 4096 x 11008 21.6 (22.1); 32000 x 4096, 1 token 41.5 (47).  In a decode step of 32 such layers
 // 122 -> 94 us a layer, attention and norms included.
 // Slabs of more than 128 rows take two MMAs per 16 features of K: rows [0, 128) and rows [rows - 128, rows), whose overlap is
 // computed twice and stored once.  Slabs of 32 rows read past their end in shared memory: those accumulator rows are not stored.

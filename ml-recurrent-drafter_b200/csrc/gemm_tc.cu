@@ -1524,7 +1524,7 @@ RowsShape rows_shape_of(int m_max, int rows) {
 // Slabs of gemm_rows_kernel for m_max tokens; rows 0 where it does not serve.  One wave of slabs has to cover the matrix, and K has to be
 // whole k-blocks.  Slabs of 96 rows are left out: QKV projections of 96 heads need whole heads, and the others finish as soon
 // with 128.  A narrow slab's products cost the same as a wide one's and every CTA loads all tokens, so with many tokens other splits win:
-// 4096 x 11008 with its norm, 64 tokens 25.4 us here and 25.6 in shares of K, 110 tokens 39 and 27; 6144 x 4096, 110 tokens 16.0
+// 4096 x 11008 with its norm, 64 tokens 25.4 us here and 25.6 in pairs and shares of K, 110 tokens 39 and 27; 6144 x 4096, 110 tokens 16.0
 // here and 17.8 in pairs.
 RowsShape rows_shape(int m_max, int N, int K) {
   RowsShape s{};

@@ -93,3 +93,35 @@ def test_an_infinite_value_that_is_seen(shares):
     want = outs[0].clone()
     want[:2, 5], want[2:, 7] = float("inf"), -float("inf")
     assert torch.equal(outs[1], want)
+
+
+@pytest.mark.parametrize("nh,nkv", [(3, 3), (6, 2)])
+def test_shares_of_several_causal_tokens(nh, nkv):
+    """Cut and whole differ by the rounding of the probabilities to bf16 and of the results, 2^-8 of a value each on both sides."""
+    from recurrent_drafting import _lib
+
+    lengths, new, slots, shares = [333, 90], [3, 2], 340, 4
+    g = torch.Generator(device="cuda").manual_seed(nh)
+    q = torch.randn(5, nh * HD, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(2, nkv, slots, HD, generator=g, device="cuda").bfloat16() for _ in "kv")
+    gate, sink = torch.randn(5, nh, generator=g, device="cuda").bfloat16(), torch.randn(nh, generator=g, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    row_start, zero = torch.tensor([0, 3, 5], **i32), torch.zeros(2, **i32)
+    base, status = torch.tensor([n - m for n, m in zip(lengths, new)], **i32), torch.zeros(1, **i32)
+    plan = _lib.load().rd_attention_plan_create(_lib.ptr(q), 5, _lib.ptr(k), _lib.ptr(v), 2, nh, nkv, HD, slots)
+    whole, cut, size = (torch.empty_like(q) for _ in range(3))
+    ws = torch.empty(_lib.load().rd_attention_split_workspace_bytes(5, nh, shares), dtype=torch.uint8, device="cuda")
+    arrays = (_lib.ptr(row_start), _lib.ptr(zero), _lib.ptr(base), 3)
+    tail = (HD ** -0.5, _lib.MASK_WINDOW, 200, 4, _lib.ptr(gate), nh, _lib.ptr(sink))
+
+    def run_whole(out):
+        _lib.call("rd_attention_tc_masked", plan, _lib.ptr(out), *arrays, _lib.ATTN_CAUSAL, None, None, 0, *tail, _lib.ptr(status), _lib.stream())
+
+    run_whole(whole)
+    _lib.call("rd_attention_tc_masked_split", plan, _lib.ptr(cut), *arrays, *tail, shares, _lib.ptr(ws), ws.numel(), _lib.ptr(status), _lib.stream())
+    v.abs_()
+    run_whole(size)
+    torch.cuda.synchronize()
+    _lib.load().rd_attention_plan_destroy(plan)
+    assert int(status.item()) == 0
+    assert ((cut.double() - whole.double()).abs() <= 2.0 ** -7 * (whole.double().abs() + 1.1 * size.double())).all()
