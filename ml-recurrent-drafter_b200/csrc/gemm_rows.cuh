@@ -71,9 +71,10 @@ __device__ __forceinline__ void umma_commit_if(uint64_t* bar, uint32_t on) {
 // All products of a CTA, issued by one thread; `on` = 0 runs one step without products and commits (`full` then never completes, and a
 // wait for the phase before its first passes at once).
 // MM: rows of a product.  Reading its weights takes the tensor core 32 cycles for 128 rows however few the tokens, so slabs of 32
-// and 64 rows take products of 64.  TWO: slabs of more than 128 rows.  KB: k-blocks of a step; the last step's, past K, are zeros.
+// and 64 rows take products of 64.  TWO: slabs of more than 128 rows.  KB: k-blocks of a step, of which the last step has `last`: a share
+// of K may end inside a load, whose other k-blocks are the next share's.
 template <int MM, bool TWO, int KB>
-__device__ __forceinline__ bool rows_mma(int rows, int cols, int steps, int stages, uint32_t tmem_base, uint32_t upper_cols, uint32_t s_w,
+__device__ __forceinline__ bool rows_mma(int rows, int cols, int steps, int last, int stages, uint32_t tmem_base, uint32_t upper_cols, uint32_t s_w,
                                          uint32_t s_a, int a_block, uint64_t* full, uint64_t* empty, uint64_t* acc_full, volatile int* abort_flag, uint32_t on) {
   const uint32_t idesc = (umma_instr_desc(cols) & 0x00ffffffu) | ((uint32_t)(MM >> 4) << 24);
   const uint64_t dw0 = umma_smem_desc(s_w), da0 = umma_smem_desc(s_a);
@@ -88,12 +89,13 @@ __device__ __forceinline__ bool rows_mma(int rows, int cols, int steps, int stag
     tc_fence_after();
 #pragma unroll
     for (int b = 0; b < KB; ++b) {
+      const uint32_t counts = b < last || i + 1 < steps ? on : 0;
 #pragma unroll
-      for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_if(tmem_base, dw + b * w_block + 2 * k, da + b * a_block + 2 * k, idesc, acc | b | k, on);
+      for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_if(tmem_base, dw + b * w_block + 2 * k, da + b * a_block + 2 * k, idesc, acc | b | k, counts);
       if (TWO) {
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k)
-          umma_f16_if(tmem_base + upper_cols, dw + b * w_block + upper + 2 * k, da + b * a_block + 2 * k, idesc, acc | b | k, on);
+          umma_f16_if(tmem_base + upper_cols, dw + b * w_block + upper + 2 * k, da + b * a_block + 2 * k, idesc, acc | b | k, counts);
       }
     }
     acc = 1;
@@ -269,11 +271,15 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int steps = (K / BK + sh.kb - 1) / sh.kb, step0 = 0;
-  if (EPI == kEpiResShares) {  // of this CTA's share
-    step0 = (int)blockIdx.y * steps / (int)gridDim.y;
-    steps = ((int)blockIdx.y + 1) * steps / (int)gridDim.y - step0;
+  int block0 = 0, blocks = K / BK;  // k-blocks
+  if (EPI == kEpiResShares) {
+    // of this CTA's share: cut where gemm_tc_pair_kernel cuts, however many k-blocks a load has, so that a row's sums are the same at
+    // every capacity
+    const int all = blocks;
+    block0 = (int)blockIdx.y * all / (int)gridDim.y;
+    blocks = ((int)blockIdx.y + 1) * all / (int)gridDim.y - block0;
   }
+  const int steps = (blocks + sh.kb - 1) / sh.kb, last = blocks - (steps - 1) * sh.kb;
   const int row0 = blockIdx.x * sh.rows;
   rd::pdl_launch_dependents();
   // weight loads before the dependency wait: as many stages as there are with the most tokens
@@ -291,7 +297,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       for (int i = 0; i < ahead; ++i) {
         mbar_expect_tx_if(&full[i], w_bytes, 1);
-        tma_load_3d(smem + i * w_bytes, &map_w, &full[i], 0, row0, (step0 + i) * sh.kb, 1);
+        tma_load_3d(smem + i * w_bytes, &map_w, &full[i], 0, row0, block0 + i * sh.kb, 1);
       }
     }
     __syncwarp();
@@ -329,7 +335,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
             break;
           }
           mbar_expect_tx_if(&full[stage], w_bytes, 1);
-          tma_load_3d(smem + stage * w_bytes, &map_w, &full[stage], 0, row0, (step0 + i) * sh.kb, 1);
+          tma_load_3d(smem + stage * w_bytes, &map_w, &full[stage], 0, row0, block0 + i * sh.kb, 1);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
             break;
           }
           mbar_expect_tx_if(&full[stage], a_bytes, on);
-          tma_load_3d(sA + stage * a_bytes, &maps_a.m[a_map], &full[stage], 0, 0, (step0 + i) * sh.kb, on);
+          tma_load_3d(sA + stage * a_bytes, &maps_a.m[a_map], &full[stage], 0, 0, block0 + i * sh.kb, on);
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;
@@ -368,7 +374,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
         const int n = on ? steps : 1;
         const uint32_t w = smem_u32(smem), a = smem_u32(sA);
         auto run = [&](auto mm, auto two, auto kb) {
-          return rows_mma<mm.value, two.value, kb.value>(sh.rows, cols, n, stages, tmem_base, sh.tmem_cols / 2, w, a, a_block, on ? full : idle, empty,
+          return rows_mma<mm.value, two.value, kb.value>(sh.rows, cols, n, last, stages, tmem_base, sh.tmem_cols / 2, w, a, a_block, on ? full : idle, empty,
                                                          acc_full, abort_flag, on);
         };
         if (sh.rows < BM)
