@@ -132,7 +132,8 @@ __device__ __forceinline__ bool rows_epilogue(const EpiArgs& epi, const RowsShap
   const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
   if constexpr (EPI == kEpiQkvRope) {
     const int head = row0 / BM;
-    const bool is_v = head >= epi.nh + epi.nkv, gate = head >= epi.nh + 2 * epi.nkv;
+    const int gate0 = row0 - (epi.nh + 2 * epi.nkv) * BM;  // of a slab of gates: its first one
+    const bool is_v = head >= epi.nh + epi.nkv, gate = gate0 >= 0;
     rope_meta_stage(epi, s_pos, s_dst, 0, M, quarter * 32 + lane, head < epi.nh, is_v);
     asm volatile("bar.sync 1, 128;" ::: "memory");  // the staged entries are visible
     RopeRows cs;
@@ -148,7 +149,7 @@ __device__ __forceinline__ bool rows_epilogue(const EpiArgs& epi, const RowsShap
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
       if (gate) {
-        epilogue_gate_block(v, epi, lane, quarter * 32, c, M);
+        epilogue_gate_block(v, epi, lane, gate0 + quarter * 32, c, M);
       } else {
         if (c > 0) cs.request(epi, s_pos, quarter, lane, c, M, is_v);
         epilogue_rope_block<true>(v, epi, ring, quarter, lane, head, c, M, s_dst + c, cs, nullptr, ss_red + ((c >> 5) & 1) * 128,
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
           if (gate) {
-            epilogue_gate_block(v, epi, lane, f - lane, i * 32, M);
+            epilogue_gate_block(v, epi, lane, (head - epi.nh - 2 * epi.nkv) * BM + f - lane, i * 32, M);
             continue;
           }
           const uint32_t to = mapa_u32(smem_u32(ring + ((i / parts) * 4 + f / 32) * 32 * kScrLd + f % 32), i % parts);
