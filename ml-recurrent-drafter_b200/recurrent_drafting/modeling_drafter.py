@@ -270,7 +270,8 @@ class Drafter(torch.nn.Module):
         code = _lib.dtype_code(self.dtype)
         st = _lib.stream()
         a, x = ws["a"], ws["x"]
-        ctx, start = prompt_state.contiguous(), init_token.contiguous()
+        ctx = prompt_state.contiguous()
+        start = init_token.to(ctx.device).expand(B).contiguous()  # one is all rows'; another number than B is an error
         for k in range(Lb - 1):
             bin_, bout = ws["beams"][k % 2], ws["beams"][(k + 1) % 2]
             if k == 0:
