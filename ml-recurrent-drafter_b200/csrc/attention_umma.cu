@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       uint64_t dense = 0;  // requested ahead of the wait for the scores
       if (DENSE && live && tile_of(t) < mask_words) dense = reinterpret_cast<const uint64_t*>(tree_mask)[(int64_t)(rs + qi) * mask_words + tile_of(t)];
       uint8_t* v = sV + (t % L::kVStages) * L::kVStage;
-      uint4* mine = reinterpret_cast<uint4*>(v) + r;  // DENSE: pieces r, r + 128, ... of V are this thread's to look over
+      uint4* mine = reinterpret_cast<uint4*>(v) + r;  // DENSE: pieces r, r + 128, ... of V are this thread's to look over; PARTS: to clear
       if (DENSE) {
         if (!mbar_wait(&v_full[t % L::kVStages], (t / L::kVStages) & 1, abort_flag)) {
           ok = false;
@@ -735,6 +735,19 @@ __global__ void __launch_bounds__(kThreads, 2)
           for (int i = 0; i < 32; ++i) ob[i] = __float_as_uint(__uint_as_float(ob[i]) * a);
           tmem_st32(lane_addr + kColO + c * 32, ob);
         }
+      }
+      if (PARTS && j0 + BNK > kv_end) {
+        // The row ends inside this tile, its last: the values past its end are whatever an earlier request or the next head left there.
+        // A probability of 0 does not hide a NaN or an infinity, so they become zeros, as in the kernel for other short calls.
+        if (!mbar_wait(&v_full[t % L::kVStages], (t / L::kVStages) & 1, abort_flag)) {
+          ok = false;
+          site = 6;
+          break;
+        }
+#pragma unroll 1
+        for (int i = (kv_end - j0) * 8 + r; i < BNK * 8; i += BMQ)  // 16-byte pieces of both boxes; whole rows, wherever the swizzle puts them
+          mine[i - r] = mine[i - r + kSubTile / 16] = make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the product reads what was written here
       }
       if (PARTS) {
         // both P buffers hold this tile's: PV of the tile before has to be done
