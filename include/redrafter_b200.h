@@ -186,8 +186,9 @@ RD_API void rd_gemm_plan_destroy(void* plan);
  * chain of this library's launches, an rd_embed_gather, rd_stream_norm with ids, rd_drafter_begin or rd_drafter_prepare: these let what comes after
  * them start only when all that came before them is complete, so that W is as the stream's earlier work left it. */
 RD_API void rd_gemm_plan_early(void* plan);
-/* 1 if plans of this size are served by the kernel for few tokens (up to 256, fewer for matrices of few features; K a multiple of
- * 64): one wave of CTAs, each with a slab of weight rows, all of K and all tokens.  A row's sums then run over K in one piece
+/* 1 if plans of this size fit the kernel for few tokens (up to 256, fewer for matrices of few features; K a multiple of 64): one wave
+ * of CTAs, each with a slab of weight rows, all of K and all tokens.  A call takes it where it finishes first, up to 192 tokens (half of
+ * the capacity, if the count is on the device) and fewer for some epilogues; a row's sums run over K in one piece either way
  * (rd_gemm_bf16_tc_res_shares has its own slabs). */
 RD_API int rd_gemm_few_rows(int m_max, int N, int K);
 RD_API int rd_gemm_bf16_tc(const void* plan, int out_dtype, void* C, int64_t ldc, const void* bias, const void* R,

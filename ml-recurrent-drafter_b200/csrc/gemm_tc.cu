@@ -1521,8 +1521,8 @@ RowsShape rows_shape_of(int m_max, int rows) {
   return s;
 }
 
-// Slabs of gemm_rows_kernel for m_max tokens; rows 0 where it does not serve.  One wave of slabs has to cover the matrix, and K has to be
-// whole k-blocks.  Slabs of 96 rows are left out: QKV projections of 96 heads need whole heads, and the others finish as soon
+// Slabs of gemm_rows_kernel for m_max tokens; rows 0 where it cannot serve (where it does: rows_first).  One wave of slabs has to cover
+// the matrix, and K has to be whole k-blocks.  Slabs of 96 rows are left out: QKV projections of 96 heads need whole heads, and the others finish as soon
 // with 128.  A narrow slab's products cost the same as a wide one's and every CTA loads all tokens, so with many tokens other splits win:
 // 4096 x 11008 with its norm, 64 tokens 25.4 us here and 25.6 in pairs and shares of K, 110 tokens 39 and 27; 6144 x 4096, 110 tokens 16.0
 // here and 17.8 in pairs.
@@ -1567,12 +1567,35 @@ int launch_rows(const GemmPlan* p, const EpiArgs& e, const int32_t* m_dev, int32
   return RD_OK;
 }
 
+// Whether slabs of gemm_rows_kernel finish before the pair kernel; the values are the same.  A slab loads all tokens, a CTA of a pair
+// half of them, and a pair multiplies 256 weight rows at a time, so the more tokens the less the earlier start gives.  After an RMS norm,
+// weights early, bf16, one B200, us, slabs / pairs:
+//   whole projections up to 192 tokens: 12288 x 4096, 160 27.1 / 28.7, 192 29.4 / 29.7, 208 33.7 / 30.4; 22016 x 4096 with SwiGLU, 160
+//     44.4 / 47.2, 192 48.7 / 48.9, 256 59.0 / 53.8; 32000 x 8192, 192 103.8 / 103.4, 256 122.9 / 115.7;
+//   rotary heads in slabs of 64 rows, a cluster's exchange per 32 tokens, up to 96: 6144 x 4096, 96 21.4 / 23.1, 112 23.9 / 23.4; those with
+//     a norm of their own, which costs the pairs more, as others: 5120 x 4096, 112 23.6 / 24.4;
+//   arg-max and slice maxima of more than a slab of 128 rows per CTA, an epilogue that grows with the tokens and not with K: 32000 x 4096 with
+//     maxima, 96 56.8 / 58.9, 112 61.7 / 60.5, 256 79.0 / 71.2; 32000 x 2048, 64 31.6 / 32.3, 80 34.3 / 33.7, 256 52.7 / 45.2;
+//   shares of K, with the norm that adds them: 4096 x 11008, 192 30.0 / 32.1, 256 34.3 / 34.9; 8192 x 8192, 192 40.5 / 42.5, 256 46.0 /
+//     45.3; 8192 x 28672, 192 97.8 / 97.1, 256 118.4 / 106.7: up to 192, smaller matrices always.
+// A count on the device is a packed draft's, about half of its capacity (225 tokens of room, 110 live: 12288 x 4096 27.6 / 29.0, 22016 x
+// 4096 42.2 / 45.3).
+template <int EPI>
+bool rows_first(const GemmPlan* p, const EpiArgs& e, bool counted) {
+  const int tokens = counted ? (p->m_max + 1) / 2 : p->m_max;
+  if (EPI == kEpiResShares) return p->cut.rows > 0 && (tokens <= 192 || (int64_t)p->N * p->K < 1 << 26);
+  // the folded RMS norms need 128 features in a CTA, rotary heads a cluster of whole slabs
+  if (p->rows.rows == 0 || e.gamma || e.ss_in || (EPI == kEpiQkvRope && p->rows.rows > BM)) return false;
+  int most = 192;
+  if (EPI == kEpiQkvRope && p->rows.rows == 64 && !e.head_norm) most = 96;
+  if ((EPI == kEpiArgmax || EPI == kEpiSliceMax) && p->rows.rows > BM) most = p->K >= 4096 ? 96 : 64;
+  return tokens <= most;
+}
+
 template <int EPI>
 int launch_out(const GemmPlan* p, int out_dtype, const EpiArgs& e, const int32_t* m_dev, int32_t* status, cudaStream_t s) {
   const int sm_count = multiprocessors();
-  // the folded RMS norms need 128 features in a CTA, rotary heads a cluster of whole slabs
-  if (EPI == kEpiResShares ? p->cut.rows > 0
-                           : p->rows.rows > 0 && !e.gamma && !e.ss_in && (EPI != kEpiQkvRope || p->rows.rows <= BM))
+  if (rows_first<EPI>(p, e, m_dev != nullptr))
     return out_dtype == RD_F32 ? launch_rows<EPI, true>(p, e, m_dev, status, s) : launch_rows<EPI, false>(p, e, m_dev, status, s);
   // upper bound of the tile count with the finest chunking the kernel may choose (64 tokens)
   const int chunks = (p->m_max + 63) / 64;
