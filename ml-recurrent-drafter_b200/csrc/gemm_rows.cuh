@@ -1,9 +1,9 @@
 // The projections of few tokens (one user's decode steps, small batches, one row's draft): included by gemm_tc.cu, whose
 // epilogues, descriptors and waits it uses.
 //
-// Such a call is bound by the bytes of its weights, which 96 CTAs of this shape and more read at 7.2 TB/s.  gemm_tc_pair_kernel reads
-// them through few SMs (one pair per 256 features: 96 of 148 SMs for 12288 features, 32 for 4096) and only once the kernel before has
-// finished.  Here
+// Such a call is bound by the bytes of its weights, which one wave of these CTAs reads at 5.7 to 6.3 TB/s of a copy's 6.5 (the times
+// below).  gemm_tc_pair_kernel reads them through few SMs (one pair per 256 features: 96 of 148 SMs for 12288 features, 32 for 4096)
+// and only once the kernel before has finished.  With many tokens it wins all the same (rows_first).  Here
 //   * every CTA owns `rows` weight rows (32 .. 256, the fewest that let one wave cover the matrix), all of K and all tokens: one
 //     tile per CTA, and the sums of a row in the order of gemm_tc_pair_kernel.  Projections whose norm adds shares of K (kEpiResShares) have
 //     slabs of 128 rows instead and a share a CTA (cut_shape has the rule and the figures);

@@ -292,9 +292,10 @@ class GroupedAttention(_Mixer):
 
     def _tensor_core(self, ctx: StepContext, q: torch.Tensor) -> bool:
         """What the tcgen05 attention serves: prompts, draft trees, and single tokens of grouped heads, which share a tile.  Other calls of a
-        few tokens take the kernel that shares keys among a group's heads and a cluster's CTAs (single tokens, 32 heads on 8, one B200, back to
-        back: 6 rows of 320 keys 12.9 us there and 8.8 here, 24 rows 18.8 and 15.8, 8 rows of 1120 keys 16.1 and 16.9, 1 row of 1900 keys
-        11.3 and 9.9; in a decode step 6 rows of 320 keys 17.2 and 13.4 with the merge, 13.8 in one share)."""
+        few tokens take the kernel that shares keys among a group's heads and a cluster's CTAs.  Single tokens, 32 heads on 8, window 1024, one
+        B200, back to back with the merge, us there and here: 6 rows of 320 keys 13.8 and 10.3, 24 rows of 340 20.1 and 17.3, 64 rows of 340
+        39.0 and 32.4, 1 row of 1900 12.0 and 10.3, 8 rows of 1120 18.0 and 17.9, 32 rows of 1120 43.2 and 40.0.  The closest, 16 heads on
+        4 with 8 rows of 1120 keys: 14.0 and 14.0, and under a chunk of 1024, of which two tiles are visible, 9.7 and 10.3."""
         c, v = self.cfg, self.visible
         tree = ctx.mode == _lib.ATTN_TREE
         return (q.dtype == torch.bfloat16 and c.dim == 128 and c.vdim == 128 and q.stride(0) == c.heads * 128 and c.scale > 0
