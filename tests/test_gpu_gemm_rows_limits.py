@@ -82,3 +82,51 @@ def test_shares_on_both_sides(n, k):
     slack = (k + 16) * 2.0 ** -24 * (a[:50].double().abs() @ lin.weight.double().abs().T)  # any order of k fp32 additions
     assert ((seen[0].double().sum(0) - exact).abs() <= slack).all()
     assert all(torch.equal(x, seen[0]) for x in seen)
+
+
+# more live tokens than half of the capacity: slabs still serve where the count is on the device.  Slabs of 128, 160, 192, 224 and 256 rows
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("m,live,n,k", [(256, 256, 18944, 128), (256, 256, 22016, 192), (225, 225, 26000, 576), (256, 241, 32000, 128), (256, 250, 37888, 64)])
+def test_a_full_capacity_with_a_count(m, live, n, k, early):
+    from recurrent_drafting import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    lin = _linear(n, k, g)
+    a, r = torch.randn(m, k, generator=g, device="cuda").bfloat16(), torch.randn(m, n, generator=g, device="cuda")
+    md, status = torch.tensor([live], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = [torch.full((m, n), 5.0, device="cuda") for _ in range(3)]
+    for c in outs:  # one after the other: with early weights a launch begins while the one before runs
+        lin(a, c, _lib.EPI_RES, residual=r, m_dev=md, status=status, early=early)
+    act = torch.empty(m, n // 2, dtype=torch.bfloat16, device="cuda")
+    lin(a, act, _lib.EPI_SWIGLU, m_dev=md, status=status, early=early)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    acc = a.double() @ lin.weight.double().T
+    slack = (k + 16) * 2.0 ** -24 * (r.double().abs() + a.double().abs() @ lin.weight.double().abs().T)  # any order of k fp32 additions
+    for c in outs:
+        assert ((c.double() - acc - r.double()).abs()[:live] <= slack[:live]).all()
+        assert (c[live:] == 5.0).all()
+        assert torch.equal(c, outs[0])
+    want = (torch.nn.functional.silu(acc[:, 0::2]) * acc[:, 1::2])[:live]
+    # one rounding to bf16 of fp32 sums and an approximate exponential
+    assert ((act[:live].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-4 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("m,k", [(128, 512), (192, 4096)])
+@pytest.mark.parametrize("n", [20000, 32000])
+def test_maxima_of_a_full_capacity_with_a_count(m, k, n):
+    from recurrent_drafting import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    lin = _linear(n, k, g)
+    a = torch.randn(m, k, generator=g, device="cuda").bfloat16()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    md, status = torch.tensor([m], **i32), torch.zeros(1, **i32)
+    plain, logits, top, tok = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda"), torch.empty(n // 32, m, device="cuda"), torch.empty(m, **i32)
+    lin(a, plain, status=status)
+    assert lin.with_slice_max(a, logits, top, m_dev=md, status=status, early=True)
+    ws = torch.empty(_lib.load().rd_gemm_argmax_workspace_bytes(m, n), dtype=torch.uint8, device="cuda")
+    lin.argmax(a, tok, ws, md, m, status)
+    assert int(status.item()) == 0
+    assert torch.equal(logits, plain) and torch.equal(top, plain.view(m, n // 32, 32).amax(dim=2).T)
+    assert torch.equal(tok.long(), plain.argmax(dim=1))
