@@ -10,7 +10,7 @@
 namespace {
 
 constexpr int kNormMaxThreads = 1024;
-constexpr int kNormWarmTokens = 64;
+constexpr int kNormWarmTokens = 20;
 
 // One block per token.  The row is formed in fp32 (embedding gather, or the weighted sum of `n_hist` stored
 // rows), written to x when asked for, kept in shared memory, and normalised in groups of H / groups
@@ -18,7 +18,9 @@ constexpr int kNormWarmTokens = 64;
 // A row's stored rows are some 16 KB each, so few tokens pay for trips to memory one after the other: eight stored rows and the weight
 // are requested together.  warm: launches of few tokens run the body once on shared memory ahead of the dependency wait,
 // because its instructions come from L2 or memory the first time.  6 tokens of 4096 features, 2 .. 9 stored rows, in a decode step: 6.8
-// -> 6.1 us a launch; 8 tokens, one stored row 5.6 -> 4.8.
+// -> 6.1 us a launch; 8 tokens, one stored row 5.6 -> 4.8.  With more tokens the first run delays the projection that follows: a layer
+// of the two hybrid decoders, width 4096, us with and without it, 16 tokens 88.8 / 89.8 and 105.9 / 106.2, 24 105.5 / 102.5 and 112.6 /
+// 109.7, 64 161.2 / 158.2 and 124.8 / 121.5.
 template <typename T, int VEC, bool SHARES, bool FEW>
 __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
     const T* table, const int64_t* ids, float embed_scale, float* hist_,

@@ -23,12 +23,17 @@ __global__ void embed_gather_kernel(const T* table, const int64_t* ids, T* out,
 }
 
 // One block per row.  A row is some 8 KB, so the time is the trips to memory one after the other: the row and the weight are
-// requested together and kept in registers (kNormVecs 16-byte pieces a thread; longer rows are read twice).  WARM: launches of few
+// requested together and kept in registers (kNormVecs 16-byte pieces a thread; longer rows are read twice).  WARM: launches of the fewest
 // rows, whose blocks find room beside the kernel before, run the body once on shared memory ahead of the dependency wait, because
 // its instructions come from L2 or memory the first time.  1 row of 4096 in a decode step: 4.0 -> 2.5 us (3.0 without the
 // first run); 110 rows in shares 6.2 -> 5.5.
+// Both only as long as the blocks are few: a row in registers takes 64 of them a thread (128 with shares; 31 and 40 without), and a CTA of
+// the projection that follows starts on an SM only when enough are free.  Decode steps of Llama layers, one B200, us a layer, held / not:
+// width 4096, 96 rows 192.1 / 196.6, 128 230.9 / 235.2, 192 307.9 / 308.0, drafts of 450 rows of room and 200 live 168.6 / 164.8, 1800 and
+// 760 316.2 / 310.6; width 2048, 96 69.2 / 76.7, 450 and 200 94.3 / 91.2, 1800 and 760 117.4 / 112.8.  With and without the first run:
+// width 4096, 8 rows 94.6 / 95.5, 20 111.3 / 111.9, 24 114.3 / 113.2, 64 156.2 / 154.8; width 2048, 20 49.3 / 49.8, 24 48.8 / 48.6.
 constexpr int kNormVecs = 4;
-constexpr int kNormWarmRows = 64, kNormHeldRows = 2048;  // many rows: more blocks on an SM instead (8192 rows: 38 us re-read, 43 held)
+constexpr int kNormWarmRows = 20, kNormHeldRows = 128;  // a count on the device is taken for half of the capacity, as in a packed draft
 template <typename T, bool SHARES, bool HELD>
 __global__ void __launch_bounds__(SHARES ? 512 : 256) rmsnorm_kernel(T* x, const T* w, T* y,
                                                       int m_max, const int32_t* m_dev, int H, float eps,
@@ -390,7 +395,7 @@ static int rmsnorm_launch(int dtype, void* x, const void* weight, void* y, int m
   // few rows find room beside the kernel before (its grid leaves some SMs free); the stand-in row is at most 48 KB
   const size_t room = (size_t)H * (shares > 1 ? 4 : (dtype == RD_F32 ? 4 : 2));
   const int n_threads = shares > 1 ? 512 : 256;
-  const bool held = vectorised && m_max <= kNormHeldRows && H / vec <= kNormVecs * n_threads;
+  const bool held = vectorised && (m_dev ? (m_max + 1) / 2 : m_max) <= kNormHeldRows && H / vec <= kNormVecs * n_threads;
   const int warm = held && m_max <= kNormWarmRows && room <= 48 * 1024;
   cudaError_t err = cudaSuccess;
   RD_DISPATCH_T(dtype, {
