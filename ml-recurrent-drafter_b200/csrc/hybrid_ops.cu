@@ -21,7 +21,10 @@ constexpr int kNormWarmTokens = 20;
 // -> 6.1 us a launch; 8 tokens, one stored row 5.6 -> 4.8.  With more tokens the first run delays the projection that follows: a layer
 // of the two hybrid decoders, width 4096, us with and without it, 16 tokens 88.8 / 89.8 and 105.9 / 106.2, 24 105.5 / 102.5 and 112.6 /
 // 109.7, 64 161.2 / 158.2 and 124.8 / 121.5.
-template <typename T, int VEC, bool SHARES, bool FEW>
+// kFew: as above.  kMany: four stored rows at once, 45 registers a thread and five blocks of 256 threads on an SM.  kTurn: a row's loads as
+// the compiler orders them, 32 registers, with shares 46 (kMany would take 51 there, four blocks).
+enum Rows { kFew, kMany, kTurn };
+template <typename T, int VEC, bool SHARES, Rows ROWS>
 __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
     const T* table, const int64_t* ids, float embed_scale, float* hist_,
     int64_t hist_stride_, const float* coeff_, int n_hist_, float* x_out_, const T* w_,
@@ -30,7 +33,8 @@ __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
   float* row = smem;              // [H]
   float* part_sum = smem + H;     // [groups * parts]
   const int tid = threadIdx.x, n_thr = blockDim.x;
-  constexpr int U = FEW ? 8 : 4;  // many tokens: more blocks on an SM instead
+  constexpr bool FEW = ROWS == kFew, TOGETHER = ROWS != kTurn;
+  constexpr int U = FEW ? 8 : 4;
   // the first kernel of a step: what follows may read weights ahead of its own wait (rd_gemm_plan_early)
   const bool first = table != nullptr;
   if (!first) rd::pdl_launch_dependents();
@@ -62,8 +66,8 @@ __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
       w = w_;
       dst = y + (int64_t)t * H;
     }
-    T g0[VEC];  // the weight of this thread's first features
-    if (tid * VEC < H) {
+    T g0[VEC];  // TOGETHER: the weight of this thread's first features
+    if (TOGETHER && tid * VEC < H) {
       if constexpr (VEC == 4 && sizeof(T) == 2)
         *reinterpret_cast<uint2*>(g0) = *reinterpret_cast<const uint2*>(w + tid * VEC);
       else if constexpr (VEC == 4)
@@ -98,7 +102,7 @@ __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
           } else {
             acc[0] = src[d];
           }
-        } else {
+        } else if constexpr (TOGETHER) {
           for (int j0 = 0; j0 < n_hist; j0 += U) {
             float f[U][VEC], c[U];
 #pragma unroll
@@ -116,6 +120,18 @@ __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
 #pragma unroll
               for (int e = 0; e < VEC; ++e) acc[e] = fmaf(c[u], f[u][e], acc[e]);
             }
+          }
+        } else {
+#pragma unroll 4
+          for (int j = 0; j < n_hist; ++j) {
+            const float c = coeff[j];
+            float f[VEC];
+            if constexpr (VEC == 4)
+              *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(src + (int64_t)j * hist_stride + d);
+            else
+              f[0] = src[(int64_t)j * hist_stride + d];
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] = fmaf(c, f[e], acc[e]);
           }
         }
 #pragma unroll
@@ -152,7 +168,7 @@ __global__ void __launch_bounds__(kNormMaxThreads) stream_norm_kernel(
     const bool whole = gsize % VEC == 0;  // a vector lies in one group
     for (int d = tid * VEC; d < H; d += n_thr * VEC) {
       T o[VEC], g[VEC];
-      if (d == tid * VEC) {
+      if (TOGETHER && d == tid * VEC) {
 #pragma unroll
         for (int e = 0; e < VEC; ++e) g[e] = g0[e];
       } else if constexpr (VEC == 4 && sizeof(T) == 2)
@@ -291,9 +307,13 @@ static int stream_norm_launch(int dtype, const void* table, const int64_t* ids, 
   const bool vec = H % 4 == 0 && bits % 16 == 0 && hist_stride % 4 == 0;
   int threads = ((vec ? H / 4 : H) + 31) / 32 * 32;
   // few tokens: the row's loads all in flight at once; many tokens: small blocks, several per SM
-  const bool few = m_max <= 2 * 148;
-  const int most = few ? kNormMaxThreads : 256;
+  const int most = m_max <= 2 * 148 ? kNormMaxThreads : 256;
   threads = threads > most ? most : threads;
+  // kFew as long as all blocks run at the same time: its 64 registers leave an SM room for 1024 threads.  Layers of the two hybrid
+  // decoders, one B200, us with kFew / kTurn: width 4096, 145 tokens of a prompt 139.2 / 140.2, 193 152.3 / 148.0 (kMany 151.1), decode
+  // steps of 192 340.6 / 336.1 (343.1); width 2048, whose rows have 512 threads, 193 95.1 / 97.2, 257 98.8 / 101.4.  Past 296 tokens kMany
+  // / kTurn: width 2048, 512 115.7 / 118.4; shares 700 128.2 / 123.9.
+  const bool few = m_max <= 2 * 148 && (int64_t)m_max * threads <= 148 * 1024;
   const int warps = threads / 32;
   const int parts = groups >= warps ? 1 : (warps + groups - 1) / groups;
   size_t smem = ((size_t)H + (size_t)groups * parts) * sizeof(float);
@@ -304,11 +324,12 @@ static int stream_norm_launch(int dtype, const void* table, const int64_t* ids, 
   if (warm) smem = with_stand_in;
   cudaError_t err = cudaSuccess;
   RD_DISPATCH_T(dtype, {
-    auto few_kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true, true> : stream_norm_kernel<T, 1, true, true>)
-                                 : (vec ? stream_norm_kernel<T, 4, false, true> : stream_norm_kernel<T, 1, false, true>);
-    auto many_kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true, false> : stream_norm_kernel<T, 1, true, false>)
-                                  : (vec ? stream_norm_kernel<T, 4, false, false> : stream_norm_kernel<T, 1, false, false>);
-    auto kern = few ? few_kern : many_kern;
+    auto few_kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true, kFew> : stream_norm_kernel<T, 1, true, kFew>)
+                                 : (vec ? stream_norm_kernel<T, 4, false, kFew> : stream_norm_kernel<T, 1, false, kFew>);
+    auto turn_kern = sh.count > 1 ? (vec ? stream_norm_kernel<T, 4, true, kTurn> : stream_norm_kernel<T, 1, true, kTurn>)
+                                  : (vec ? stream_norm_kernel<T, 4, false, kTurn> : stream_norm_kernel<T, 1, false, kTurn>);
+    auto many_kern = vec ? stream_norm_kernel<T, 4, false, kMany> : stream_norm_kernel<T, 1, false, kMany>;
+    auto kern = few ? few_kern : (sh.count > 1 || m_max <= 2 * 148) ? turn_kern : many_kern;
     if (smem > 48 * 1024) {
       err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       RD_CHECK_CHAINED(err);
